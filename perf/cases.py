@@ -46,35 +46,35 @@ STD = 0.02
 def listed():
     return [
         # one step of a small chat server: eight requests with about 2,000 tokens each (the benchmark's headline)
-        dict(name="decode step, 1B, batch 8", kind="engine_decode", preset="llama-3.2-1b", batch=8, context=2048),
+        dict(name="decode step 1B batch 8", kind="engine_decode", preset="llama-3.2-1b", batch=8, context=2048),
         # the time to a first token: one prompt of 2,048 tokens through the same model (the benchmark's prefill)
-        dict(name="prompt step, 1B, 2048", kind="engine_prompt", preset="llama-3.2-1b", tokens=2048),
+        dict(name="prompt step 1B 2048", kind="engine_prompt", preset="llama-3.2-1b", tokens=2048),
         # a busy server's attention layer: 64 requests decode over contexts of very different lengths
-        dict(name="attention, 64 decodes", kind="attention", dtype="bf16", hidden=2048, heads=32, kv_heads=8, dim=64,
+        dict(name="attention 64 decodes", kind="attention", dtype="bf16", hidden=2048, heads=32, kv_heads=8, dim=64,
              portions="", singles=64, context=4096),
         # a mixed step at the 8B sizes: a prompt, the second portion of another, and 30 requests that decode
-        dict(name="attention, mixed, 8B", kind="attention", dtype="bf16", hidden=4096, heads=32, kv_heads=8, dim=128,
+        dict(name="attention mixed 8B", kind="attention", dtype="bf16", hidden=4096, heads=32, kv_heads=8, dim=128,
              portions="1531+0 517+1200", singles=30, context=3000),
         # the true 32-bit mode (trace replays): portions of two prompts beside a few single tokens
-        dict(name="attention, float32", kind="attention", dtype="f32", hidden=2048, heads=32, kv_heads=8, dim=64,
+        dict(name="attention float32", kind="attention", dtype="f32", hidden=2048, heads=32, kv_heads=8, dim=64,
              portions="512+0 200+300", singles=8, context=1024),
         # the feed-forward of a decode step, where the weights' bytes are the work
-        dict(name="feed-forward, 8 tokens", kind="feed_forward", dtype="bf16", hidden=2048, inter=8192, tokens=8),
+        dict(name="feed-forward 8 tokens", kind="feed_forward", dtype="bf16", hidden=2048, inter=8192, tokens=8),
         # the feed-forward of a prompt portion of an odd length at the 8B sizes
-        dict(name="feed-forward, 1999, 8B", kind="feed_forward", dtype="bf16", hidden=4096, inter=14336, tokens=1999),
+        dict(name="feed-forward 1999 8B", kind="feed_forward", dtype="bf16", hidden=4096, inter=14336, tokens=1999),
         # the feed-forward of a portion in the 32-bit mode
-        dict(name="feed-forward, float32", kind="feed_forward", dtype="f32", hidden=2048, inter=8192, tokens=700),
+        dict(name="feed-forward float32", kind="feed_forward", dtype="f32", hidden=2048, inter=8192, tokens=700),
         # routed experts over a portion of a prompt
-        dict(name="experts, 777 tokens", kind="experts", hidden=2048, inter=1024, experts=16, top=4, groups=4, kept=3,
+        dict(name="experts 777 tokens", kind="experts", hidden=2048, inter=1024, experts=16, top=4, groups=4, kept=3,
              shared=4096, tokens=777),
         # the delta rule over two prompts and two one-token prompts
-        dict(name="delta rule, prompts", kind="delta_rule", hidden=2048, heads=16, dk=64, dv=128, taps=4, rank=64,
+        dict(name="delta rule prompts", kind="delta_rule", hidden=2048, heads=16, dk=64, dv=128, taps=4, rank=64,
              head_decay=False, portions="1500 517 1 1"),
         # state-space duality over one whole prompt
-        dict(name="state space, 2048", kind="state_space", hidden=2048, heads=64, dim=64, states=128, groups=1, taps=4,
+        dict(name="state space 2048", kind="state_space", hidden=2048, heads=64, dim=64, states=128, groups=1, taps=4,
              norm_groups=1, portions="2048"),
         # the sampler behind a step of 64 requests, with the request defaults
-        dict(name="sample, 64 rows", kind="sample", rows=64, vocab=128256, temperature=0.7, top_k=40, top_p=0.9),
+        dict(name="sample 64 rows", kind="sample", rows=64, vocab=128256, temperature=0.7, top_k=40, top_p=0.9),
     ]
 
 
