@@ -13,60 +13,21 @@
 // what else is in the batch; the sampled token's own log-probability is
 // returned as well.
 //
-// No sort: the k-th largest value and the top-p cut are found by a 3-pass
-// radix selection over order-preserving 32-bit keys (11+11+10 bits) with
-// shared-memory histograms of counts or of probability mass.  Entries equal
-// to the k-th largest value are all kept; entries equal to the value at which
-// the cumulative probability crosses top_p are all dropped.
-//
-// One block of 1024 threads per row.
+// No sort.  A cluster of blocks shares a row (sample_kernel below): every block copies its stretch of the row into
+// shared memory once and all passes read that copy.  Requests with a moderate top_k finish on a short list of
+// candidates in one block; the rest find the k-th largest value and the top-p cut by a search over the digits of
+// order-preserving 32-bit keys.  Entries equal to the k-th largest value are all kept; entries equal to the value at
+// which the cumulative probability crosses top_p are all dropped.
 #include "common.cuh"
 #include <cooperative_groups.h>
 namespace cg = cooperative_groups;
 
 namespace {
-constexpr int THREADS = 1024;
-constexpr int BINS = 2048;
 constexpr int MAX_LOGPROBS = 32;
-constexpr int LIST_MAX = 128;
 
 __device__ __forceinline__ uint32_t to_key(float v) {
   uint32_t u = __float_as_uint(v);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
-struct Smem {
-  uint32_t hist_count[BINS];
-  float hist_mass[BINS];
-  float scratch[32];
-  int scratch_i[32];
-  uint32_t bcast[4];
-  float bcast_f[2];
-  float list_val[LIST_MAX];
-  int list_idx[LIST_MAX];
-  int list_n;
-};
-
-__device__ float block_max_arg(float v, int idx, int* out_idx, Smem& s) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-    if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
-  }
-  __syncthreads();
-  if (lane == 0) { s.scratch[warp] = v; s.scratch_i[warp] = idx; }
-  __syncthreads();
-  float bv = s.scratch[0];
-  int bi = s.scratch_i[0];
-  for (int w = 1; w < THREADS / 32; ++w) {
-    const float ov = s.scratch[w];
-    const int oi = s.scratch_i[w];
-    if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-  }
-  *out_idx = bi;
-  return bv;
 }
 
 // Philox4x32-10, one block of four words for (seed, counter).
@@ -84,267 +45,530 @@ __device__ __forceinline__ float philox_uniform(uint64_t seed, uint32_t counter)
   return (float)(c0 >> 8) * (1.0f / 16777216.0f);  // [0, 1)
 }
 
-// Scans the bins from the top with warp 0.  COUNT mode: finds the bin where the
-// count from the top reaches `need`.  MASS mode: finds the bin whose inclusion
-// first makes the mass from the top exceed `limit`.  Results in s.bcast:
-// [0] = bin, [1] = found, and the amount above that bin in bcast[2] (count) or
-// bcast_f[0] (mass).
-template <bool MASS>
-__device__ void scan_bins(Smem& s, int nbins, uint32_t need, float limit) {
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    uint32_t run_c = 0;
-    float run_m = 0.f;
-    bool found = false;
-    for (int c = 0; c < nbins / 32 && !found; ++c) {
-      const int bin = nbins - 1 - (c * 32 + lane);
-      uint32_t vc = MASS ? 0u : s.hist_count[bin];
-      float vm = MASS ? s.hist_mass[bin] : 0.f;
-      uint32_t ic = vc;
-      float im = vm;
+// The largest value of a block and its lowest index; every thread gets both.  `sv` and `si` hold one entry per warp.
+template <int N_WARPS>
+__device__ float block_max_arg(float v, int idx, int* out_idx, float* sv, int* si) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t tc = __shfl_up_sync(0xffffffffu, ic, o);
-        const float tm = __shfl_up_sync(0xffffffffu, im, o);
-        if (lane >= o) { ic += tc; im += tm; }
-      }
-      const bool hit = MASS ? (run_m + im > limit && vm > 0.f) : (run_c + ic >= need);
-      const uint32_t ballot = __ballot_sync(0xffffffffu, hit);
-      if (ballot) {
-        const int first = __ffs(ballot) - 1;
-        if (lane == first) {
-          s.bcast[0] = (uint32_t)bin;
-          s.bcast[1] = 1u;
-          s.bcast[2] = run_c + ic - vc;
-          s.bcast_f[0] = run_m + im - vm;
-        }
-        found = true;
-      } else {
-        run_c += __shfl_sync(0xffffffffu, ic, 31);
-        run_m += __shfl_sync(0xffffffffu, im, 31);
-      }
-    }
-    if (!found && lane == 0) s.bcast[1] = 0u;
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+    if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
   }
   __syncthreads();
-}
-
-// Key of the k-th largest element (k >= 1, k <= V).
-__device__ uint32_t select_kth(const float* x, int V, uint32_t k, Smem& s) {
-  uint32_t prefix = 0, mask = 0, need = k;
-  const int shifts[3] = {21, 10, 0}, bits[3] = {11, 11, 10};
-  for (int p = 0; p < 3; ++p) {
-    const int nb = 1 << bits[p];
-    for (int i = threadIdx.x; i < nb; i += THREADS) s.hist_count[i] = 0;
-    __syncthreads();
-    for (int j = threadIdx.x; j < V; j += THREADS) {
-      const uint32_t key = to_key(x[j]);
-      if ((key & mask) == prefix) atomicAdd(&s.hist_count[(key >> shifts[p]) & (nb - 1)], 1u);
-    }
-    __syncthreads();
-    scan_bins<false>(s, nb, need, 0.f);
-    const uint32_t bin = s.bcast[0];
-    need -= s.bcast[2];
-    prefix |= bin << shifts[p];
-    mask |= (uint32_t)(nb - 1) << shifts[p];
-    __syncthreads();
+  if (lane == 0) { sv[warp] = v; si[warp] = idx; }
+  __syncthreads();
+  float bv = sv[0];
+  int bi = si[0];
+  for (int w = 1; w < N_WARPS; ++w) {
+    const float ov = sv[w];
+    const int oi = si[w];
+    if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
   }
-  return prefix;
+  *out_idx = bi;
+  return bv;
 }
 
-// Largest key T such that the mass of {key >= key_floor and key >= T} exceeds
-// `limit` (so {key > T} is the set whose cumulative mass stays <= limit).
-// Returns false when even the whole set stays within the limit.
-__device__ bool select_mass_cut(const float* x, int V, float xmax, float inv_t, uint32_t key_floor, float limit,
-                                uint32_t* cut, Smem& s) {
+// ---- sampling: a cluster of 2, 4 or 8 blocks per row (by the vocabulary alone: the order of every sum, and so a
+// row's token, does not depend on what else is in the batch).
+//
+// What bounds it: the row's one trip from memory, then a chain of block-wide passes and cluster barriers.  The form
+// before this one, a block per row with nine passes over the row through L2 and histograms of floats in shared memory
+// (a compare-and-swap loop per element), took 182 us for 64 rows of 128,256 (0.18 TB/s); see SAMPLE_FIGURES below.
+//
+// Threshold without a histogram: a block's stretch is cut into 64 groups (eight lanes of a warp each).  The K-th
+// largest of all groups' maxima has at least K elements at or above it, so it bounds the K-th largest element from
+// below, and only about K elements lie above it when the row is in no particular order.  Those are handed, in index
+// order, to block 0 of the cluster, which finds the exact K-th value, the top-p cut, the draw and the
+// log-probabilities among them.  K is limited to half the groups (the bound gets loose beyond) and the list to
+// LIST_CAP entries a block; rows that do not fit (and top_k 0) take the search over digits instead: eight rounds of
+// sixteen bins, each bin's mass summed in registers in a fixed order, one exchange between the blocks a round.
+constexpr int SAMPLE_THREADS = 512;
+constexpr int SAMPLE_WARPS = SAMPLE_THREADS / 32;
+constexpr int GROUPS = SAMPLE_WARPS * 4;          // groups of eight lanes in a block
+constexpr int MAX_RANKS = 8;
+constexpr int LIST_CAP = 256;                     // candidates a block hands over
+constexpr int SAMPLE_STAGE_BYTES = 160 * 1024;    // a stretch beyond this is read from global memory in every pass
+
+struct SampleSmem {
+  // written by every block of the cluster
+  float group_max[MAX_RANKS][GROUPS];
+  float max_v[MAX_RANKS];
+  int max_i[MAX_RANKS];
+  float sum_exp[MAX_RANKS];
+  int list_n[MAX_RANKS];
+  float bins[2][MAX_RANKS][16];
+  float list_v[MAX_RANKS * LIST_CAP];             // block r's at r * LIST_CAP (used in block 0)
+  int list_i[MAX_RANKS * LIST_CAP];
+  float result[2];                                // key of the cut (as bits) and kept mass, for the distribution
+  // the block's own
+  float scratch[32];
+  int scratch_i[32];
+  float warp_bins[SAMPLE_WARPS][16];
+  uint32_t word[2];
+  float value[2];
+  float packed_v[MAX_RANKS * LIST_CAP];
+  int packed_i[MAX_RANKS * LIST_CAP];
+  float packed_e[MAX_RANKS * LIST_CAP];
+};
+
+// What a block needs to walk its stretch: warp w owns the elements [w0, w1), in steps of 32.
+struct Stretch {
+  const float* x;      // the stretch (shared memory, or the row itself)
+  int first;           // index of x[0] in the row
+  int w0, w1;          // this warp's elements
+};
+
+// Mass of the sixteen values that digit `shift` of the key can take, over the elements whose key is at least `floor`
+// and agrees with `prefix` under `mask`; an element weighs exp((v - xmax) * inv_t), or 1 with COUNT.  All blocks of
+// the cluster get all sixteen sums (`total[16]` in the caller's registers, the same in every thread).
+template <bool COUNT>
+__device__ void digit_mass(const Stretch& s, cg::cluster_group& cluster, SampleSmem& sm, int parity, uint32_t floor,
+                           uint32_t prefix, uint32_t mask, int shift, float xmax, float inv_t, float (&total)[16]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float acc[16];
+#pragma unroll
+  for (int b = 0; b < 16; ++b) acc[b] = 0.f;
+  for (int j = s.w0 + lane; j < s.w1; j += 32) {
+    const float v = s.x[j];
+    const uint32_t key = to_key(v);
+    const bool in = key >= floor && (key & mask) == prefix;
+    const float w = in ? (COUNT ? 1.f : expf((v - xmax) * inv_t)) : 0.f;
+    const int bin = (key >> shift) & 15;
+#pragma unroll
+    for (int b = 0; b < 16; ++b) acc[b] += bin == b ? w : 0.f;
+  }
+#pragma unroll
+  for (int b = 0; b < 16; ++b) acc[b] = warp_sum(acc[b]);
+  if (lane == 0)
+#pragma unroll
+    for (int b = 0; b < 16; ++b) sm.warp_bins[warp][b] = acc[b];
+  __syncthreads();
+  const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  if (threadIdx.x < 16 * ranks) {
+    const int b = threadIdx.x & 15;
+    float m = 0.f;
+    for (int w = 0; w < SAMPLE_WARPS; ++w) m += sm.warp_bins[w][b];
+    *cluster.map_shared_rank(&sm.bins[parity][rank][b], threadIdx.x >> 4) = m;
+  }
+  cluster.sync();
+#pragma unroll
+  for (int b = 0; b < 16; ++b) {
+    float m = 0.f;
+    for (int r = 0; r < ranks; ++r) m += sm.bins[parity][r][b];
+    total[b] = m;
+  }
+}
+
+// The largest key T whose set {key >= floor, key >= T} has a mass above `limit` (with FRACTION: above `limit` times
+// the mass of {key >= floor}).  False when not even the whole set has.
+template <bool COUNT, bool FRACTION>
+__device__ bool find_cut(const Stretch& s, cg::cluster_group& cluster, SampleSmem& sm, uint32_t floor, float limit,
+                         float xmax, float inv_t, uint32_t* cut) {
   uint32_t prefix = 0, mask = 0;
-  const int shifts[3] = {21, 10, 0}, bits[3] = {11, 11, 10};
-  for (int p = 0; p < 3; ++p) {
-    const int nb = 1 << bits[p];
-    for (int i = threadIdx.x; i < nb; i += THREADS) s.hist_mass[i] = 0.f;
-    __syncthreads();
-    for (int j = threadIdx.x; j < V; j += THREADS) {
-      const float v = x[j];
-      const uint32_t key = to_key(v);
-      if (key >= key_floor && (key & mask) == prefix)
-        atomicAdd(&s.hist_mass[(key >> shifts[p]) & (nb - 1)], expf((v - xmax) * inv_t));
+  float above = 0.f;
+  for (int round = 0; round < 8; ++round) {
+    const int shift = 28 - 4 * round;
+    float total[16];
+    digit_mass<COUNT>(s, cluster, sm, round & 1, floor, prefix, mask, shift, xmax, inv_t, total);
+    if (FRACTION && round == 0) {
+      float all = 0.f;
+#pragma unroll
+      for (int b = 15; b >= 0; --b) all += total[b];
+      limit *= all;
     }
-    __syncthreads();
-    scan_bins<true>(s, nb, 0u, limit);
-    const bool found = s.bcast[1] != 0u;
-    const uint32_t bin = s.bcast[0];
-    const float above = s.bcast_f[0];
-    __syncthreads();
-    if (!found) {
-      if (p == 0) return false;
-      // rounding: the finer histogram sums to a hair less than the coarse bin did;
-      // the crossing element is then the smallest key of this prefix
-      *cut = prefix;
-      return true;
+    int pick = -1, last = -1;
+    float run = above, run_pick = above, run_last = above;
+#pragma unroll
+    for (int b = 15; b >= 0; --b) {
+      if (total[b] > 0.f) {
+        if (pick < 0) { last = b; run_last = run; }
+        if (pick < 0 && run + total[b] > limit) { pick = b; run_pick = run; }
+      }
+      run += total[b];
     }
-    limit -= above;
-    prefix |= bin << shifts[p];
-    mask |= (uint32_t)(nb - 1) << shifts[p];
+    if (pick < 0) {
+      if (round == 0) return false;
+      // rounding: the digits sum to a hair less than their prefix did; the cut is then its smallest element
+      pick = max(last, 0), run_pick = run_last;
+    }
+    above = run_pick;
+    prefix |= (uint32_t)pick << shift;
+    mask |= 15u << shift;
   }
   *cut = prefix;
   return true;
 }
 
-__global__ void __launch_bounds__(THREADS)
-sample_kernel(const float* __restrict__ logits, int64_t row_stride, int V, const float* __restrict__ temperature,
-              const int* __restrict__ top_k, const float* __restrict__ top_p, const int64_t* __restrict__ seed,
-              const int* __restrict__ counter, const int* __restrict__ n_logprobs, int lp_stride,
-              int* __restrict__ out_token, float* __restrict__ out_logprob, int* __restrict__ out_ncand,
-              float* __restrict__ out_top_lp, int* __restrict__ out_top_id, float* __restrict__ probs_out) {
-  __shared__ Smem s;
-  pdl_trigger();
-  pdl_wait();
-  const int row = blockIdx.x;
-  const float* x = logits + (int64_t)row * row_stride;
-  const int tid = threadIdx.x;
-
-  // pass 1: maximum and its (lowest) index
-  float vmax = -INFINITY;
-  int imax = 0x7fffffff;
-  for (int j = tid; j < V; j += THREADS) {
-    const float v = x[j];
-    if (v > vmax) { vmax = v; imax = j; }
+// This block's elements with a key of at least `floor`, in index order, to block 0's list; `counts` (one per warp) is
+// scratch.  Every block of the cluster learns how many each found; no more than LIST_CAP are handed over.
+__device__ void hand_over(const Stretch& s, cg::cluster_group& cluster, SampleSmem& sm, uint32_t floor) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rank = (int)cluster.block_rank();
+  int mine = 0;
+  for (int j = s.w0 + lane; j < s.w1; j += 32) mine += to_key(s.x[j]) >= floor;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+  __syncthreads();
+  if (lane == 0) sm.scratch_i[warp] = mine;
+  __syncthreads();
+  int at = 0, all = 0;
+  for (int w = 0; w < SAMPLE_WARPS; ++w) {
+    if (w < warp) at += sm.scratch_i[w];
+    all += sm.scratch_i[w];
   }
-  int arg;
-  const float xmax = block_max_arg(vmax, imax, &arg, s);
-  // pass 2: log-sum-exp of the raw logits
-  float se = 0.f;
-  for (int j = tid; j < V; j += THREADS) se += expf(x[j] - xmax);
-  const float log_z = xmax + logf(block_sum(se, s.scratch));
+  if ((int)threadIdx.x < (int)cluster.num_blocks()) *cluster.map_shared_rank(&sm.list_n[rank], threadIdx.x) = all;
+  if (mine > 0 && at < LIST_CAP) {
+    float* list_v = cluster.map_shared_rank(sm.list_v, 0) + rank * LIST_CAP;
+    int* list_i = cluster.map_shared_rank(sm.list_i, 0) + rank * LIST_CAP;
+    for (int j0 = s.w0; j0 < s.w1; j0 += 32) {
+      const int j = j0 + lane;
+      const float v = j < s.w1 ? s.x[j] : 0.f;
+      const bool in = j < s.w1 && to_key(v) >= floor;
+      const uint32_t votes = __ballot_sync(0xffffffffu, in);
+      const int slot = at + __popc(votes & ((1u << lane) - 1));
+      if (in && slot < LIST_CAP) { list_v[slot] = v; list_i[slot] = s.first + j; }
+      at += __popc(votes);
+    }
+  }
+  cluster.sync();
+}
 
+__global__ void __launch_bounds__(SAMPLE_THREADS)
+sample_kernel(const float* __restrict__ logits, int64_t row_stride, int V, int per, int staged, int vectors,
+              const float* __restrict__ temperature, const int* __restrict__ top_k, const float* __restrict__ top_p,
+              const int64_t* __restrict__ seed, const int* __restrict__ counter, const int* __restrict__ n_logprobs,
+              int lp_stride, int* __restrict__ out_token, float* __restrict__ out_logprob, int* __restrict__ out_ncand,
+              float* __restrict__ out_top_lp, int* __restrict__ out_top_id, float* __restrict__ probs_out) {
+  extern __shared__ __align__(16) float stage[];
+  __shared__ SampleSmem sm;
+  pdl_trigger();
+  cluster_arrive_started();
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
+  const int row = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int first = min(V, rank * per), n = min(V, first + per) - first;
+  const int seg = (((n + SAMPLE_WARPS - 1) / SAMPLE_WARPS) + 31) & ~31;
+  Stretch s;
+  s.first = first;
+  s.w0 = min(n, warp * seg), s.w1 = min(n, s.w0 + seg);
+  pdl_wait();
+  const float* x = logits + (int64_t)row * row_stride;
+  s.x = x + first;
+  if (staged) {
+    const float* src = x + first;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(stage);
+    if (vectors) {
+      for (int j = tid * 4; j + 3 < n; j += SAMPLE_THREADS * 4)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + j * 4), "l"(src + j) : "memory");
+      for (int j = (n & ~3) + tid; j < n; j += SAMPLE_THREADS) stage[j] = src[j];
+    } else {
+      for (int j = tid; j < n; j += SAMPLE_THREADS)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + j * 4), "l"(src + j) : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    s.x = stage;
+  }
   const float temp = temperature ? temperature[row] : 0.f;
   const int k_in = top_k ? top_k[row] : 0;
   const float p_in = top_p ? top_p[row] : 1.f;
+  const int n_lp_in = min(n_logprobs ? n_logprobs[row] : 0, min(MAX_LOGPROBS, lp_stride));
   const bool greedy = !(temp > 0.f) || k_in == 1;
+
+  // maxima of the groups, of the block and (after the exchange) of the row; log-sum-exp of the raw logits
+  float vmax = -INFINITY;
+  int imax = 0x7fffffff;
+#pragma unroll 4
+  for (int j = s.w0 + lane; j < s.w1; j += 32) {
+    const float v = s.x[j];
+    if (v > vmax) { vmax = v; imax = first + j; }
+  }
+  float gmax = vmax;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
+  int barg;
+  const float bmax = block_max_arg<SAMPLE_WARPS>(vmax, imax, &barg, sm.scratch, sm.scratch_i);
+  float se = 0.f;
+  if (bmax > -INFINITY) {
+#pragma unroll 4
+    for (int j = s.w0 + lane; j < s.w1; j += 32) se += expf(s.x[j] - bmax);
+  }
+  se = block_sum(se, sm.scratch);
+  cluster_wait_started();
+  if ((lane & 7) == 0)
+    for (int r = 0; r < ranks; ++r) *cluster.map_shared_rank(&sm.group_max[rank][warp * 4 + (lane >> 3)], r) = gmax;
+  if (tid < ranks) {
+    *cluster.map_shared_rank(&sm.max_v[rank], tid) = bmax;
+    *cluster.map_shared_rank(&sm.max_i[rank], tid) = barg;
+    *cluster.map_shared_rank(&sm.sum_exp[rank], tid) = se;
+  }
+  cluster.sync();
+  float xmax = sm.max_v[0];
+  int arg = sm.max_i[0];
+  for (int r = 1; r < ranks; ++r)
+    if (sm.max_v[r] > xmax) { xmax = sm.max_v[r]; arg = sm.max_i[r]; }
+  if (arg >= V) arg = 0;                           // nothing above -inf in the row
+  float z = 0.f;
+  for (int r = 0; r < ranks; ++r)
+    if (sm.sum_exp[r] > 0.f) z += sm.sum_exp[r] * expf(sm.max_v[r] - xmax);
+  const float log_z = xmax + logf(z);
   const uint32_t key_max = to_key(xmax);
-  int token = arg;
+
+  const uint32_t k = (k_in <= 0 || k_in >= V) ? (uint32_t)V : (uint32_t)k_in;
+  const int groups = ranks * GROUPS;
+  bool listed = !greedy && k <= (uint32_t)groups / 2;             // the token comes from the list
+  const int want = listed ? (int)k : (greedy ? 0 : n_lp_in);      // how many elements the list has to hold
+  int n_list = 0;                                                 // entries of block 0's list, packed below
+  if (want > 0) {
+    // the want-th largest of the groups' maxima: a lower bound of the want-th largest element
+    if (tid == 0) sm.word[0] = 0xffffffffu;
+    __syncthreads();
+    if (tid < groups) {
+      const float* all = &sm.group_max[0][0];
+      const float mine = all[tid];
+      int larger = 0;
+      for (int g = 0; g < groups; g += 4) {
+        const float4 o = *reinterpret_cast<const float4*>(all + g);
+        larger += (o.x > mine) + (o.y > mine) + (o.z > mine) + (o.w > mine);
+      }
+      if (larger < want) atomicMin(&sm.word[0], to_key(mine));
+    }
+    __syncthreads();
+    hand_over(s, cluster, sm, sm.word[0]);
+    bool fits = true;
+    for (int r = 0; r < ranks; ++r) fits = fits && sm.list_n[r] <= LIST_CAP;
+    if (!fits) {
+      listed = false;
+      if (n_lp_in > 0) {
+        // exactly the elements at or above the K-th largest (ties beyond the list's end are left out)
+        uint32_t floor = 0;
+        find_cut<true, false>(s, cluster, sm, 0u, (float)n_lp_in - 0.5f, xmax, 1.f, &floor);
+        hand_over(s, cluster, sm, floor);
+      }
+    }
+    if (rank == 0) {
+      for (int r = 0; r < ranks; ++r) {
+        const int c = min(sm.list_n[r], LIST_CAP);
+        for (int i = tid; i < c; i += SAMPLE_THREADS) {
+          sm.packed_v[n_list + i] = sm.list_v[r * LIST_CAP + i];
+          sm.packed_i[n_list + i] = sm.list_i[r * LIST_CAP + i];
+        }
+        n_list += c;
+      }
+      __syncthreads();
+    }
+  }
+
   int ncand = 1;
   uint32_t key_cut = key_max;
   float inv_t = 1.f, z_kept = 1.f;
-
-  if (!greedy) {
+  if (greedy) {
+    if (rank == 0 && tid == 0) {
+      out_token[row] = arg;
+      out_logprob[row] = x[arg] - log_z;
+      out_ncand[row] = 1;
+      if (n_lp_in > 0) {
+        out_top_lp[(int64_t)row * lp_stride] = x[arg] - log_z;
+        out_top_id[(int64_t)row * lp_stride] = arg;
+      }
+    }
+  } else {
     inv_t = 1.0f / temp;
-    const uint32_t k = (k_in <= 0 || k_in >= V) ? (uint32_t)V : (uint32_t)k_in;
-    const uint32_t key_k = k < (uint32_t)V ? select_kth(x, V, k, s) : 0u;
-    key_cut = key_k;
-    if (p_in < 1.f) {
-      float zk = 0.f;
-      for (int j = tid; j < V; j += THREADS) {
-        const float v = x[j];
-        if (to_key(v) >= key_k) zk += expf((v - xmax) * inv_t);
-      }
-      zk = block_sum(zk, s.scratch);
-      uint32_t cross;
-      if (select_mass_cut(x, V, xmax, inv_t, key_k, p_in * zk, &cross, s)) {
-        // everything above the crossing value is kept; the maximum always is
-        key_cut = cross >= key_max ? key_max : max(key_k, cross + 1u);
-      }
-    }
-    // mass and count of what is kept; per-thread contiguous chunks give an index-ordered prefix
-    const int chunk = (V + THREADS - 1) / THREADS;
-    const int lo = min(V, tid * chunk), hi = min(V, lo + chunk);
-    float mine = 0.f;
-    int cnt = 0;
-    for (int j = lo; j < hi; ++j) {
-      const float v = x[j];
-      if (to_key(v) >= key_cut) { mine += expf((v - xmax) * inv_t); ++cnt; }
-    }
-    // inclusive scan over threads (warp scan, then warps in order)
-    const int lane = tid & 31, warp = tid >> 5;
-    float inc = mine;
-    int inc_c = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float t = __shfl_up_sync(0xffffffffu, inc, o);
-      const int tc = __shfl_up_sync(0xffffffffu, inc_c, o);
-      if (lane >= o) { inc += t; inc_c += tc; }
-    }
-    __syncthreads();
-    if (lane == 31) { s.scratch[warp] = inc; s.scratch_i[warp] = inc_c; }
-    __syncthreads();
-    float before = 0.f, total = 0.f;
-    int total_c = 0;
-    for (int w = 0; w < THREADS / 32; ++w) {
-      if (w < warp) before += s.scratch[w];
-      total += s.scratch[w];
-      total_c += s.scratch_i[w];
-    }
-    z_kept = total;
-    ncand = total_c;
     const float u = philox_uniform((uint64_t)(seed ? seed[row] : 0), (uint32_t)(counter ? counter[row] : 0));
-    const float target = u * total;
-    const float start = before + inc - mine;
-    if (tid == 0) s.bcast[3] = 0xffffffffu;
-    __syncthreads();
-    if (cnt > 0 && target >= start && target < start + mine) {
-      float run = start;
-      int pick = -1;
-      for (int j = lo; j < hi; ++j) {
-        const float v = x[j];
-        if (to_key(v) >= key_cut) {
-          pick = j;
-          run += expf((v - xmax) * inv_t);
-          if (target < run) break;
+    if (listed) {
+      if (rank == 0) {
+        // the exact k-th largest value, then the top-p cut, among the list's entries
+        if (tid == 0) sm.word[0] = 0xffffffffu, sm.word[1] = 0u;
+        __syncthreads();
+        for (int i = tid; i < n_list; i += SAMPLE_THREADS) {
+          const float v = sm.packed_v[i];
+          int larger = 0;
+          for (int o = 0; o < n_list; ++o) larger += sm.packed_v[o] > v;
+          if (larger < (int)k) atomicMin(&sm.word[0], to_key(v));
+        }
+        __syncthreads();
+        const uint32_t key_k = sm.word[0];
+        key_cut = key_k;
+        float mass = 0.f;
+        for (int i = tid; i < n_list; i += SAMPLE_THREADS) {
+          const float v = sm.packed_v[i];
+          const float e = to_key(v) >= key_k ? expf((v - xmax) * inv_t) : 0.f;
+          sm.packed_e[i] = e;
+          mass += e;
+        }
+        mass = block_sum(mass, sm.scratch);
+        if (p_in < 1.f) {
+          const float limit = p_in * mass;
+          for (int i = tid; i < n_list; i += SAMPLE_THREADS) {
+            const float v = sm.packed_v[i];
+            float above = 0.f;                     // mass of everything at or above this value
+            for (int o = 0; o < n_list; ++o) above += sm.packed_v[o] >= v ? sm.packed_e[o] : 0.f;
+            if (to_key(v) >= key_k && above > limit) atomicMax(&sm.word[1], to_key(v));
+          }
+          __syncthreads();
+          const uint32_t cross = sm.word[1];
+          // everything above the crossing value is kept; the maximum always is
+          if (cross) key_cut = cross >= key_max ? key_max : max(key_k, cross + 1u);
+        }
+        if (warp == 0) {
+          // kept mass and count, then the draw by an index-ordered prefix of the kept masses
+          float total = 0.f;
+          int count = 0;
+          for (int i0 = 0; i0 < n_list; i0 += 32) {
+            const int i = i0 + lane;
+            const bool in = i < n_list && to_key(sm.packed_v[i]) >= key_cut;
+            total += warp_sum(in ? sm.packed_e[i] : 0.f);
+            count += __popc(__ballot_sync(0xffffffffu, in));
+          }
+          const float target = u * total;
+          float run = 0.f;
+          int pick = -1;
+          for (int i0 = 0; i0 < n_list && pick < 0; i0 += 32) {
+            const int i = i0 + lane;
+            const bool in = i < n_list && to_key(sm.packed_v[i]) >= key_cut;
+            float inc = in ? sm.packed_e[i] : 0.f;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const float t = __shfl_up_sync(0xffffffffu, inc, o);
+              if (lane >= o) inc += t;
+            }
+            const uint32_t hit = __ballot_sync(0xffffffffu, in && target < run + inc);
+            if (hit) pick = i0 + __ffs(hit) - 1;
+            run += __shfl_sync(0xffffffffu, inc, 31);
+          }
+          if (lane == 0) {
+            // rounding can leave the target past the end: take the maximum then
+            out_token[row] = pick < 0 ? arg : sm.packed_i[pick];
+            out_logprob[row] = (pick < 0 ? xmax : sm.packed_v[pick]) - log_z;
+            out_ncand[row] = count;
+            sm.scratch_i[0] = count;
+            sm.value[0] = total;
+          }
+        }
+        __syncthreads();
+        ncand = sm.scratch_i[0];
+        z_kept = sm.value[0];
+        if (probs_out && tid < ranks) {
+          float* result = cluster.map_shared_rank(sm.result, tid);
+          result[0] = __uint_as_float(key_cut);
+          result[1] = z_kept;
         }
       }
-      atomicMin(&s.bcast[3], (uint32_t)pick);
+      if (probs_out) {
+        cluster.sync();
+        key_cut = __float_as_uint(sm.result[0]);
+        z_kept = sm.result[1];
+      }
+    } else {
+      uint32_t key_k = 0u;
+      if (k < (uint32_t)V) find_cut<true, false>(s, cluster, sm, 0u, (float)k - 0.5f, xmax, 1.f, &key_k);
+      key_cut = key_k;
+      if (p_in < 1.f) {
+        uint32_t cross = 0u;
+        if (find_cut<false, true>(s, cluster, sm, key_k, p_in, xmax, inv_t, &cross))
+          key_cut = cross >= key_max ? key_max : max(key_k, cross + 1u);
+      }
+      // kept mass and count of every warp's elements, of every block and of the row
+      float mine = 0.f;
+      int count = 0;
+      for (int j = s.w0 + lane; j < s.w1; j += 32) {
+        const float v = s.x[j];
+        if (to_key(v) >= key_cut) { mine += expf((v - xmax) * inv_t); ++count; }
+      }
+      mine = warp_sum(mine);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
+      __syncthreads();
+      if (lane == 0) { sm.scratch[warp] = mine; sm.scratch_i[warp] = count; }
+      __syncthreads();
+      float block_mass = 0.f;
+      int block_count = 0;
+      for (int w = 0; w < SAMPLE_WARPS; ++w) block_mass += sm.scratch[w], block_count += sm.scratch_i[w];
+      cluster.sync();                              // the last round's bins have been read everywhere
+      if (tid < ranks) {
+        float* dst = cluster.map_shared_rank(&sm.bins[0][rank][0], tid);
+        dst[0] = block_mass;
+        dst[1] = __int_as_float(block_count);
+      }
+      cluster.sync();
+      float total = 0.f;
+      ncand = 0;
+      for (int r = 0; r < ranks; ++r) total += sm.bins[0][r][0], ncand += __float_as_int(sm.bins[0][r][1]);
+      z_kept = total;
+      const float target = u * total;
+      float before = 0.f;
+      int owner = -1;
+      for (int r = 0; r < ranks && owner < 0; ++r) {
+        if (target < before + sm.bins[0][r][0]) owner = r;
+        else before += sm.bins[0][r][0];
+      }
+      if (owner < 0 && rank == 0 && tid == 0) {    // rounding can leave the target past the end: the maximum then
+        out_token[row] = arg;
+        out_logprob[row] = xmax - log_z;
+      }
+      if (owner == rank) {
+        float run = before;
+        int w_own = -1, w_last = 0;
+        for (int w = 0; w < SAMPLE_WARPS && w_own < 0; ++w) {
+          if (sm.scratch_i[w] > 0) w_last = w;
+          if (target < run + sm.scratch[w]) w_own = w;
+          else run += sm.scratch[w];
+        }
+        if (w_own < 0) w_own = w_last;
+        if (warp == w_own) {
+          int pick = -1, last = -1;
+          for (int j0 = s.w0; j0 < s.w1 && pick < 0; j0 += 32) {
+            const int j = j0 + lane;
+            const float v = j < s.w1 ? s.x[j] : 0.f;
+            const bool in = j < s.w1 && to_key(v) >= key_cut;
+            const float e = in ? expf((v - xmax) * inv_t) : 0.f;
+            float inc = e;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const float t = __shfl_up_sync(0xffffffffu, inc, o);
+              if (lane >= o) inc += t;
+            }
+            const uint32_t kept = __ballot_sync(0xffffffffu, in);
+            const uint32_t hit = __ballot_sync(0xffffffffu, in && target < run + inc);
+            if (kept) last = j0 + 31 - __clz(kept);
+            if (hit) pick = j0 + __ffs(hit) - 1;
+            run += __shfl_sync(0xffffffffu, inc, 31);
+          }
+          if (pick < 0) pick = last;
+          if (lane == 0) {
+            out_token[row] = pick < 0 ? arg : first + pick;
+            out_logprob[row] = (pick < 0 ? xmax : s.x[pick]) - log_z;
+          }
+        }
+      }
+      if (rank == 0 && tid == 0) out_ncand[row] = ncand;
     }
-    __syncthreads();
-    // rounding can leave the target past the last chunk: take the maximum then
-    token = s.bcast[3] == 0xffffffffu ? arg : (int)s.bcast[3];
+    // log-probabilities of the highest candidates
+    const int n_lp = min(n_lp_in, ncand);
+    if (rank == 0 && n_lp > 0) {
+      for (int i = tid; i < n_list; i += SAMPLE_THREADS) {
+        const float v = sm.packed_v[i];
+        const int id = sm.packed_i[i];
+        int place = 0;
+        for (int o = 0; o < n_list && place < n_lp; ++o) {
+          const float ov = sm.packed_v[o];
+          place += ov > v || (ov == v && sm.packed_i[o] < id);
+        }
+        if (place < n_lp) {
+          out_top_lp[(int64_t)row * lp_stride + place] = v - log_z;
+          out_top_id[(int64_t)row * lp_stride + place] = id;
+        }
+      }
+    }
   }
-
   if (probs_out) {
-    float* po = probs_out + (int64_t)row * V;
-    for (int j = tid; j < V; j += THREADS) {
-      const float v = x[j];
+    float* po = probs_out + (int64_t)row * V + first;
+    for (int j = s.w0 + lane; j < s.w1; j += 32) {
+      const float v = s.x[j];
       float p = 0.f;
-      if (greedy) p = (j == arg) ? 1.f : 0.f;
+      if (greedy) p = first + j == arg ? 1.f : 0.f;
       else if (to_key(v) >= key_cut) p = expf((v - xmax) * inv_t) / z_kept;
       po[j] = p;
-    }
-  }
-  if (tid == 0) {
-    out_token[row] = token;
-    out_logprob[row] = x[token] - log_z;
-    out_ncand[row] = ncand;
-  }
-
-  // log-probabilities of the highest candidates
-  int n_lp = n_logprobs ? n_logprobs[row] : 0;
-  n_lp = min(min(n_lp, ncand), min(MAX_LOGPROBS, lp_stride));
-  if (n_lp > 0) {
-    __syncthreads();
-    const uint32_t key_n = select_kth(x, V, (uint32_t)n_lp, s);
-    if (tid == 0) s.list_n = 0;
-    __syncthreads();
-    for (int j = tid; j < V; j += THREADS) {
-      const float v = x[j];
-      if (to_key(v) >= key_n) {
-        const int slot = atomicAdd(&s.list_n, 1);
-        if (slot < LIST_MAX) { s.list_val[slot] = v; s.list_idx[slot] = j; }
-      }
-    }
-    __syncthreads();
-    const int n_list = min(s.list_n, LIST_MAX);
-    if (tid < n_list) {
-      const float v = s.list_val[tid];
-      const int id = s.list_idx[tid];
-      int rank = 0;
-      for (int o = 0; o < n_list; ++o) {
-        const float ov = s.list_val[o];
-        const int oi = s.list_idx[o];
-        if (ov > v || (ov == v && oi < id)) ++rank;
-      }
-      if (rank < n_lp) {
-        out_top_lp[(int64_t)row * lp_stride + rank] = v - log_z;
-        out_top_id[(int64_t)row * lp_stride + rank] = id;
-      }
     }
   }
 }
@@ -353,11 +577,13 @@ sample_kernel(const float* __restrict__ logits, int64_t row_stride, int V, const
 // SM's port takes longer than the rest of a decode step's tail): each block takes a stretch of the
 // row, pushes its (maximum, index) into every block's shared memory, and after one cluster barrier
 // rank 0 picks the winner (the lowest index among equal maxima, as a single block would).
+constexpr int THREADS = 1024;
 constexpr int ARGMAX_CLUSTER = 8;
 __global__ void __launch_bounds__(THREADS)
 argmax_kernel(const float* __restrict__ logits, int64_t row_stride, int V, int* __restrict__ out_token,
               const int* __restrict__ out_index) {
-  __shared__ Smem s;
+  __shared__ float warp_v[THREADS / 32];
+  __shared__ int warp_i[THREADS / 32];
   __shared__ float peer_v[ARGMAX_CLUSTER];
   __shared__ int peer_i[ARGMAX_CLUSTER];
   pdl_trigger();
@@ -376,7 +602,7 @@ argmax_kernel(const float* __restrict__ logits, int64_t row_stride, int V, int* 
     if (v > vmax) { vmax = v; imax = j; }
   }
   int arg;
-  const float best = block_max_arg(vmax, imax, &arg, s);
+  const float best = block_max_arg<THREADS / 32>(vmax, imax, &arg, warp_v, warp_i);
   cluster_wait_started();
   if (threadIdx.x == 0) {
     *cluster.map_shared_rank(&peer_v[rank], 0) = best;
@@ -400,9 +626,27 @@ GLLM_API int gllm_sample(const float* logits, int64_t row_stride, int rows, int 
                          cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (V <= 0) return (int)cudaErrorInvalidValue;
-  return gllm_launch(sample_kernel, dim3(rows), dim3(THREADS), 0, stream, logits, row_stride, V, temperature, top_k,
-                     top_p, seed, counter, n_logprobs, lp_stride, out_token, out_logprob, out_ncand, out_top_lp,
-                     out_top_id, probs_out);
+  // 16,000 elements a block at 128,256: two blocks of 512 threads fit an SM.  Fewer blocks a row for small
+  // vocabularies, whose passes are short beside the barriers between the blocks.
+  const int ranks = V > 32768 ? 8 : (V > 8192 ? 4 : 2);
+  const int per = (((V + ranks - 1) / ranks) + 3) & ~3;
+  const int staged = (size_t)per * sizeof(float) <= (size_t)SAMPLE_STAGE_BYTES;
+  const int vectors = row_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+  const size_t smem = staged ? (size_t)per * sizeof(float) : 0;
+  const cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_STAGE_BYTES);
+  if (e != cudaSuccess) return (int)e;
+  // (rows lie along y, at most 65,535 a launch)
+  for (int r0 = 0; r0 < rows; r0 += 65535) {
+    const int nr = rows - r0 < 65535 ? rows - r0 : 65535;
+    auto at = [r0](auto* p, int64_t step) { return p ? p + r0 * step : p; };
+    const int rc = gllm_launch_cluster(
+        sample_kernel, dim3(ranks, nr), dim3(SAMPLE_THREADS), smem, stream, (unsigned)ranks, at(logits, row_stride),
+        row_stride, V, per, staged, vectors, at(temperature, 1), at(top_k, 1), at(top_p, 1), at(seed, 1),
+        at(counter, 1), at(n_logprobs, 1), lp_stride, at(out_token, 1), at(out_logprob, 1), at(out_ncand, 1),
+        at(out_top_lp, lp_stride), at(out_top_id, lp_stride), at(probs_out, V));
+    if (rc != 0) return rc;
+  }
+  return 0;
 }
 
 // out_index (optional): row r's result goes to out_token[out_index[r]] instead of out_token[r].

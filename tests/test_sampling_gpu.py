@@ -120,3 +120,67 @@ def test_equal_logits_are_kept_or_dropped_together():
     # softmax .78 .105 .105 .04: top_p .9 is crossed inside the tie, so both tied values go
     out = ops.sample(logits.cuda(), **_args(1, 1.0, 0, 0.9), return_probs=True)
     assert int(out["num_candidates"][0]) == 1 and float(out["probs"][0, 3]) == 1.0
+
+
+def _rows_for(vocab, kind):
+    g = torch.Generator().manual_seed(7)
+    logits = 2.0 * torch.randn(4, vocab, generator=g)
+    if kind == "sorted":            # the largest values side by side: more candidates in one block than a list holds
+        logits = logits.sort(-1, descending=True).values
+    elif kind == "ties":            # a handful of distinct values
+        logits = logits.round()
+    elif kind == "masked":          # most of the vocabulary closed
+        logits[:, vocab // 7 + 1:] = float("-inf")
+    return logits
+
+
+@pytest.mark.parametrize("vocab", [1, 5, 130, 8192, 8193, 32769, 128256, 400003])
+@pytest.mark.parametrize("kind", ["plain", "sorted", "ties", "masked"])
+@pytest.mark.parametrize("top_k,top_p", [(0, 0.9), (0, 1.0), (40, 0.9), (64, 1.0), (129, 0.8), (300, 1.0)])
+def test_cuts_at_the_edges_of_the_row_split(vocab, kind, top_k, top_p):
+    """The kept set, the draw within it and the log-probabilities, over vocabularies on both sides of the rules that cut
+    a row (blocks per row, staging, unaligned rows) and rows whose candidates do not fit the short list.  The expected
+    mass of a kept set is summed in 64 bits; a cut may fall either way only where that mass is within 1e-5 of top_p."""
+    from gllm_b200 import ops
+
+    logits = _rows_for(vocab, kind)
+    wide = torch.zeros(4, vocab + 3, device="cuda")             # rows off the 16-byte grid
+    wide[:, :vocab] = logits.cuda()
+    args = _args(4, 0.8, top_k, top_p, nlp=7)
+    out = ops.sample(wide[:, :vocab], **args, max_logprobs=8, return_probs=True)
+    flat = ops.sample(logits.cuda(), **args, max_logprobs=8)
+    z = logits.double()
+    lp = torch.log_softmax(z, -1)
+    for r in range(4):
+        if top_k == 1 or vocab == 1:
+            keep = z[r] == z[r].max()
+        else:
+            k = vocab if top_k == 0 else min(top_k, vocab)
+            kth = z[r].topk(k).values[-1]
+            p = torch.softmax(torch.where(z[r] >= kth, z[r], torch.tensor(float("-inf"), dtype=z.dtype)) / 0.8, -1)
+            order = p.argsort(descending=True, stable=True)
+            mass = p[order].cumsum(0)
+            at_or_above = torch.empty_like(p)
+            last = (z[r][order][:, None] == z[r][order][None]).long() if vocab < 200 else None
+            if last is not None:
+                end = last.shape[1] - 1 - last.flip(1).argmax(1)
+            else:
+                values, inverse, counts = torch.unique(-z[r][order], return_inverse=True, return_counts=True)
+                end = counts.cumsum(0)[inverse] - 1
+            at_or_above[order] = mass[end]
+            keep = (z[r] >= kth) & ((at_or_above <= top_p) | (z[r] == z[r].max()) | (top_p == 1.0))
+            if top_p < 1.0 and bool(((at_or_above - top_p).abs() < 1e-5).any()):
+                continue
+        got = out["probs"][r].cpu() > 0
+        weight = torch.softmax(torch.where(keep, z[r], torch.tensor(float("-inf"), dtype=z.dtype)) / 0.8, -1)
+        seen = weight > 1e-30                                   # (a kept element may weigh nothing in 32 bits)
+        assert torch.equal(got & seen, keep & seen), (int(got.sum()), int(keep.sum()))
+        assert int(out["num_candidates"][r]) == int(keep.sum())
+        torch.testing.assert_close(out["probs"][r].double().cpu(), weight, rtol=2e-4, atol=1e-7)
+        token = int(out["tokens"][r])
+        assert bool(keep[token]) and int(flat["tokens"][r]) == token
+        assert abs(float(out["logprobs"][r]) - float(lp[r, token])) < 1e-4 * max(1.0, abs(float(lp[r, token])))
+        n = min(7, int(keep.sum()))
+        best = torch.sort(lp[r], descending=True, stable=True)
+        assert out["top_ids"][r, :n].tolist() == best.indices[:n].tolist()
+        torch.testing.assert_close(out["top_logprobs"][r, :n].double().cpu(), best.values[:n], rtol=1e-4, atol=1e-4)
