@@ -1,14 +1,21 @@
 // True 32-bit matrix product on the CUDA cores: C[M,N] = A[M,K] * B[N,K]^T,
 // the `x @ W.T` of gllm/model/layers/linear.py:20 with W stored [out, in].
 //
-// No tensor-core mode of any kind (no TF32): every product is an FFMA.  Each
-// output element is accumulated by one thread over k = 0..K-1 in ascending
-// order whatever M is, so a token's result does not depend on the batch it is
-// in.  This is the reference path that shows faults bf16 hides.  Two kernels:
-// a 128 x 128 tile with 8 x 8 outputs per thread, 16-byte global loads and the
-// next tile's loads in flight while this one is multiplied (rows 16-byte
-// aligned, K a multiple of 4), and a plain 64 x 64 tile for everything else
-// and for steps of few tokens, where the weight's trip from memory is the time.
+// No tensor-core mode of any kind (no TF32): every product is a 32-bit fused
+// multiply-add.  Each output element is accumulated by one thread in an order
+// that does not depend on M, so a token's result does not depend on the batch
+// it is in.  This is the reference path that shows faults bf16 hides.  Two
+// kernels: tiles of 16 x 16 to 64 x 64 outputs on packed multiply-adds with
+// asynchronous copies (rows 16-byte aligned, K a multiple of 4), and a plain
+// 64 x 64 tile for everything else (k = 0..K-1 in ascending order).
+//
+// What bounds the packed kernel: the multiply-add pipe (74 TFLOP/s at 128 a
+// clock and SM; a loop of nothing but packed multiply-adds reaches 105 a
+// clock) and the shared-memory loads that feed it.  2,048 x 8,192 x 2,048:
+// 1,413 us = 48.6 TFLOP/s, 1,909 us = 36.0 with a 128 x 128 tile of scalar
+// multiply-adds and one k-tile in flight; 700 x 2,048 x 8,192: 626 against
+// 1,097 us; 8 x 16,384 x 2,048: 64 against 381.  Error against 64 bits at
+// K = 2,048: 5.7e-7 (two partial sums) against 8.1e-7.
 #include "common.cuh"
 
 namespace {
@@ -68,84 +75,140 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
   }
 }
 
-// ---- 128 x 128 x 16 tile, 256 threads, 8 x 8 outputs per thread (as 2 x 2 blocks of 4 x 4, 64 apart, so
-// that a warp's shared-memory reads are 16-byte vectors without bank conflicts)
-constexpr int WM = 128, WN = 128, WK = 16;
+// ---- tiles whose rows lie in shared memory as they do in memory, [row][k], filled by cp.async several k-tiles ahead.
+// A thread owns TM x TN outputs (rows and columns TY and TX apart).  Four k at a time it reads 16 bytes of each of its
+// rows and multiplies them as two packed pairs (fma.rn.f32x2), so an output is kept as two sums, of the products with
+// even and with odd k, each in ascending order; they are added at the end.
+constexpr int PK = 32, PITCH = PK + 4;   // (a pitch of 9 sixteen-byte pieces: eight neighbouring rows on eight bank groups)
 
-__global__ void __launch_bounds__(256)
-gemm_f32_wide_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M, int N,
-                     int K, int64_t lda, int64_t ldb, int64_t ldc) {
-  __shared__ __align__(16) float As[WK][WM];
-  __shared__ __align__(16) float Bs[WK][WN];
+__device__ __forceinline__ void fma2(unsigned long long& c, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+
+template <int BM_, int BN_, int TM_, int TN_, int STAGES, int UNROLL>
+__global__ void __launch_bounds__((BM_ / TM_) * (BN_ / TN_))
+gemm_f32_pairs_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M, int N,
+                      int K, int64_t lda, int64_t ldb, int64_t ldc) {
+  constexpr int TY = BM_ / TM_, TX = BN_ / TN_, THREADS = TX * TY, ROWS = BM_ + BN_;
+  static_assert(TX % 8 == 0 && TY % 4 == 0, "a warp's threads lie 4 by 8");
+  extern __shared__ __align__(16) float tiles[];          // [STAGES][BM_ + BN_][PITCH]
   pdl_trigger();
+  // A warp's threads lie 4 rows by 8 columns, a half warp 4 by 4: a 16-byte load is served a half warp at a time when
+  // its addresses fit one pass over the banks, so neither operand's load takes more than two.
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tx = (warp % (TX / 8)) * 8 + (lane & 3) + (lane >> 4) * 4, ty = (warp / (TX / 8)) * 4 + ((lane >> 2) & 3);
+  const int m0 = blockIdx.y * BM_, n0 = blockIdx.x * BN_;
+  // a thread copies piece `piece` of the rows row0, row0 + STEP, ...: of A's first, of B's behind them
+  constexpr int PIECES = PK / 4, STEP = THREADS / PIECES, COPIES = ROWS / STEP;
+  static_assert(THREADS % PIECES == 0 && BM_ % STEP == 0 && BN_ % STEP == 0, "whole rows per round of copies");
+  const int piece = tid % PIECES, row0 = tid / PIECES;
+  const float* a_src = A + (int64_t)(m0 + row0) * lda + piece * 4;
+  const float* b_src = B + (int64_t)(n0 + row0) * ldb + piece * 4;
+  const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(tiles) + (uint32_t)((row0 * PITCH + piece * 4) * sizeof(float));
+  auto request = [&](int k0, int stage) {
+    const bool k_in = k0 + piece * 4 < K;
+    const uint32_t dst = dst0 + (uint32_t)(stage * ROWS * PITCH * sizeof(float));
+#pragma unroll
+    for (int c = 0; c < COPIES; ++c) {
+      const bool is_a = c < BM_ / STEP;
+      const int r = is_a ? c * STEP : c * STEP - BM_;
+      const bool in = k_in && (is_a ? m0 + row0 + r < M : n0 + row0 + r < N);
+      const float* src = is_a ? a_src + k0 + r * lda : b_src + k0 + r * ldb;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)(c * STEP * PITCH * sizeof(float))),
+                   "l"(in ? src : A), "r"(in ? 16 : 0) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  unsigned long long acc[TM_][TN_];
+#pragma unroll
+  for (int i = 0; i < TM_; ++i)
+#pragma unroll
+    for (int j = 0; j < TN_; ++j) acc[i][j] = 0ull;
+  const int k_tiles = (K + PK - 1) / PK;
   pdl_wait();
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * WM, n0 = blockIdx.x * WN;
-  float acc[8][8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-  // a thread loads two 16-byte pieces of A and two of B per k-tile: rows lrow and lrow + 64, columns lk .. lk + 3
-  const int lrow = tid >> 2, lk = (tid & 3) * 4;
-  float4 ra[2], rb[2];
-  auto load_tile = [&](int k0) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int am = m0 + lrow + h * 64, bn = n0 + lrow + h * 64, k = k0 + lk;
-      ra[h] = (am < M && k < K) ? *reinterpret_cast<const float4*>(A + (int64_t)am * lda + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-      rb[h] = (bn < N && k < K) ? *reinterpret_cast<const float4*>(B + (int64_t)bn * ldb + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  };
-  auto store_tile = [&]() {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = lrow + h * 64;
-      As[lk + 0][r] = ra[h].x; As[lk + 1][r] = ra[h].y; As[lk + 2][r] = ra[h].z; As[lk + 3][r] = ra[h].w;
-      Bs[lk + 0][r] = rb[h].x; Bs[lk + 1][r] = rb[h].y; Bs[lk + 2][r] = rb[h].z; Bs[lk + 3][r] = rb[h].w;
-    }
-  };
-  load_tile(0);
-  for (int k0 = 0; k0 < K; k0 += WK) {
-    store_tile();
-    __syncthreads();
-    if (k0 + WK < K) load_tile(k0 + WK);               // in flight while this tile is multiplied
-#pragma unroll
-    for (int kk = 0; kk < WK; ++kk) {
-      float a[8], b[8];
-      const float4 a0 = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&As[kk][64 + ty * 4]);
-      const float4 b0 = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&Bs[kk][64 + tx * 4]);
-      a[0] = a0.x; a[1] = a0.y; a[2] = a0.z; a[3] = a0.w; a[4] = a1.x; a[5] = a1.y; a[6] = a1.z; a[7] = a1.w;
-      b[0] = b0.x; b[1] = b0.y; b[2] = b0.z; b[3] = b0.w; b[4] = b1.x; b[5] = b1.y; b[6] = b1.z; b[7] = b1.w;
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
+  for (int t = 0; t < STAGES - 1; ++t) {
+    if (t < k_tiles) request(t * PK, t);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
   }
+  int stage = 0;
+  for (int t = 0; t < k_tiles; ++t) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();                                       // tile t is there, and nobody reads tile t - 1 any more
+    const int ahead = t + STAGES - 1;
+    if (ahead < k_tiles) request(ahead * PK, stage == 0 ? STAGES - 1 : stage - 1);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* a_s = tiles + (stage * ROWS + ty) * PITCH;
+    const float* b_s = tiles + (stage * ROWS + BM_ + tx) * PITCH;
+#pragma unroll UNROLL
+    for (int kk = 0; kk < PK; kk += 4) {
+      ulonglong2 a[TM_];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
+      for (int i = 0; i < TM_; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(a_s + i * TY * PITCH + kk);
+#pragma unroll
+      for (int j = 0; j < TN_; ++j) {
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(b_s + j * TX * PITCH + kk);
+#pragma unroll
+        for (int i = 0; i < TM_; ++i) fma2(acc[i][j], a[i].x, b.x);
+#pragma unroll
+        for (int i = 0; i < TM_; ++i) fma2(acc[i][j], a[i].y, b.y);
+      }
+    }
+    stage = stage + 1 == STAGES ? 0 : stage + 1;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < TM_; ++i) {
+    const int m = m0 + ty + i * TY;
     if (m >= M) continue;
 #pragma unroll
-    for (int jh = 0; jh < 2; ++jh) {
-      const int n = n0 + jh * 64 + tx * 4;
-      float* dst = C + (int64_t)m * ldc + n;
-      if (n + 3 < N && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
-        *reinterpret_cast<float4*>(dst) = make_float4(acc[i][jh * 4], acc[i][jh * 4 + 1], acc[i][jh * 4 + 2], acc[i][jh * 4 + 3]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (n + j < N) dst[j] = acc[i][jh * 4 + j];
-      }
+    for (int j = 0; j < TN_; ++j) {
+      const int n = n0 + tx + j * TX;
+      if (n < N)
+        C[(int64_t)m * ldc + n] = __uint_as_float((uint32_t)acc[i][j]) + __uint_as_float((uint32_t)(acc[i][j] >> 32));
     }
   }
 }
+
+template <int BM_, int BN_, int TM_, int TN_, int STAGES, int UNROLL>
+int gemm_f32_pairs(const float* A, const float* B, float* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
+                   cudaStream_t stream) {
+  const dim3 grid((N + BN_ - 1) / BN_, (M + BM_ - 1) / BM_);
+  if (grid.y > 65535) return (int)cudaErrorInvalidValue;
+  constexpr size_t smem = sizeof(float) * STAGES * (BM_ + BN_) * PITCH;
+  auto kernel = gemm_f32_pairs_kernel<BM_, BN_, TM_, TN_, STAGES, UNROLL>;
+  // Blocks that start while the kernel before them drains land wherever a place frees first.  Asking for a share of an
+  // SM's shared memory that lets no SM take more than its even share of the blocks keeps them spread.
+  const int64_t per_sm = ((int64_t)grid.x * grid.y + gllm_sm_count() - 1) / gllm_sm_count();
+  const int64_t share = 228 * 1024 / per_sm - 1024;              // (1 KB of every block's share is the system's)
+  const size_t ask = share > (int64_t)smem ? (size_t)(share < 227 * 1024 ? share : 227 * 1024) : smem;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  if (e != cudaSuccess) return (int)e;
+  return gllm_launch(kernel, grid, dim3((BM_ / TM_) * (BN_ / TN_)), ask, stream, A, B, C, M, N, K, lda, ldb, ldc);
+}
 }  // namespace
+
+// Which tile: the one whose fullest SM ends first.  A tile's time per k is `chain` (ns) while it has an SM to itself and
+// `work` times the tiles of the SM once they fill it; tiles of two warps count in pairs (an SM has four schedulers).
+// Measured per tile at K = 8,192 and 148 SMs (one tile an SM; 10 and more): the larger a tile the less it reads per
+// product, the smaller the better it spreads.  Steps of up to 16 tokens take the smallest tile, which streams the
+// weight best (16,384 x 2,048: 64 us against 95 with 32 x 32).
+static int pairs_tile_of(int M, int N) {
+  struct Tile { int m, n, pairs; float chain, work; };
+  static const Tile tiles[] = {{16, 16, 1, 10.4f, 3.66f}, {32, 16, 1, 13.2f, 5.2f}, {32, 32, 1, 19.4f, 7.4f},
+                               {64, 32, 1, 30.f, 13.8f}, {64, 64, 0, 33.7f, 26.4f}, {64, 64, 1, 56.4f, 25.f}};
+  if (M <= 16) return 0;
+  int best = 0;
+  float best_time = 0.f;
+  for (int i = 0; i < 6; ++i) {
+    const Tile& t = tiles[i];
+    int64_t per_sm = ((int64_t)((M + t.m - 1) / t.m) * ((N + t.n - 1) / t.n) + gllm_sm_count() - 1) / gllm_sm_count();
+    if (t.pairs) per_sm = (per_sm + 1) & ~(int64_t)1;
+    const float work = t.work * (float)per_sm, time = work > t.chain ? work : t.chain;
+    if (i == 0 || time < best_time) best = i, best_time = time;
+  }
+  return best;
+}
 
 GLLM_API int gllm_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, int64_t lda,
                            int64_t ldb, int64_t ldc, cudaStream_t stream) {
@@ -153,10 +216,15 @@ GLLM_API int gllm_gemm_f32(const float* A, const float* B, float* C, int M, int 
   if (K <= 0) return (int)cudaErrorInvalidValue;
   const bool vectors = K % 4 == 0 && lda % 4 == 0 && ldb % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 &&
                        (reinterpret_cast<uintptr_t>(B) & 15) == 0;
-  if (vectors && M > 64) {
-    dim3 wide((N + WN - 1) / WN, (M + WM - 1) / WM);
-    if (wide.y > 65535) return (int)cudaErrorInvalidValue;
-    return gllm_launch(gemm_f32_wide_kernel, wide, dim3(256), 0, stream, A, B, C, M, N, K, lda, ldb, ldc);
+  if (vectors) {
+    switch (pairs_tile_of(M, N)) {
+      case 0: return gemm_f32_pairs<16, 16, 2, 2, 6, 8>(A, B, C, M, N, K, lda, ldb, ldc, stream);
+      case 1: return gemm_f32_pairs<32, 16, 4, 2, 6, 8>(A, B, C, M, N, K, lda, ldb, ldc, stream);
+      case 2: return gemm_f32_pairs<32, 32, 4, 4, 4, 8>(A, B, C, M, N, K, lda, ldb, ldc, stream);
+      case 3: return gemm_f32_pairs<64, 32, 8, 4, 4, 8>(A, B, C, M, N, K, lda, ldb, ldc, stream);
+      case 4: return gemm_f32_pairs<64, 64, 8, 4, 3, 8>(A, B, C, M, N, K, lda, ldb, ldc, stream);
+      default: return gemm_f32_pairs<64, 64, 8, 8, 3, 1>(A, B, C, M, N, K, lda, ldb, ldc, stream);
+    }
   }
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   if (grid.y > 65535) return (int)cudaErrorInvalidValue;

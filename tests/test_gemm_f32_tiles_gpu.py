@@ -1,0 +1,24 @@
+"""Every tile the 32-bit product chooses from, at sizes that end inside one: rows, columns and k."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n", [(1, 17), (16, 2050), (33, 2050), (65, 2047), (100, 2050), (250, 2050), (350, 3073),
+                                 (500, 2046), (712, 3070), (1030, 4100)])
+@pytest.mark.parametrize("k", [4, 100, 1028])
+def test_every_tile_ends_where_the_matrix_does(m, n, k):
+    from gllm_b200 import ops
+
+    g = torch.Generator().manual_seed(m + n + k)
+    wide = torch.randn(m, k + 8, generator=g).cuda()
+    a, b = wide[:, 4:4 + k], torch.randn(n, k, generator=g).cuda()      # rows of a wider matrix
+    got = ops.linear(a, b)
+    want = a.double() @ b.double().T
+    # two sums of k / 2 products each: at most (k / 2 + 1) * 2^-24 times the sum of the products' magnitudes
+    bound = (k / 2 + 1) * 2.0 ** -24 * (a.double().abs() @ b.double().abs().T)
+    assert bool(((got.double() - want).abs() <= bound + 1e-30).all())
+    # a row's result does not depend on the rest of the batch, whichever tile the batch took
+    assert torch.equal(ops.linear(a[m - 1:m].contiguous(), b)[0], got[m - 1])
