@@ -1,7 +1,8 @@
 // Causal attention over the paged cache on the CUDA cores, for any head size
 // up to 256 and any number of heads and groups.
-// It is the whole attention of the 32-bit path and the fallback of the bf16
-// path for head sizes its tensor-core kernels do not take.
+// It serves the head sizes that the tiled kernels of the 32-bit path
+// (attention_f32.cu) and the tensor-core kernels of the bf16 path do not take,
+// and calls that bring no description of their batch.
 //
 // It replaces the gather of the padded context plus the dense
 // softmax(QK^T / sqrt(D) + bias) V of the reference

@@ -210,6 +210,8 @@ def modules_for(dtype: torch.dtype, head_dims=(), sampling: bool = False, module
         names = ["elementwise", "gemm_fp32"]
         if head_dims:
             names.append("attention_simt")
+        if any(d in (32, 64, 128) for d in head_dims):
+            names.append("attention_f32")
     else:
         names = ["elementwise", "gemm_bf16", "gemm_bf16_pair"]
         if head_dims:
@@ -1038,6 +1040,12 @@ def paged_attention(
         if attention_bf16.supports(d, block_size) and batch is not None:
             return attention_bf16.paged_attention_bf16(qkv, cache_layer, block_table, positions, token_row,
                                                        num_heads, scale, win, batch, out)
+    elif batch is not None:
+        from gllm_b200.ops import attention_f32
+
+        if attention_f32.takes(qkv, cache_layer, num_heads, batch, out):
+            return attention_f32.paged_attention_f32(qkv, cache_layer, block_table, positions, token_row, num_heads,
+                                                     scale, win, batch, out)
     return paged_attention_simt(qkv, qkv.shape[1], cache_layer, block_table, positions, token_row, num_heads,
                                 scale, win, out)
 

@@ -1,0 +1,73 @@
+"""Attention of the 32-bit path over the paged cache (``csrc/attention_f32.cu``): a tiled kernel for portions of
+prompts, a split-KV kernel for the single tokens behind them in the flat batch.  Head sizes 32, 64 and 128, 16-byte
+aligned rows; anything else runs the warp-per-token kernel (``ops.paged_attention_simt``)."""
+
+from __future__ import annotations
+
+from ctypes import c_float, c_int, c_int64, c_void_p
+
+import torch
+
+from gllm_b200.ops.build import load_module
+
+P = c_void_p
+HEAD_DIMS = (32, 64, 128)
+MAX_GROUP = 64                     # query heads per kv head that a tile of rows holds
+_fns = None
+
+
+def _functions():
+    global _fns
+    if _fns is None:
+        lib = load_module("attention_f32")
+        portions, singles, chunk = (lib.gllm_attention_f32_portions, lib.gllm_attention_f32_singles,
+                                    lib.gllm_attention_f32_chunk)
+        portions.argtypes = [P, c_int64, P, c_int64, P, P, c_int, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int,
+                             c_int, c_float, c_int, P, P]
+        singles.argtypes = [P, c_int64, P, c_int64, P, P, c_int, P, P, c_int, P, P, c_int, c_int, c_int, c_int, c_int,
+                            c_int, c_float, c_int, P, P]
+        for f in (portions, singles, chunk):
+            f.restype = c_int
+        chunk.argtypes = []
+        _fns = portions, singles, int(chunk())
+    return _fns
+
+
+def takes(qkv: torch.Tensor, cache_layer: torch.Tensor, num_heads: int, batch, out: torch.Tensor) -> bool:
+    d, hkv = cache_layer.shape[4], cache_layer.shape[2]
+    return (d in HEAD_DIMS and num_heads // hkv <= MAX_GROUP and qkv.data_ptr() % 16 == 0 and qkv.stride(0) % 4 == 0
+            and cache_layer.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0 and out.stride(0) % 4 == 0
+            and max(batch.num_prefill_requests, qkv.shape[0] - batch.num_prefill_tokens) <= 65535)
+
+
+def paged_attention_f32(qkv, cache_layer, block_table, positions, token_row, num_heads, scale, window, batch, out):
+    from gllm_b200 import ops
+    from gllm_b200.ops.attention_bf16 import visible_spans
+
+    portions, singles, chunk = _functions()
+    num_pages, _, hkv, block_size, d = cache_layer.shape
+    n, n_pf = qkv.shape[0], batch.num_prefill_tokens
+    status, stream = ops.status_word(qkv.device).data_ptr(), ops._stream()
+    if n_pf > 0:
+        ops._check(portions(
+            qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), cache_layer.data_ptr(), block_table.data_ptr(),
+            block_table.stride(0), batch.cu_q.data_ptr(), batch.context_lens.data_ptr(), batch.state_slots.data_ptr(),
+            batch.num_prefill_requests, batch.max_q_len, num_heads, hkv, d, block_size, num_pages, float(scale),
+            int(window), status, stream), "attention_f32_portions")
+    if n_pf < n:
+        rest, chunks = n - n_pf, visible_spans(batch.max_seq_len, chunk, int(window))
+        n_o, n_ml = rest * num_heads * chunks * d, rest * num_heads * chunks * 2
+        if batch.workspace is not None:
+            part_o = batch.workspace.get("attention_decode_partial_out", n_o, torch.float32)
+            part_ml = batch.workspace.get("attention_decode_partial_max_sum", n_ml, torch.float32)
+        else:
+            part_o = torch.empty(n_o, dtype=torch.float32, device=qkv.device)
+            part_ml = torch.empty(n_ml, dtype=torch.float32, device=qkv.device)
+        q, o = qkv[n_pf:], out[n_pf:]
+        ops._check(singles(
+            q.data_ptr(), q.stride(0), o.data_ptr(), o.stride(0), cache_layer.data_ptr(), block_table.data_ptr(),
+            block_table.stride(0), positions[n_pf:].data_ptr(), token_row[n_pf:].data_ptr(), rest, part_o.data_ptr(),
+            part_ml.data_ptr(), num_heads, hkv, d, block_size, num_pages, chunks, float(scale), int(window), status,
+            stream), "attention_f32_singles")
+        ops.launch_count += 1      # two kernels: chunks and merge
+    return out

@@ -41,6 +41,7 @@ MODULES = {
     "elementwise": "elementwise.cu",
     "gemm_fp32": "gemm_fp32.cu",
     "attention_simt": "attention_simt.cu",
+    "attention_f32": "attention_f32.cu",
     "sampling": "sampling.cu",
     "gemm_bf16": "gemm_bf16.cu",
     "gemm_bf16_pair": "gemm_bf16_pair.cu",

@@ -1,0 +1,56 @@
+"""The 32-bit path's tiled attention and its split-KV form for single tokens, at the edges of tiles, chunks and groups."""
+
+import math
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from test_kernels_gpu import _paged_case, _plain_attn
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("hq,hkv,d,bs,window", [
+    (4, 1, 64, 16, None), (32, 8, 64, 16, None), (3, 1, 32, 8, None), (6, 2, 128, 32, 100), (12, 1, 64, 4, 70),
+    (40, 2, 32, 16, 64), (7, 7, 128, 8, None), (64, 1, 64, 16, 129), (5, 5, 64, 16, 1),
+])
+@pytest.mark.parametrize("q_counts", [(64, 17, 2), (15, 200, 3), (129, 65, 64)])
+def test_portions_and_single_tokens(hq, hkv, d, bs, window, q_counts):
+    from gllm_b200 import ops
+    from gllm_b200.engine.step import Workspace
+    from gllm_b200.ops import attention_f32
+
+    g = torch.Generator().manual_seed(hq + d)
+    lens, counts = [64, 517, 130, 1, 128, 129, 700], list(q_counts) + [1] * 4
+    lens = [max(n, c) for n, c in zip(lens, counts)]
+    pool, table, ks, vs, qs, pos, rows = _paged_case(g, torch.float32, lens, hq, hkv, d, bs, counts)
+    if window:                                              # pages that no query of this step needs are given back
+        for r, (n, c) in enumerate(zip(lens, counts)):
+            table[r + 1, :max(0, n - c - window + 1) // bs] = -1
+    n, n_pf = pos.numel(), sum(q_counts)
+    qkv = torch.zeros(n, (hq + 2 * hkv) * d)
+    qkv[:, : hq * d] = torch.cat(qs).reshape(n, hq * d)
+    batch = SimpleNamespace(
+        num_prefill_tokens=n_pf, num_prefill_requests=3, max_seq_len=max(lens), max_q_len=max(counts),
+        workspace=Workspace(torch.device("cuda")),
+        cu_q=torch.tensor([0] + counts).cumsum(0).to(torch.int32).cuda(),
+        context_lens=torch.tensor([a - b for a, b in zip(lens, counts)], dtype=torch.int32).cuda(),
+        state_slots=torch.arange(1, len(lens) + 1, dtype=torch.int32).cuda(),
+    )
+    scale = 1.0 / math.sqrt(d)
+    args = (pool.cuda(), table.cuda(), pos.cuda(), rows.cuda(), hq, scale)
+    out = torch.full((n, hq * d), float("nan"), device="cuda")
+    assert attention_f32.takes(qkv.cuda(), args[0], hq, batch, out)
+    ops.paged_attention(qkv.cuda(), *args, window=window, batch=batch, out=out)
+    # the general kernel on the same operands, which it takes without the batch's description
+    general = ops.paged_attention(qkv.cuda(), *args, window=window)
+    ops.check_status()
+    off = 0
+    for r, nq in enumerate(counts):
+        want = _plain_attn(qs[r], ks[r], vs[r], pos[off:off + nq].long(), window, scale)
+        got = out[off:off + nq].double().cpu().view(nq, hq, d)
+        # scores of up to 3 * d in magnitude, rounded over d products: 1e-5 of it in the exponent
+        torch.testing.assert_close(got, want, rtol=1e-4, atol=1e-5)
+        torch.testing.assert_close(got, general[off:off + nq].double().cpu().view(nq, hq, d), rtol=1e-4, atol=1e-5)
+        off += nq
