@@ -9,7 +9,10 @@
 // start of the step and written back at its end, so a prompt may be cut anywhere.  States, decays,
 // gates, step sizes and every sum over a state are fp32 whatever the activations' type; the order of
 // the sums depends on nothing but the sizes of the model.
+#include <type_traits>
+
 #include "common.cuh"
+#include "state_space_chunks.cuh"
 
 namespace {
 
@@ -335,7 +338,7 @@ matrix_recurrence_kernel(int,
                          float* __restrict__ state,                       // [slots, heads, dvx, dk]
                          const int* __restrict__ cu_q, const int* __restrict__ state_slots,
                          float* __restrict__ out, int64_t out_stride,     // [n, heads * out_cols]
-                         int heads, int dk, int dv, int lanes, int tc, int kv_div) {
+                         int heads, int dk, int dv, int lanes, int tc, int kv_div, int below) {
   constexpr int PF = REC_LOOKAHEAD / THREADS;
   constexpr int mode = MODE;
   extern __shared__ __align__(16) float smem[];
@@ -350,6 +353,7 @@ matrix_recurrence_kernel(int,
   const int col = blockIdx.x * cols + cix;
   const int sub = threadIdx.x % lanes;
   const int start = cu_q[r], end = cu_q[r + 1];
+  if (end - start >= below) return;              // another kernel of the step takes the longer requests
   const int slot = state_slots[r];
   const bool live = col < dvx;
   // one buffer: q [tc][dkp], gate or key [tc][dkp], v [tc][cols], keep | take | exp(-m') [3][tc] (padded to 4)
@@ -836,6 +840,8 @@ int selective_scan_launch(const T* xc, const float* dt_raw, const float* dt_bias
                      state_slots, out, channels, n_state, taps, lanes, tc);
 }
 
+constexpr int CHUNK_MIN_TOKENS = 8;
+
 template <typename T>
 int matrix_recurrence_launch(int mode, const T* q, int64_t q_stride, const T* k, int64_t k_stride, const T* v,
                              int64_t v_stride, const float* gates, int64_t gates_stride, const float* gate_bias,
@@ -864,6 +870,19 @@ int matrix_recurrence_launch(int mode, const T* q, int64_t q_stride, const T* k,
                        dim3(REC_THREADS), 0, stream, mode, q, q_stride, k, k_stride, v, v_stride, gates, gates_stride,
                        gate_bias, lower, q_scale, state, cu_q, state_slots, out, out_stride, heads, dk, dv, lanes, kv_div);
   }
+  // Requests of eight tokens and more go through chunks of 64 on the tensor cores; shorter ones beside them (decoded
+  // tokens: their states' bytes are the work, which eight small blocks an SM move better than one large one) stay here.
+  int below = 0x7fffffff;
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+    if (mode == 2 && max_q_len >= CHUNK_MIN_TOKENS &&
+        ssd::takes(q, q_stride, k, k_stride, v, v_stride, state, out, out_stride, dk, dv)) {
+      const int rc = ssd::launch(q, q_stride, k, k_stride, v, v_stride, gates, gates_stride, gate_bias, lower, q_scale,
+                                 state, cu_q, state_slots, out, out_stride, num_requests, heads, dk, dv, kv_div,
+                                 num_requests == 1 ? 0 : CHUNK_MIN_TOKENS, stream);
+      if (rc != 0 || num_requests == 1) return rc;
+      below = CHUNK_MIN_TOKENS;
+    }
+  }
   int dpt = dk <= 128 ? 4 : 16;
   // the step-sized recurrence has many heads of many value columns: with 65 .. 256 key channels eight per thread
   // measured 1.2x faster than four (1.00 against 1.23 ms for 64 heads of 128 x 64 over 2,048 tokens); up to 64, four
@@ -882,7 +901,7 @@ int matrix_recurrence_launch(int mode, const T* q, int64_t q_stride, const T* k,
   if (tc * dkp > REC_LOOKAHEAD || tc * cols > REC_LOOKAHEAD) return (int)cudaErrorInvalidValue;
   const size_t smem = sizeof(float) * 2 * (size_t)tc * (2 * dkp + cols + 4);
   void (*kernel)(int, const T*, int64_t, const T*, int64_t, const T*, int64_t, const float*, int64_t, const float*,
-                 const float*, float, float*, const int*, const int*, float*, int64_t, int, int, int, int, int, int);
+                 const float*, float, float*, const int*, const int*, float*, int64_t, int, int, int, int, int, int, int);
 #define GLLM_REC_PICK(M)                                                                            \
   kernel = dpt == 4 ? matrix_recurrence_kernel<T, 4, REC_THREADS, M>                                \
                     : (dpt == 8 ? matrix_recurrence_kernel<T, 8, REC_THREADS, M> : matrix_recurrence_kernel<T, 16, REC_THREADS, M>)
@@ -896,7 +915,7 @@ int matrix_recurrence_launch(int mode, const T* q, int64_t q_stride, const T* k,
   }
   return gllm_launch(kernel, dim3((dvx + cols - 1) / cols, heads, num_requests), dim3(threads), smem, stream, mode, q,
                      q_stride, k, k_stride, v, v_stride, gates, gates_stride, gate_bias, lower, q_scale, state, cu_q,
-                     state_slots, out, out_stride, heads, dk, dv, lanes, tc, kv_div);
+                     state_slots, out, out_stride, heads, dk, dv, lanes, tc, kv_div, below);
 }
 
 template <typename T>

@@ -1,0 +1,64 @@
+"""The step-sized matrix recurrence in chunks: lengths at the chunk's edges, shorter requests beside longer ones, a
+prompt cut in two, shared and separate groups, slow and fast decays, against 64 bits and the token-by-token kernel."""
+
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,dk,dv,groups", [(2, 128, 64, 1), (4, 64, 32, 2), (3, 128, 96, 3)])
+@pytest.mark.parametrize("lens", [(8,), (63, 64), (65, 1, 7), (130, 2, 9, 200)])
+@pytest.mark.parametrize("speed", [0.01, 1.0, 40.0])
+def test_chunks_against_64_bits(heads, dk, dv, groups, lens, speed):
+    from gllm_b200.ops import stateful
+
+    g = torch.Generator().manual_seed(heads * dk + sum(lens))
+    n, R, hg, offset = sum(lens), len(lens), heads // groups, 8
+    wide = torch.randn(n, offset + heads * dv + 2 * groups * dk, generator=g).to(torch.bfloat16).cuda()
+    x = wide[:, offset:offset + heads * dv]
+    b, c = wide[:, offset + heads * dv:][:, :groups * dk], wide[:, offset + heads * dv + groups * dk:]
+    raw, bias = torch.randn(n, heads, generator=g).cuda(), torch.randn(heads, generator=g).cuda() - 3.0
+    A = -speed * (0.5 + torch.rand(heads, generator=g)).cuda()
+    slots = torch.randperm(R + 2, generator=g)[:R].to(torch.int32).cuda()
+    first = torch.randn(R + 2, heads, dv, dk, generator=g).cuda()
+
+    def run(state, cuts, offset):
+        cu = torch.tensor([0] + list(cuts)).cumsum(0).to(torch.int32).cuda()
+        rows = slice(offset, offset + sum(cuts))
+        return stateful.matrix_recurrence(
+            stateful.STEP_SIZED, c[rows], b[rows], x[rows], raw[rows], bias, A, 0.0, 0.5, state, None, cu,
+            slots[-len(cuts):].contiguous(), len(cuts), heads, dk, dv, max_q_len=max(cuts), heads_per_group=hg)
+
+    state = first.clone()
+    got = run(state, lens, 0).view(n, heads, dv)
+    dt = torch.nn.functional.softplus(raw.double() + bias.double())
+    decay = torch.exp(A.double() * dt)
+    B, C = (t.double().view(n, groups, dk).repeat_interleave(hg, 1) for t in (b, c))
+    X, want, after, at = x.double().reshape(n, heads, dv), torch.empty(n, heads, dv, dtype=torch.float64).cuda(), first.double(), 0
+    size, size_after = torch.zeros_like(want), first.double().abs()          # the same sums over magnitudes
+    for r, length in enumerate(lens):
+        s, m = after[slots[r].item()], size_after[slots[r].item()]
+        for t in range(at, at + length):
+            fed = (dt[t][:, None] * X[t])[..., None]
+            s = s * decay[t][:, None, None] + fed * B[t][:, None]
+            # (a request of fewer than 8 tokens walks them one by one and subtracts what the state loses from it: each
+            # step rounds at the old state's size, whatever is left of it)
+            m = m * (decay[t][:, None, None] if length >= 8 else 1.0) + fed.abs() * B[t][:, None].abs()
+            want[t], size[t] = 0.5 * (s @ C[t][..., None])[..., 0], 0.5 * (m @ C[t].abs()[..., None])[..., 0]
+        after[slots[r].item()], size_after[slots[r].item()] = s, m
+        at += length
+    # 32-bit sums: each term is rounded a handful of times and carries the roundings of one decay per chunk (64 times
+    # 2^-24 of the terms' magnitudes covers a sum over a chunk and 200 tokens' worth of state)
+    assert bool(((got.double() - want).abs() <= 64 * 2.0 ** -24 * size + 1e-30).all())
+    assert bool(((state.double() - after).abs() <= 64 * 2.0 ** -24 * size_after + 1e-30).all())
+    untouched = [i for i in range(R + 2) if i not in slots.tolist()]
+    assert torch.equal(state[untouched], first[untouched])
+    # the last request cut in two, its first part in a step of its own
+    last = lens[-1]
+    if last >= 16:
+        again, cut = first.clone(), last // 2 + 3
+        parts = [run(again, (cut,), n - last), run(again, (last - cut,), n - last + cut)]
+        torch.testing.assert_close(torch.cat(parts).view(last, heads, dv), got[n - last:], rtol=1e-4, atol=1e-4 * float(size.max()))
+        torch.testing.assert_close(again[slots[-1].item()], state[slots[-1].item()], rtol=1e-4, atol=1e-4 * float(size_after.max()))
