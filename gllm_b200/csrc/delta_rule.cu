@@ -18,6 +18,7 @@
 // The flat batch holds prompt portions beside single tokens: request r owns rows cu_q[r] .. cu_q[r+1]-1 and row
 // state_slots[r] of the state tensors, so a prompt may be cut anywhere.
 #include "common.cuh"
+#include "delta_chunks.cuh"
 
 namespace {
 
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(DELTA_THREADS)
 delta_rule_kernel(const float* __restrict__ qk, const float* __restrict__ v, const float* __restrict__ g,
                   const float* __restrict__ beta, float* __restrict__ state, const int* __restrict__ cu_q,
                   const int* __restrict__ state_slots, float* __restrict__ out, int heads, int kv_heads, int dk,
-                  int dv, int tc) {
+                  int dv, int tc, int below) {
   extern __shared__ __align__(16) float sm[];
   pdl_trigger();
   pdl_wait();
@@ -158,7 +159,7 @@ delta_rule_kernel(const float* __restrict__ qk, const float* __restrict__ v, con
   const int col0 = blockIdx.x * cols, col = col0 + cix;
   const bool live = col < dv;
   const int t0 = cu_q[r], t1 = cu_q[r + 1];
-  if (t1 <= t0) return;
+  if (t1 <= t0 || t1 - t0 >= below) return;                // (longer requests may be another kernel's)
   constexpr int gw = HEAD ? 1 : dkp;                       // decays of a token in shared memory
   // (a token's decay per head lies behind its beta)
   const int buf_floats = (tc * (2 * dkp + gw + cols + 1) + 3) & ~3;
@@ -341,12 +342,43 @@ int delta_prep_launch(const T* x, int64_t x_stride, const float* conv_w, float* 
                      x_stride, conv_state, cu_q, state_slots, channels, taps);
 }
 
+// Requests of CHUNK_FROM tokens and more go through chunks when a step's longest has CHUNK_LONGEST: the two kernels'
+// start and one chunk take 38 us, what 140 tokens take one by one.  Many requests at once fill the machine with the
+// token-by-token kernel too (its form of 32 channels a thread, from 240 blocks on): eight of 512 tokens, 16 heads of
+// 64 x 128, take it 268 us and the chunks 340; four of them 307 against 186, two 168 against 91.
+constexpr int CHUNK_LONGEST = 160, CHUNK_FROM = 16, MANY_BLOCKS = 240;
+
+// Floats of workspace with which delta_rule runs its longer requests in chunks; 0 when it walks every token anyway.
+// (A step whose records would pass a gigabyte is walked.)
+int64_t chunk_workspace(int n_tokens, int num_requests, int heads, int dk, int dv, int max_q_len) {
+  if (dk != delta_chunks::DK || dv % delta_chunks::COLS || max_q_len < CHUNK_LONGEST || num_requests > 65535) return 0;
+  const int64_t longer = std::max(1, std::min(num_requests, n_tokens / delta_chunks::L));
+  if (longer * heads * ((dv + 63) / 64) >= MANY_BLOCKS && num_requests > 1) return 0;
+  const int64_t floats = delta_chunks::workspace_floats(n_tokens, num_requests, heads, dv);
+  return floats <= (int64_t)1 << 28 ? floats : 0;
+}
+
 int delta_rule_launch(const float* qk, const float* v, const float* g, const float* beta, float* state,
                       const int* cu_q, const int* state_slots, float* out, int num_requests, int heads, int kv_heads,
-                      int dk, int dv, int max_q_len, int decay_width, cudaStream_t stream) {
+                      int dk, int dv, int max_q_len, int decay_width, float* workspace, int n_tokens,
+                      cudaStream_t stream) {
   if (num_requests <= 0) return 0;
   if ((decay_width != 1 && decay_width != dk) || heads > 65535 || num_requests > 65535 || dk < 1 || dv < 1 || dk > 512 || heads % kv_heads)
     return (int)cudaErrorInvalidValue;
+  // The longer requests go through chunks of 64 where the caller gave their records room; shorter ones beside them
+  // (decoded tokens) stay here.
+  int below = 0x7fffffff;
+  if (workspace != nullptr) {
+    if (chunk_workspace(n_tokens, num_requests, heads, dk, dv, max_q_len) == 0 ||
+        ((reinterpret_cast<uintptr_t>(qk) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(g) |
+          reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(workspace)) & 15) != 0)
+      return (int)cudaErrorInvalidValue;
+    const int from = num_requests == 1 ? 0 : CHUNK_FROM;
+    const int rc = delta_chunks::launch(qk, v, g, beta, state, cu_q, state_slots, out, workspace, n_tokens, num_requests,
+                                        heads, kv_heads, dv, decay_width == 1, from, stream);
+    if (rc != 0 || num_requests == 1) return rc;
+    below = from;
+  }
   // Key channels a thread keeps (DPT).  More of them mean fewer threads a column, so fewer rounds of shuffles and more
   // independent work per warp, but fewer warps in all.  Measured: four for heads of up to 64 key channels and eight
   // beyond when one prompt runs alone (every warp the step can have is wanted); eight when every request brings one
@@ -360,7 +392,7 @@ int delta_rule_launch(const float* qk, const float* v, const float* g, const flo
   if (vec) {
     dpt = dk <= 64 ? 4 : (dk <= 256 ? 8 : 16);
     if (dk <= 64 && max_q_len == 1) dpt = std::min(8, std::max(4, dk));
-    if (dk > 32 && dk <= 64 && max_q_len != 1 && (int64_t)((dv + 63) / 64) * heads * num_requests >= 240) dpt = 32;
+    if (dk > 32 && dk <= 64 && max_q_len != 1 && (int64_t)((dv + 63) / 64) * heads * num_requests >= MANY_BLOCKS) dpt = 32;
   }
   if (const char* e = getenv("GLLM_B200_DELTA_DPT")) {
     const int want = atoi(e);
@@ -374,7 +406,7 @@ int delta_rule_launch(const float* qk, const float* v, const float* g, const flo
   while (tc > 2 && 2 * tc * per_token * sizeof(float) > 96 * 1024) tc >>= 1;
   const size_t smem = sizeof(float) * 2 * (size_t)((tc * per_token + 3) & ~3);
   using Kernel = void (*)(const float*, const float*, const float*, const float*, float*, const int*, const int*, float*,
-                          int, int, int, int, int);
+                          int, int, int, int, int, int);
   Kernel kernel = nullptr;
 #define GLLM_DELTA_PICK(D, L) \
   if (dpt == D && lanes == L)                                                           \
@@ -410,7 +442,7 @@ int delta_rule_launch(const float* qk, const float* v, const float* g, const flo
     if (e != cudaSuccess) return (int)e;
   }
   return gllm_launch(kernel, dim3((dv + cols - 1) / cols, heads, num_requests), dim3(DELTA_THREADS), smem_ask, stream, qk, v,
-                     g, beta, state, cu_q, state_slots, out, heads, kv_heads, dk, dv, tc);
+                     g, beta, state, cu_q, state_slots, out, heads, kv_heads, dk, dv, tc, below);
 }
 }  // namespace
 
@@ -431,7 +463,12 @@ GLLM_DELTA_EXPORTS(__nv_bfloat16, bf16)
 
 GLLM_API int gllm_delta_rule(const float* qk, const float* v, const float* g, const float* beta, float* state,
                              const int* cu_q, const int* state_slots, float* out, int num_requests, int heads,
-                             int kv_heads, int dk, int dv, int max_q_len, int decay_width, cudaStream_t stream) {
+                             int kv_heads, int dk, int dv, int max_q_len, int decay_width, float* workspace,
+                             int n_tokens, cudaStream_t stream) {
   return delta_rule_launch(qk, v, g, beta, state, cu_q, state_slots, out, num_requests, heads, kv_heads, dk, dv, max_q_len,
-                           decay_width, stream);
+                           decay_width, workspace, n_tokens, stream);
+}
+// Floats of `workspace` that let gllm_delta_rule take a step's longer requests in chunks (0: it does not).
+GLLM_API int64_t gllm_delta_rule_workspace(int n_tokens, int num_requests, int heads, int dk, int dv, int max_q_len) {
+  return chunk_workspace(n_tokens, num_requests, heads, dk, dv, max_q_len);
 }

@@ -9,10 +9,12 @@ row ``state_slots[r]`` of every state tensor.  States are fp32 and are read and 
 from __future__ import annotations
 
 import os
+from ctypes import c_int, c_int64
 
 import torch
 
 from gllm_b200.ops import _check, _cuda, _fn, _ptr, _stream, _suffix, status_word
+from gllm_b200.ops.build import load_module
 
 # GLLM_B200_SIGMOID_MMA=0: the sigmoid attention of bf16 models stays on the CUDA-core kernel (for measurements)
 USE_TENSOR_CORES = os.environ.get("GLLM_B200_SIGMOID_MMA", "1") != "0"
@@ -333,11 +335,28 @@ def delta_rule(qk: torch.Tensor, v: torch.Tensor, g: torch.Tensor, beta: torch.T
         raise ValueError("the delta rule's operands do not fit together")
     decay_width = 1 if g.shape[1] == heads else dk
     out = torch.empty((n, heads * dv), dtype=torch.float32, device=qk.device)
+    # the records of the chunks that the longer requests are cut into (none: every token is walked)
+    floats = 0
+    if all(t.data_ptr() % 16 == 0 for t in (qk, v, g, state)):
+        floats = _delta_workspace()(n, int(num_requests), heads, dk, dv, int(max_q_len))
+    workspace = torch.empty(floats, dtype=torch.float32, device=qk.device) if floats else None
     f = _fn("delta_rule", "gllm_delta_rule")
     _check(f(qk.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(), state.data_ptr(), cu_q.data_ptr(),
              state_slots.data_ptr(), out.data_ptr(), int(num_requests), heads, kv_heads, dk, dv, int(max_q_len),
-             decay_width, _stream()), "delta_rule")
+             decay_width, _ptr(workspace), n, _stream()), "delta_rule")
     return out
+
+
+_workspace_floats = None
+
+
+def _delta_workspace():
+    global _workspace_floats
+    if _workspace_floats is None:
+        f = load_module("delta_rule").gllm_delta_rule_workspace
+        f.argtypes, f.restype = [c_int] * 6, c_int64
+        _workspace_floats = f
+    return _workspace_floats
 
 
 # ------------------------------------------------------------------ sigmoid attention

@@ -1,0 +1,75 @@
+"""The delta rule in chunks: lengths at the edges of chunks and of their blocks of sixteen, short requests beside long
+ones, a prompt cut in two, shared query and key heads, decays per channel and per head from almost none to all at once."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(g, n, heads, kv_heads, dk, dv, per_head, speed):
+    unit = lambda t: t / t.norm(dim=-1, keepdim=True)  # noqa: E731
+    q, k = (unit(torch.randn(n, kv_heads, dk, generator=g)) for _ in range(2))
+    qk = torch.cat([q.reshape(n, -1) * dk ** -0.5, k.reshape(n, -1)], 1).cuda()
+    v = torch.randn(n, heads * dv, generator=g).cuda()
+    rate = speed * torch.rand(heads * (1 if per_head else dk), generator=g)
+    loss = -torch.expm1(-rate * torch.rand(n, rate.numel(), generator=g)).cuda()
+    if n > 40:
+        loss[40] = 1.0                                   # everything forgotten at once
+    return qk, v, loss, torch.sigmoid(torch.randn(n, heads, generator=g)).cuda()
+
+
+def _exact(qk, v, loss, beta, state, slots, lens, heads, kv_heads, dk, dv):
+    """Token by token in 64 bits; returns the outputs (``state`` is updated)."""
+    n, share = qk.shape[0], heads // kv_heads
+    q, k = (t.double().view(n, kv_heads, dk).repeat_interleave(share, 1) for t in qk.chunk(2, 1))
+    keep = (1.0 - loss.double()).view(n, heads, -1).expand(-1, -1, dk)
+    out, at = torch.empty(n, heads, dv, dtype=torch.float64, device="cuda"), 0
+    for r, length in enumerate(lens):
+        s = state[slots[r]]
+        for t in range(at, at + length):
+            s = s * keep[t][:, None]
+            u = beta[t].double()[:, None] * (v[t].double().view(heads, dv) - (s @ k[t][..., None])[..., 0])
+            s = s + u[..., None] * k[t][:, None]
+            out[t] = (s @ q[t][..., None])[..., 0]
+        state[slots[r]] = s
+        at += length
+    return out
+
+
+@pytest.mark.parametrize("heads,kv_heads,dv", [(2, 2, 128), (4, 2, 16), (3, 1, 80)])
+@pytest.mark.parametrize("lens", [(160,), (63, 192), (165, 1, 7), (130, 2, 33, 200), (15, 181, 48)])
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("speed", [0.002, 0.3, 30.0])
+def test_chunks_against_64_bits(heads, kv_heads, dv, lens, per_head, speed):
+    from gllm_b200.ops import stateful
+
+    g = torch.Generator().manual_seed(heads * dv + sum(lens))
+    n, R, dk = sum(lens), len(lens), 64
+    qk, v, loss, beta = _inputs(g, n, heads, kv_heads, dk, dv, per_head, speed)
+    slots = torch.randperm(R + 2, generator=g)[:R].tolist()
+    first = torch.randn(R + 2, heads, dv, dk, generator=g).cuda()
+
+    def run(state, cuts, at, slots):
+        cu = torch.tensor([0] + list(cuts)).cumsum(0).to(torch.int32).cuda()
+        rows = slice(at, at + sum(cuts))
+        return stateful.delta_rule(qk[rows], v[rows], loss[rows], beta[rows].contiguous(), state, cu,
+                                   torch.tensor(slots, dtype=torch.int32).cuda(), len(cuts), heads, kv_heads, dk, dv,
+                                   max_q_len=max(cuts))
+
+    state, after = first.clone(), first.double()
+    got = run(state, lens, 0, slots).view(n, heads, dv)
+    want = _exact(qk, v, loss, beta, after, slots, lens, heads, kv_heads, dk, dv)
+    # the state and every write are of the size of v and the first state (one); a token's rounding is 2^-24 of that in
+    # each of 64 products, and the rule never lets an error grow: 64 * 2^-24 with a factor of two for the chunk's inverse
+    bound = 128 * 2.0 ** -24
+    assert float((got.double() - want).abs().max()) <= bound * float(first.abs().max())
+    assert float((state.double() - after).abs().max()) <= bound * float(first.abs().max())
+    untouched = [i for i in range(R + 2) if i not in slots]
+    assert torch.equal(state[untouched], first[untouched])
+    last = lens[-1]
+    if last >= 33:                                       # the last request in two steps
+        again, cut = first.clone(), last - 17
+        parts = [run(again, (cut,), n - last, slots[-1:]), run(again, (last - cut,), n - last + cut, slots[-1:])]
+        assert float((torch.cat(parts).view(last, heads, dv) - got[n - last:]).abs().max()) <= 2 * bound * float(first.abs().max())
+        assert float((again[slots[-1]] - state[slots[-1]]).abs().max()) <= 2 * bound * float(first.abs().max())
