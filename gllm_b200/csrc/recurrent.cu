@@ -1147,6 +1147,57 @@ head_norm_kernel(const float* __restrict__ o, int64_t o_stride, int o_cols, int 
   }
 }
 
+// The same without a denominator for heads on 16-byte boundaries: a lane keeps its columns, PIECES times four, between
+// the two passes.  What bounds it: the bytes.  2,019 tokens of 16 heads of 128, bfloat16: 11.5 us against 17.7.
+template <typename T, int PIECES>
+__global__ void __launch_bounds__(128)
+head_norm_wide_kernel(const float* __restrict__ o, int64_t o_stride, int o_cols, const float* __restrict__ w,
+                      int w_head_stride, const T* __restrict__ gate, int64_t gate_stride, int gate_silu,
+                      T* __restrict__ out, int64_t out_stride, int n_tokens, int heads, int dv, float eps) {
+  struct alignas(4 * sizeof(T)) Four { T v[4]; };
+  pdl_trigger();
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t item = (int64_t)blockIdx.x * 4 + warp;
+  if (item >= (int64_t)n_tokens * heads) return;
+  const int t = (int)(item / heads), h = (int)(item - (int64_t)t * heads);
+  const float* row = o + (int64_t)t * o_stride + (int64_t)h * o_cols;
+  float4 x[PIECES];
+  Four z[PIECES];
+  float ss = 0.f;
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    const int c = (lane + 32 * p) * 4;
+    if (c < dv) {
+      x[p] = *reinterpret_cast<const float4*>(row + c);
+      if (gate) z[p] = *reinterpret_cast<const Four*>(gate + (int64_t)t * gate_stride + (int64_t)h * dv + c);
+    }
+  }
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p)
+    if ((lane + 32 * p) * 4 < dv) ss = fmaf(x[p].x, x[p].x, fmaf(x[p].y, x[p].y, fmaf(x[p].z, x[p].z, fmaf(x[p].w, x[p].w, ss))));
+  ss = warp_sum(ss);
+  const float inv = 1.0f / sqrtf(ss / (float)dv + eps);
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    const int c = (lane + 32 * p) * 4;
+    if (c < dv) {
+      const float4 ws = *reinterpret_cast<const float4*>(w + (int64_t)h * w_head_stride + c);
+      float v[4] = {x[p].x * inv * ws.x, x[p].y * inv * ws.y, x[p].z * inv * ws.z, x[p].w * inv * ws.w};
+      Four r;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (gate) {
+          const float g = to_float(z[p].v[e]);
+          v[e] *= gate_silu ? siluf_(g) : sigmoidf_(g);
+        }
+        r.v[e] = from_float<T>(v[e]);
+      }
+      *reinterpret_cast<Four*>(out + (int64_t)t * out_stride + (int64_t)h * dv + c) = r;
+    }
+  }
+}
+
 // --------------------------------------------------------------- gated norm over groups of columns
 // One block per (token, group of `group_width` neighbouring columns):
 //     u[c] = (y[c] + skip[c / head_width] * x[c]) * silu(z[c])        (the skip term only with `skip`)
@@ -1409,6 +1460,14 @@ int head_norm_launch(const float* o, int64_t o_stride, int o_cols, int with_den,
   if (n_tokens <= 0) return 0;
   const int64_t blocks = ((int64_t)n_tokens * heads + 3) / 4;
   if (blocks > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
+  const uintptr_t activations = reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(out);
+  if (!with_den && dv % 4 == 0 && dv <= 512 && o_stride % 4 == 0 && o_cols % 4 == 0 && w_head_stride % 4 == 0 &&
+      gate_stride % 4 == 0 && out_stride % 4 == 0 && activations % (4 * sizeof(T)) == 0 &&
+      ((reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) {
+    auto kernel = dv <= 128 ? head_norm_wide_kernel<T, 1> : (dv <= 256 ? head_norm_wide_kernel<T, 2> : head_norm_wide_kernel<T, 4>);
+    return gllm_launch(kernel, dim3((unsigned)blocks), dim3(128), 0, stream, o, o_stride, o_cols, w, w_head_stride, gate,
+                       gate_stride, gate_silu, out, out_stride, n_tokens, heads, dv, eps);
+  }
   return gllm_launch(head_norm_kernel<T>, dim3((unsigned)blocks), dim3(128), 0, stream, o, o_stride, o_cols, with_den,
                      den_eps, w, w_head_stride, gate, gate_stride, gate_silu, out, out_stride, n_tokens, heads, dv, eps);
 }
