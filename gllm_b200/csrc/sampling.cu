@@ -74,13 +74,13 @@ __device__ float block_max_arg(float v, int idx, int* out_idx, float* sv, int* s
 //
 // What bounds it: the row's one trip from memory, then a chain of block-wide passes and cluster barriers.  The form
 // before this one, a block per row with nine passes over the row through L2 and histograms of floats in shared memory
-// (a compare-and-swap loop per element), took 270 us a call for 64 rows of 128,256 (top_k 40, top_p 0.9); this one takes 66 us.
+// (a compare-and-swap loop per element), took 270 us a call for 64 rows of 128,256 (top_k 40, top_p 0.9); this one takes 45 us.
 //
 // Threshold without a histogram: a block's stretch is cut into 64 groups (eight lanes of a warp each).  The K-th
-// largest of all groups' maxima has at least K elements at or above it, so it bounds the K-th largest element from
-// below, and only about K elements lie above it when the row is in no particular order.  Those are handed, in index
-// order, to block 0 of the cluster, which finds the exact K-th value, the top-p cut, the draw and the
-// log-probabilities among them.  K is limited to half the groups (the bound gets loose beyond) and the list to
+// largest of all groups' maxima has at least K elements at or above it, so it (and its sixteen leading bits) bounds the
+// K-th largest element from below, and only a few more than K elements lie above it when the row is in no particular
+// order.  Those are handed, in index order, to block 0 of the cluster, which finds the exact K-th value, the top-p cut, the
+// draw and the log-probabilities among them.  K is limited to half the groups (the bound gets loose beyond) and the list to
 // LIST_CAP entries a block; rows that do not fit (and top_k 0) take the search over digits instead: eight rounds of
 // sixteen bins, each bin's mass summed in registers in a fixed order, one exchange between the blocks a round.
 constexpr int SAMPLE_THREADS = 512;
@@ -117,6 +117,22 @@ struct Stretch {
   const float* x;      // the stretch (shared memory, or the row itself)
   int first;           // index of x[0] in the row
   int w0, w1;          // this warp's elements
+  bool quads;          // x[w0] lies on a 16-byte boundary, and whole steps of 128 may be read four elements a lane
+
+  // Calls f(j, value) for this warp's elements, a lane's in ascending order; every lane of the warp takes part.
+  template <typename F> __device__ __forceinline__ void each(F f) const {
+    const int lane = threadIdx.x & 31;
+    int j0 = w0;
+    if (quads) {
+#pragma unroll 2
+      for (; j0 + 128 <= w1; j0 += 128) {
+        const int j = j0 + lane * 4;
+        const float4 v = *reinterpret_cast<const float4*>(x + j);
+        f(j, v.x), f(j + 1, v.y), f(j + 2, v.z), f(j + 3, v.w);
+      }
+    }
+    for (int j = j0 + lane; j < w1; j += 32) f(j, x[j]);
+  }
 };
 
 // Mass of the sixteen values that digit `shift` of the key can take, over the elements whose key is at least `floor`
@@ -205,7 +221,7 @@ __device__ bool find_cut(const Stretch& s, cg::cluster_group& cluster, SampleSme
 __device__ void hand_over(const Stretch& s, cg::cluster_group& cluster, SampleSmem& sm, uint32_t floor) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rank = (int)cluster.block_rank();
   int mine = 0;
-  for (int j = s.w0 + lane; j < s.w1; j += 32) mine += to_key(s.x[j]) >= floor;
+  s.each([&](int, float v) { mine += to_key(v) >= floor; });
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
   __syncthreads();
@@ -220,7 +236,33 @@ __device__ void hand_over(const Stretch& s, cg::cluster_group& cluster, SampleSm
   if (mine > 0 && at < LIST_CAP) {
     float* list_v = cluster.map_shared_rank(sm.list_v, 0) + rank * LIST_CAP;
     int* list_i = cluster.map_shared_rank(sm.list_i, 0) + rank * LIST_CAP;
-    for (int j0 = s.w0; j0 < s.w1; j0 += 32) {
+    int j0 = s.w0;
+    if (s.quads) {
+      for (; j0 + 128 <= s.w1; j0 += 128) {
+        const int j = j0 + lane * 4;
+        const float4 q = *reinterpret_cast<const float4*>(s.x + j);
+        const float v[4] = {q.x, q.y, q.z, q.w};
+        int found = 0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) found += to_key(v[e]) >= floor;
+        if (!__any_sync(0xffffffffu, found)) continue;
+        int upto = found;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, upto, o);
+          if (lane >= o) upto += t;
+        }
+        int slot = at + upto - found;
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (to_key(v[e]) >= floor) {
+            if (slot < LIST_CAP) { list_v[slot] = v[e]; list_i[slot] = s.first + j + e; }
+            ++slot;
+          }
+        at += __shfl_sync(0xffffffffu, upto, 31);
+      }
+    }
+    for (; j0 < s.w1; j0 += 32) {
       const int j = j0 + lane;
       const float v = j < s.w1 ? s.x[j] : 0.f;
       const bool in = j < s.w1 && to_key(v) >= floor;
@@ -247,8 +289,10 @@ sample_kernel(const float* __restrict__ logits, int64_t row_stride, int V, int p
   const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
   const int row = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int first = min(V, rank * per), n = min(V, first + per) - first;
-  const int seg = (((n + SAMPLE_WARPS - 1) / SAMPLE_WARPS) + 31) & ~31;
+  // (stretches of 2,048 elements and more are walked four elements a lane; shorter ones leave no warp without work)
   Stretch s;
+  s.quads = staged && per >= SAMPLE_WARPS * 128;
+  const int step = s.quads ? 128 : 32, seg = (n + SAMPLE_WARPS * step - 1) / (SAMPLE_WARPS * step) * step;
   s.first = first;
   s.w0 = min(n, warp * seg), s.w1 = min(n, s.w0 + seg);
   pdl_wait();
@@ -278,21 +322,16 @@ sample_kernel(const float* __restrict__ logits, int64_t row_stride, int V, int p
   // maxima of the groups, of the block and (after the exchange) of the row; log-sum-exp of the raw logits
   float vmax = -INFINITY;
   int imax = 0x7fffffff;
-#pragma unroll 4
-  for (int j = s.w0 + lane; j < s.w1; j += 32) {
-    const float v = s.x[j];
+  s.each([&](int j, float v) {
     if (v > vmax) { vmax = v; imax = first + j; }
-  }
+  });
   float gmax = vmax;
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
   int barg;
   const float bmax = block_max_arg<SAMPLE_WARPS>(vmax, imax, &barg, sm.scratch, sm.scratch_i);
   float se = 0.f;
-  if (bmax > -INFINITY) {
-#pragma unroll 4
-    for (int j = s.w0 + lane; j < s.w1; j += 32) se += expf(s.x[j] - bmax);
-  }
+  if (bmax > -INFINITY) s.each([&](int, float v) { se += expf(v - bmax); });
   se = block_sum(se, sm.scratch);
   cluster_wait_started();
   if ((lane & 7) == 0)
@@ -320,28 +359,37 @@ sample_kernel(const float* __restrict__ logits, int64_t row_stride, int V, int p
   const int want = listed ? (int)k : (greedy ? 0 : n_lp_in);      // how many elements the list has to hold
   int n_list = 0;                                                 // entries of block 0's list, packed below
   if (want > 0) {
-    // the want-th largest of the groups' maxima: a lower bound of the want-th largest element
-    if (tid == 0) sm.word[0] = 0xffffffffu;
-    __syncthreads();
-    if (tid < groups) {
-      const float* all = &sm.group_max[0][0];
-      const float mine = all[tid];
-      int larger = 0;
-      for (int g = 0; g < groups; g += 4) {
-        const float4 o = *reinterpret_cast<const float4*>(all + g);
-        larger += (o.x > mine) + (o.y > mine) + (o.z > mine) + (o.w > mine);
-      }
-      if (larger < want) atomicMin(&sm.word[0], to_key(mine));
+    // A lower bound of the want-th largest element: the largest key of sixteen leading bits at or above which lie `want`
+    // of the groups' maxima.  Four bits a round, warp w trying digit w.
+    uint32_t floor = 0;
+    const float* all = &sm.group_max[0][0];
+    uint32_t keys[MAX_RANKS * GROUPS / 32];
+#pragma unroll
+    for (int i = 0; i < MAX_RANKS * GROUPS / 32; ++i) keys[i] = i * 32 < groups ? to_key(all[i * 32 + lane]) : 0u;
+#pragma unroll 1
+    for (int shift = 28; shift >= 16; shift -= 4) {
+      const uint32_t trial = floor | (uint32_t)warp << shift;
+      int at_least = 0;
+#pragma unroll
+      for (int i = 0; i < MAX_RANKS * GROUPS / 32; ++i) at_least += i * 32 < groups && keys[i] >= trial;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) at_least += __shfl_xor_sync(0xffffffffu, at_least, o);
+      if (lane == 0) sm.scratch_i[warp] = at_least;
+      __syncthreads();
+      int digit = 0;
+#pragma unroll
+      for (int d = 1; d < SAMPLE_WARPS; ++d) digit = sm.scratch_i[d] >= want ? d : digit;
+      floor |= (uint32_t)digit << shift;
+      __syncthreads();
     }
-    __syncthreads();
-    hand_over(s, cluster, sm, sm.word[0]);
+    hand_over(s, cluster, sm, floor);
     bool fits = true;
     for (int r = 0; r < ranks; ++r) fits = fits && sm.list_n[r] <= LIST_CAP;
     if (!fits) {
       listed = false;
       if (n_lp_in > 0) {
         // exactly the elements at or above the K-th largest (ties beyond the list's end are left out)
-        uint32_t floor = 0;
+        floor = 0;
         find_cut<true, false>(s, cluster, sm, 0u, (float)n_lp_in - 0.5f, xmax, 1.f, &floor);
         hand_over(s, cluster, sm, floor);
       }
