@@ -20,7 +20,6 @@
 #include <algorithm>
 
 #include "common.cuh"
-#include "conv_window.cuh"
 
 // The gated delta rule in chunks of 64 tokens, for heads of 64 key channels; fp32 throughout.
 //

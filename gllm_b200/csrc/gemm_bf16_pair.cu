@@ -79,11 +79,21 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
       : "memory");
 }
 
+// A grouped product: the tokens' rows come in tiles of 256 that each belong to one group, whose weight is rows
+// group_of_tile[tile] * group_rows .. of W; tiles behind num_tiles[0] do not exist.  row_scale (gated form, null or one
+// number per row): gate and up are multiplied by it first.  group_of_tile null: an ordinary product.
+struct PairGroups {
+  const int* group_of_tile;
+  const int* num_tiles;
+  int group_rows;
+  const float* row_scale;
+};
+
 template <typename OutT, bool GATED>
 __global__ void __launch_bounds__(THREADS, 1)
 umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                       OutT* __restrict__ out, int M, int N, int K, int64_t ldo, int tiles_m, int num_items,
-                      int* __restrict__ status, GateAct act) {
+                      int* __restrict__ status, GateAct act, PairGroups groups) {
   extern __shared__ unsigned char smem_dyn[];
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], tmem_full_bar[2], tmem_empty_bar[2];
   __shared__ uint32_t tmem_base_slot;
@@ -131,12 +141,21 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     const int tn = w / tiles_m, tm = w - tn * tiles_m;    // neighbouring pairs share a weight tile
     row_x = tm * 2 * BM + (int)rank * BM;
     row_w = tn * BN + (int)rank * BNH;
+    if (groups.group_of_tile != nullptr) row_w += groups.group_of_tile[tm] * groups.group_rows;
+  };
+  // (which tiles there are, and whose weight they need, comes from the kernel before)
+  auto count_tiles = [&]() {
+    if (groups.group_of_tile == nullptr) return;
+    pdl_wait();
+    tiles_m = min(tiles_m, groups.num_tiles[0]);
+    num_items = tiles_m * ((N + BN - 1) / BN);
   };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
     if (lane == 0) {
       bool ok = true;
+      count_tiles();
       // pass 0: the weight tiles of the first STAGES k-blocks; pass 1: their token tiles, then both
       // operands of every later block as stages come free
       for (int pass = 0; pass < 2 && ok; ++pass) {
@@ -173,6 +192,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     // issues the products and their commits.
     if (rank == 0) {
       const bool leader = elect_one();
+      count_tiles();
       auto wait_u = [&](uint64_t* bar, uint32_t parity) -> bool {
         const bool good = mbar_wait(smem_addr(bar), parity, status, &abort_flag);
         return __all_sync(0xffffffffu, good) != 0;
@@ -209,13 +229,14 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
   } else {
     // ---------------------------------------------------------------- epilogue (both CTAs)
     pdl_wait();                                           // nothing is written before the previous kernel is done
+    count_tiles();
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
     uint32_t n_used = 0;
     for (int w = pair; w < num_items; w += num_pairs) {
       int row_x, row_w;
       tile_of(w, row_x, row_w);
-      const int col0 = row_w - (int)rank * BNH;            // the tile's first column
+      const int col0 = w / tiles_m * BN;                   // the tile's first column
       const uint32_t acc = n_used & 1u;
       mbar_wait(smem_addr(&tmem_full_bar[acc]), (n_used >> 1) & 1u, status, &abort_flag);
       epilogue_sync();                                    // a warp that gave up has set abort_flag before this
@@ -223,6 +244,8 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
       const int m = row_x + row;
+      float rs = 1.f;
+      if (GATED && groups.row_scale != nullptr && m < M) rs = groups.row_scale[m];
       if (GATED) {
         // this thread's token row holds, per 128 columns, 64 gates then their 64 ups
         const int n_out = N / 2;
@@ -236,7 +259,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
           if (m < M && f0 < n_out) {
             float y[16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) y[i] = gate_act_bf16(g[i], u[i], act);
+            for (int i = 0; i < 16; ++i) y[i] = gate_act_bf16(g[i] * rs, u[i] * rs, act);
             OutT* dst = out + (int64_t)m * ldo + f0;
             if (f0 + 16 <= n_out && sizeof(OutT) == 2 && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
               uint4 p0, p1;
@@ -331,9 +354,11 @@ int sm_count() { return gllm_sm_count(); }
 
 template <typename OutT, bool GATED>
 int pair_launch(const __nv_bfloat16* X, const __nv_bfloat16* W, OutT* out, int M, int N, int K, int64_t ldx,
-                int64_t ldw, int64_t ldo, int* status, cudaStream_t stream, GateAct act = GateAct{1.f, 0.f, 0.f}) {
+                int64_t ldw, int64_t ldo, int* status, cudaStream_t stream, GateAct act = GateAct{1.f, 0.f, 0.f},
+                PairGroups groups = PairGroups{nullptr, nullptr, 0, nullptr}, int w_rows = 0) {
   CUtensorMap map_x, map_w;
-  if (!make_map(&map_x, X, M, K, ldx, BM) || !make_map(&map_w, W, N, K, ldw, BNH)) return (int)cudaErrorInvalidValue;
+  if (w_rows <= 0) w_rows = N;                            // (grouped: the weight's map covers the rows of all groups)
+  if (!make_map(&map_x, X, M, K, ldx, BM) || !make_map(&map_w, W, w_rows, K, ldw, BNH)) return (int)cudaErrorInvalidValue;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(umma_gemm_pair_kernel<OutT, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -345,7 +370,7 @@ int pair_launch(const __nv_bfloat16* X, const __nv_bfloat16* W, OutT* out, int M
   const int num_items = tiles_m * tiles_n;
   const int pairs = num_items < sm_count() / 2 ? num_items : sm_count() / 2;
   return gllm_launch_cluster(umma_gemm_pair_kernel<OutT, GATED>, dim3(2 * pairs), dim3(THREADS), (size_t)SMEM, stream,
-                             2u, map_x, map_w, out, M, N, K, ldo, tiles_m, num_items, status, act);
+                             2u, map_x, map_w, out, M, N, K, ldo, tiles_m, num_items, status, act, groups);
 }
 }  // namespace
 
@@ -365,4 +390,30 @@ GLLM_API int gllm_gemm_bf16_pair(const __nv_bfloat16* X, const __nv_bfloat16* W,
                                             GateAct{slope, limit, offset});
   if (out_is_f32) return pair_launch<float, false>(X, W, (float*)out, M, N, K, ldx, ldw, ldo, status, stream);
   return pair_launch<__nv_bfloat16, false>(X, W, (__nv_bfloat16*)out, M, N, K, ldx, ldw, ldo, status, stream);
+}
+
+// Grouped product: the rows of X [rows, K] come in tiles of 256 that each belong to one group (``group_of_tile``,
+// ``num_tiles`` on the device); group g multiplies by W[g] of W [groups, N, K].  gated != 0: W[g]'s rows are blocks of 64
+// gate rows and the 64 up rows of the same features and out is bf16 [rows, N / 2] (slope, limit, offset as above;
+// row_scale, null or [rows]: gate and up are multiplied by the row's number first); otherwise out is fp32 [rows, N].  Rows
+// of tiles behind ``num_tiles[0]`` are neither read nor written.
+//
+// Against tiles of 128 rows on one CTA (gemm_bf16.cu) a CTA moves two thirds of the bytes per FLOP into shared memory, and
+// that bounds them both: a tile of 256 rows takes a pair about the time that one of 128 takes a single CTA.  3,108
+// rows of 16 groups times 2,048 x 2,048 (gated) and 2,048 x 1,024: 38 and 33 us against 52 and 44.
+GLLM_API int gllm_gemm_bf16_pair_grouped(const __nv_bfloat16* X, const __nv_bfloat16* W, void* out, int gated, int rows,
+                                         int N, int K, int groups, const int* group_of_tile, const int* num_tiles,
+                                         const float* row_scale, float slope, float limit, float offset, int* status,
+                                         cudaStream_t stream) {
+  if (rows <= 0 || N <= 0 || groups <= 0) return 0;
+  if (rows % (2 * BM) || K <= 0 || K % 8 || (gated && N % 128) || (row_scale != nullptr && !gated) ||
+      group_of_tile == nullptr || num_tiles == nullptr || (reinterpret_cast<uintptr_t>(X) & 15) ||
+      (reinterpret_cast<uintptr_t>(W) & 15) || (int64_t)groups * N > 0x7fffffff)
+    return (int)cudaErrorInvalidValue;
+  const PairGroups g{group_of_tile, num_tiles, N, row_scale};
+  if (gated)
+    return pair_launch<__nv_bfloat16, true>(X, W, (__nv_bfloat16*)out, rows, N, K, K, K, N / 2, status, stream,
+                                            GateAct{slope, limit, offset}, g, groups * N);
+  return pair_launch<float, false>(X, W, (float*)out, rows, N, K, K, K, N, status, stream, GateAct{1.f, 0.f, 0.f}, g,
+                                   groups * N);
 }

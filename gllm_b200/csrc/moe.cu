@@ -321,21 +321,48 @@ moe_gemm_kernel(const T* __restrict__ a, int64_t a_stride, int a_div, const T* _
   }
 }
 
+// The shared expert's result as unsummed fp32 parts [n][tokens, width], added in ascending order (p null: there are none).
+struct SharedParts {
+  const float* p;
+  int n;
+  int64_t stride;
+  template <int VEC> __device__ __forceinline__ void sum(int64_t at, float (&v)[VEC]) const {
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) v[e] = 0.f;
+    for (int k = 0; k < n; ++k) {
+      const float* src = p + k * stride + at;
+      if (VEC == 4) {
+        const float4 x = __ldcg(reinterpret_cast<const float4*>(src));
+        v[0] += x.x, v[VEC > 1 ? 1 : 0] += x.y, v[VEC > 2 ? 2 : 0] += x.z, v[VEC > 3 ? 3 : 0] += x.w;
+      } else {
+        v[0] += __ldcg(src);
+      }
+    }
+  }
+};
+
 // A thread takes VEC neighbouring columns; the rows of up to four slots are requested together.
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(RowSum y, const T* __restrict__ shared, T* __restrict__ out, int width,
+moe_combine_kernel(RowSum y, const T* __restrict__ shared, SharedParts parts, T* __restrict__ out, int width,
                    const float* __restrict__ shared_gate, int64_t shared_gate_stride) {
   pdl_trigger();
   pdl_wait();
   const int64_t t = blockIdx.x;
-  const float sg = (shared && shared_gate) ? 1.0f / (1.0f + expf(-shared_gate[t * shared_gate_stride])) : 1.0f;
+  const float sg = ((shared || parts.p) && shared_gate) ? 1.0f / (1.0f + expf(-shared_gate[t * shared_gate_stride])) : 1.0f;
   for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC; c < width; c += gridDim.y * blockDim.x * VEC) {
     float acc[VEC];
+    float sh[VEC];
+    if (parts.p) {                 // (rounded as the shared expert's own result would be)
+      parts.sum<VEC>(t * width + c, sh);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) sh[e] = to_float(from_float<T>(sh[e]));
+    }
     y.sum<VEC>(t, c, width, acc);
 #pragma unroll
     for (int e = 0; e < VEC; ++e) {
-      if (shared) acc[e] = fmaf(sg, to_float(shared[t * width + c + e]), acc[e]);
+      if (parts.p) acc[e] = fmaf(sg, sh[e], acc[e]);
+      else if (shared) acc[e] = fmaf(sg, to_float(shared[t * width + c + e]), acc[e]);
       out[t * width + c + e] = from_float<T>(acc[e]);
     }
   }
@@ -430,23 +457,29 @@ GLLM_API int gllm_moe_gemm_bf16(const __nv_bfloat16* a, int64_t a_stride, int a_
 template <typename T>
 static int moe_combine_launch(const float* y, int n_parts, int64_t part_stride, const float* weights, const T* shared, T* out,
                               const int* row_of_pair, int n_tokens, int top, int width, const float* shared_gate,
-                              int64_t shared_gate_stride, cudaStream_t stream) {
+                              int64_t shared_gate_stride, const float* shared_parts, int shared_n, int64_t shared_stride,
+                              cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
-  if (n_parts < 1 || top < 1 || width < 1) return (int)cudaErrorInvalidValue;
+  if (n_parts < 1 || top < 1 || width < 1 || (shared_parts != nullptr && (shared != nullptr || shared_n < 1)))
+    return (int)cudaErrorInvalidValue;
+  const SharedParts parts{shared_parts, shared_n, shared_stride};
   const RowSum rows{y, n_parts, part_stride, row_of_pair, weights, top};
-  const bool vec = width % 4 == 0 && part_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+  const bool vec = width % 4 == 0 && part_stride % 4 == 0 && shared_stride % 4 == 0 &&
+                   ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(shared_parts)) & 15) == 0;
   const int blocks_y = n_tokens >= 64 ? 1 : (width + (vec ? 1024 : 256) - 1) / (vec ? 1024 : 256);
   auto kernel = vec ? moe_combine_kernel<T, 4> : moe_combine_kernel<T, 1>;
-  return gllm_launch(kernel, dim3(n_tokens, blocks_y), dim3(256), 0, stream, rows, shared, out, width, shared_gate,
-                     shared_gate_stride);
+  return gllm_launch(kernel, dim3(n_tokens, blocks_y), dim3(256), 0, stream, rows, shared, parts, out, width,
+                     shared_gate, shared_gate_stride);
 }
-// y: [n_parts][rows, width] fp32, the parts added in ascending order first.
+// y: [n_parts][rows, width] fp32, the parts added in ascending order first.  shared_parts (instead of `shared`): the shared
+// expert's result as shared_n unsummed fp32 parts, shared_stride floats apart.
 #define GLLM_MOE_COMBINE(T, S)                                                                                         \
   GLLM_API int gllm_moe_combine_##S(const float* y, int n_parts, int64_t part_stride, const float* weights,            \
                                     const T* shared, T* out, const int* row_of_pair, int n_tokens, int top, int width, \
-                                    const float* shared_gate, int64_t shared_gate_stride, cudaStream_t stream) {       \
+                                    const float* shared_gate, int64_t shared_gate_stride, const float* shared_parts,   \
+                                    int shared_n, int64_t shared_stride, cudaStream_t stream) {                        \
     return moe_combine_launch<T>(y, n_parts, part_stride, weights, shared, out, row_of_pair, n_tokens, top, width,     \
-                                 shared_gate, shared_gate_stride, stream);                                             \
+                                 shared_gate, shared_gate_stride, shared_parts, shared_n, shared_stride, stream);      \
   }
 GLLM_MOE_COMBINE(float, f32)
 GLLM_MOE_COMBINE(__nv_bfloat16, bf16)

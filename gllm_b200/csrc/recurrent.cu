@@ -13,7 +13,6 @@
 #include <type_traits>
 
 #include "common.cuh"
-#include "conv_window.cuh"
 #include "mma_utils.cuh"
 
 // The step-sized matrix recurrence (state-space duality) in chunks of 64 tokens on the tensor cores, for bfloat16

@@ -159,7 +159,7 @@ _SIGNATURES = {
         "gllm_moe_align": [P, P, P, P, P, c_int, c_int, c_int, c_int, P],
         "gllm_moe_gemm_{t}": [P, c_int64, c_int, P, c_int64, c_int64, P, P, P, P, c_int, c_int, c_int, c_int, c_int, P,
                               c_float, c_float, c_float, P],
-        "gllm_moe_combine_{t}": [P, c_int, c_int64, P, P, P, P, c_int, c_int, c_int, P, c_int64, P],
+        "gllm_moe_combine_{t}": [P, c_int, c_int64, P, P, P, P, c_int, c_int, c_int, P, c_int64, P, c_int, c_int64, P],
         "gllm_moe_relu_sq_bf16": [P, P, c_int64, P],
         "gllm_moe_gather_{t}": [P, c_int64, P, P, c_int, c_int, c_int, P, P, P],
     },

@@ -58,14 +58,25 @@ def _accumulate_fn():
 
 
 _grouped = None
+_pair_grouped = None
+
+
+def _pair_grouped_fn():
+    global _pair_grouped
+    if _pair_grouped is None:
+        f = load_module("gemm_bf16_pair").gllm_gemm_bf16_pair_grouped
+        f.argtypes = [P, P, P, c_int, c_int, c_int, c_int, c_int, P, P, P, c_float, c_float, c_float, P, P]
+        f.restype = c_int
+        _pair_grouped = f
+    return _pair_grouped
 
 
 def linear_grouped(x: torch.Tensor, weight: torch.Tensor, group_of_tile: torch.Tensor, num_tiles: torch.Tensor,
                    gated: bool, wide: bool, act: tuple = (1.0, 0.0, 0.0),
                    row_scale: torch.Tensor | None = None, tile_rows: int = 128, splits: int = 1) -> torch.Tensor:
-    """``out[r] = x[r] @ weight[g(r)].T`` on the tcgen05 kernel, the rows of ``x [rows, k]`` (bf16, ``rows`` a
-    multiple of ``tile_rows``: 128, or 16, 32 or 64, for which the weight is the 128-row operand) coming in tiles of
-    ``tile_rows`` that each belong to one group: ``group_of_tile [rows / tile_rows]`` and
+    """``out[r] = x[r] @ weight[g(r)].T`` on the tcgen05 kernels, the rows of ``x [rows, k]`` (bf16, ``rows`` a
+    multiple of ``tile_rows``: 256, a tile for a pair of CTAs; 128; or 16, 32 or 64, for which the weight is the 128-row
+    operand) coming in tiles of ``tile_rows`` that each belong to one group: ``group_of_tile [rows / tile_rows]`` and
     ``num_tiles [1]`` (int32, on the device; tiles behind ``num_tiles`` are neither read nor written).  ``weight
     [groups, n, k]``; ``gated``: every group's rows are stacked by ``interleave_gate_up`` and the result is bf16
     ``silu(gate) * up`` ``[rows, n / 2]`` (or what ``act``, the slope, limit and offset of ``linear_gated``, says, of
@@ -85,6 +96,13 @@ def linear_grouped(x: torch.Tensor, weight: torch.Tensor, group_of_tile: torch.T
     groups, n, _ = weight.shape
     shape = (rows, n // 2) if gated else (rows, n) if splits == 1 else (splits, rows, n)
     out = torch.empty(shape, dtype=torch.bfloat16 if gated else torch.float32, device=x.device)
+    if tile_rows == 256:
+        if splits != 1:
+            raise ValueError("tiles of 256 rows are not cut along k")
+        _check(_pair_grouped_fn()(x.data_ptr(), weight.data_ptr(), out.data_ptr(), int(gated), rows, n, k, groups,
+                                  group_of_tile.data_ptr(), num_tiles.data_ptr(), _ptr(row_scale), *act,
+                                  status_word(x.device).data_ptr(), _stream()), "linear_grouped")
+        return out
     _check(_grouped(x.data_ptr(), weight.data_ptr(), out.data_ptr(), int(gated), rows, n, k, groups,
                     group_of_tile.data_ptr(), num_tiles.data_ptr(), int(wide), _ptr(row_scale), *act,
                     int(tile_rows), int(splits), status_word(x.device).data_ptr(), _stream()), "linear_grouped")

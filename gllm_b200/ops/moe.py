@@ -11,6 +11,10 @@ from gllm_b200.ops import RowSum, SplitSum, _check, _cuda, _fn, _parts_args, _pt
 TILE_ROWS = 16        # rows of one tile of the expert products: an expert's pairs are padded to a multiple of it
 PLAIN_GATE = (1.0, 0.0, 0.0)    # slope, limit, offset of a gated expert's activation: silu(gate) * up
 TENSOR_CORE_TILE_ROWS = 128     # the same for the tcgen05 products (the rows of one accumulator tile)
+PAIR_TILE_ROWS = 256            # ... on pairs of CTAs
+# Rows per expert from which tiles of 256 pay (16 experts of 2,048 -> 1,024, both products, tiles of 128 / 256 rows: 96 rows
+# an expert 67 / 86 us, 128 rows 90 / 86, 194 rows 116 / 92, 1,024 rows 321 / 305)
+PAIR_ROWS_PER_EXPERT = 120
 
 
 def _router_args(logits):
@@ -149,7 +153,7 @@ def expert_product(a: torch.Tensor, rows_per_input: int, weight: torch.Tensor, p
     return out
 
 
-def combine(y: torch.Tensor, weights: torch.Tensor | None, shared: torch.Tensor | None, out_dtype: torch.dtype,
+def combine(y: torch.Tensor, weights: torch.Tensor | None, shared: "torch.Tensor | SplitSum | None", out_dtype: torch.dtype,
             row_of_pair: torch.Tensor | None = None, shared_gate: torch.Tensor | None = None, tokens: int | None = None,
             top: int | None = None) -> torch.Tensor:
     """``out[t] = sum_s weights[t, s] * y[t * top + s] (+ shared[t])``, summed in slot order in fp32 (``weights`` None: 1
@@ -166,9 +170,11 @@ def combine(y: torch.Tensor, weights: torch.Tensor | None, shared: torch.Tensor 
         _cuda(row_of_pair, "row_of_pair", torch.int32)
     if (y.shape[1] != n * top and row_of_pair is None) or (row_of_pair is not None and row_of_pair.numel() != n * top):
         raise ValueError("one result row per (token, slot) pair is needed")
+    parts_ptr, n_parts, part_stride = _parts_args(shared)
     if shared is not None:
-        _cuda(shared, "shared", out_dtype)
-        if tuple(shared.shape) != (n, width):
+        if not isinstance(shared, SplitSum):
+            _cuda(shared, "shared", out_dtype)
+        if tuple(shared.shape) != (n, width) or shared.dtype != out_dtype:
             raise ValueError("the shared expert's result does not fit")
     gate_stride = 0
     if shared_gate is not None:
@@ -178,8 +184,9 @@ def combine(y: torch.Tensor, weights: torch.Tensor | None, shared: torch.Tensor 
         gate_stride = shared_gate.stride(0)
     out = torch.empty((n, width), dtype=out_dtype, device=y.device)
     _check(_fn("moe", f"gllm_moe_combine_{_suffix(out_dtype)}")(y.data_ptr(), y.shape[0], y.stride(0), _ptr(weights),
-                                                               _ptr(shared), out.data_ptr(), _ptr(row_of_pair), n,
-                                                               int(top), width, _ptr(shared_gate), gate_stride,
+                                                               _ptr(None if n_parts else shared), out.data_ptr(),
+                                                               _ptr(row_of_pair), n, int(top), width, _ptr(shared_gate),
+                                                               gate_stride, parts_ptr, n_parts, part_stride,
                                                                _stream()), "moe_combine")
     return out
 
@@ -195,8 +202,11 @@ def relu_squared_rows(x: torch.Tensor) -> torch.Tensor:
 
 def grouped_tile_rows(pairs: int, experts: int) -> int:
     """Rows of a tile of the tensor-core products: small tiles (the weight is then the 128-row operand, and a tile's rows
-    cost little) while an expert gets few rows on average."""
+    cost little) while an expert gets few rows on average; tiles for pairs of CTAs once it gets more than
+    ``PAIR_ROWS_PER_EXPERT``."""
     per_expert = pairs / experts
+    if per_expert > PAIR_ROWS_PER_EXPERT:
+        return PAIR_TILE_ROWS
     return 16 if per_expert <= 8 else 32 if per_expert <= 20 else 64 if per_expert <= 40 else TENSOR_CORE_TILE_ROWS
 
 
@@ -236,7 +246,7 @@ def apply_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_g
 
 
 def apply_choice(x: torch.Tensor, choice: Choice, w_gate_up: torch.Tensor, w_down: torch.Tensor,
-                 shared: torch.Tensor | None, tensor_cores: bool, gated: bool = True,
+                 shared: "torch.Tensor | SplitSum | None", tensor_cores: bool, gated: bool = True,
                  shared_gate: torch.Tensor | None = None, act: tuple = PLAIN_GATE, weight_on_input: bool = False,
                  defer_sum: bool = False):
     """``out[t] = sum_s weights[t, s] * expert_{ids[t, s]}(x[t]) (+ shared[t])`` with ``expert_e(x) = w_down[e]
@@ -272,7 +282,7 @@ def apply_choice(x: torch.Tensor, choice: Choice, w_gate_up: torch.Tensor, w_dow
         if not gated:
             hidden = relu_squared_rows(hidden)
         splits = 1
-        if choice.tile_rows != TENSOR_CORE_TILE_ROWS:
+        if choice.tile_rows < TENSOR_CORE_TILE_ROWS:
             splits = _down_splits(pairs, experts, w_down.shape[1], w_down.shape[2], x.device)
         y = gemm_bf16.linear_grouped(hidden, w_down, tile_expert, num_tiles, gated=False, wide=wide,
                                      tile_rows=choice.tile_rows, splits=splits)

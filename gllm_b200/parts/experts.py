@@ -129,7 +129,7 @@ class RoutedExperts(FeedForward):
         shared = None
         if self.shared is not None:
             sink, ctx.residual_sink = getattr(ctx, "residual_sink", None), None
-            shared = ops.as_tensor(self.shared.forward(x, ctx))
+            shared = self.shared.forward(x, ctx)          # (a SplitSum lives on: the experts' products take no scratch)
             ctx.residual_sink = sink
         return moe.apply_choice(x, choice, self.w_gate_up, self.w_down, shared, self.tensor_cores, gated=self.gated,
                                 shared_gate=gate, act=self.act, weight_on_input=self.weight_on_input,
