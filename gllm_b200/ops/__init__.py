@@ -268,7 +268,7 @@ def _stream() -> int:
     """The current CUDA stream's handle (every kernel is launched on it).  The raw getter costs a
     fraction of a microsecond; building a ``torch.cuda.Stream`` object for every launch cost 15 us."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(torch._C._cuda_getDevice())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -320,39 +320,50 @@ class SplitSum:
     raises."""
 
     def __init__(self, parts: torch.Tensor, dtype: torch.dtype, generation: int | None = None):
-        self.parts = parts
+        self._parts, self._buffer = parts, parts
+        self.count, self.shape, self.part_stride = parts.shape[0], parts.shape[1:], parts.stride(0)
         self.dtype = dtype
         # the count of scratch-taking products on the device when this one ran (None: the parts are
         # the caller's own memory)
         self.generation = generation
 
+    @classmethod
+    def in_scratch(cls, buffer: torch.Tensor, count: int, rows: int, cols: int, dtype: torch.dtype,
+                   generation: int) -> "SplitSum":
+        """``count`` parts ``[rows, cols]`` one after another from the start of a flat fp32 buffer."""
+        self = cls.__new__(cls)
+        self._parts, self._buffer = None, buffer
+        self.count, self.shape, self.part_stride = count, torch.Size((rows, cols)), rows * cols
+        self.dtype, self.generation = dtype, generation
+        return self
+
+    @property
+    def parts(self) -> torch.Tensor:
+        if self._parts is None:
+            self._parts = self._buffer[: self.count * self.part_stride].view(self.count, *self.shape)
+        return self._parts
+
     def check_alive(self) -> None:
         if self.generation is None:
             return
-        from gllm_b200.ops import gemm_bf16
-
-        now = gemm_bf16.scratch_generation(self.parts.device)
+        now = gemm_bf16.scratch_generation(self._buffer.device)
         if now - self.generation > 1:
             raise RuntimeError(
                 f"an unsummed product was read after {now - self.generation} further products: its partial sums "
                 "have been overwritten (sum it with ops.as_tensor before running two more products)")
 
     @property
-    def shape(self):
-        return self.parts.shape[1:]
-
-    @property
     def device(self):
-        return self.parts.device
+        return self._buffer.device
 
     def tensor(self, out: torch.Tensor | None = None) -> torch.Tensor:
         """The summed result as an ordinary tensor of ``dtype`` (into ``out``, contiguous, when given)."""
         self.check_alive()
         if out is None:
-            out = torch.empty(tuple(self.shape), dtype=self.dtype, device=self.parts.device)
+            out = self._buffer.new_empty(self.shape, dtype=self.dtype)
         f = _fn("elementwise", f"gllm_sum_parts_{_suffix(self.dtype)}")
-        _check(f(self.parts.data_ptr(), self.parts.shape[0], self.parts.stride(0), out.data_ptr(), out.numel(),
-                 _stream()), "sum_parts")
+        _check(f(self._buffer.data_ptr(), self.count, self.part_stride, out.data_ptr(), out.numel(), _stream()),
+               "sum_parts")
         return out
 
 
@@ -435,7 +446,7 @@ class DepthPending:
 def _parts_args(x):
     if isinstance(x, SplitSum):
         x.check_alive()
-        return x.parts.data_ptr(), x.parts.shape[0], x.parts.stride(0)
+        return x._buffer.data_ptr(), x.count, x.part_stride
     return None, 0, 0
 
 
@@ -710,8 +721,6 @@ def linear_gated(x: torch.Tensor, weight: torch.Tensor, slope: float = 1.0, limi
     _cuda(weight, "weight", x.dtype)
     plain = slope == 1.0 and limit is None and up_offset == 0.0
     if x.dtype == torch.bfloat16:
-        from gllm_b200.ops import gemm_bf16
-
         fused = gemm_bf16.linear_gated(x, weight, slope=slope, limit=limit, up_offset=up_offset)
         if fused is not None:
             return fused
@@ -940,19 +949,17 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
     if k != k2:
         raise ValueError(f"x has {k} columns, weight has {k2}")
     out_dtype = out_dtype or x.dtype
-    if add_into is not None and x.dtype == torch.bfloat16 and out is None and ACCUMULATE_IN_PRODUCT:
-        from gllm_b200.ops import gemm_bf16
-
-        if gemm_bf16.linear_accumulate(x, weight, add_into):
-            return ADDED
-    if x.dtype == torch.bfloat16 and split_ok and out is None:
-        from gllm_b200.ops import gemm_bf16
-
-        split = gemm_bf16.linear_split(x, weight, out_dtype)
-        if split is not None:
-            return split
+    if x.dtype == torch.bfloat16 and out is None and (split_ok or add_into is not None):
+        if gemm_bf16.tensor_core_kernel_takes(x, weight):
+            if (add_into is not None and ACCUMULATE_IN_PRODUCT
+                    and gemm_bf16.linear_accumulate(x, weight, add_into, takes=True)):
+                return ADDED
+            if split_ok:
+                split = gemm_bf16.linear_split(x, weight, out_dtype, takes=True)
+                if split is not None:
+                    return split
     if out is None:
-        out = torch.empty((m, n), dtype=out_dtype, device=x.device)
+        out = x.new_empty((m, n), dtype=out_dtype)
     else:
         _cuda(out, "out", out_dtype)
     if x.dtype == torch.float32:
@@ -961,8 +968,6 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
         f = _fn("gemm_fp32", "gllm_gemm_f32")
         _check(f(x.data_ptr(), weight.data_ptr(), out.data_ptr(), m, n, k, x.stride(0), k, n, _stream()), "gemm_f32")
         return out
-    from gllm_b200.ops import gemm_bf16
-
     return gemm_bf16.linear_bf16(x, weight, out)
 
 
@@ -1035,14 +1040,10 @@ def paged_attention(
             raise ValueError("a layer has a window or chunks, not both")
         win = -int(chunk)                 # the kernels' way of saying it (first_visible_key in csrc/common.cuh)
     if qkv.dtype == torch.bfloat16:
-        from gllm_b200.ops import attention_bf16
-
         if attention_bf16.supports(d, block_size) and batch is not None:
             return attention_bf16.paged_attention_bf16(qkv, cache_layer, block_table, positions, token_row,
                                                        num_heads, scale, win, batch, out)
     elif batch is not None:
-        from gllm_b200.ops import attention_f32
-
         if attention_f32.takes(qkv, cache_layer, num_heads, batch, out):
             return attention_f32.paged_attention_f32(qkv, cache_layer, block_table, positions, token_row, num_heads,
                                                      scale, win, batch, out)
@@ -1129,3 +1130,7 @@ def sample(
              out["logprobs"].data_ptr(), out["num_candidates"].data_ptr(), _ptr(top_lp), _ptr(top_id),
              _ptr(probs), _stream()), "sample")
     return out
+
+
+# (the modules of the products and of the attention kernels use what is defined above)
+from gllm_b200.ops import attention_bf16, attention_f32, gemm_bf16  # noqa: E402

@@ -8,11 +8,13 @@ so each kernel works on one contiguous run of tokens.
 
 from __future__ import annotations
 
+import functools
 import os
 from ctypes import c_float, c_int, c_int64, c_void_p
 
 import torch
 
+import gllm_b200.ops as ops
 from gllm_b200.ops.build import load_module
 
 P = c_void_p
@@ -62,8 +64,6 @@ def prefill_tmem_supports(head_dim: int, block_size: int, q: torch.Tensor, cache
 def prefill_attention_tmem(q, q_stride, cache_layer, block_table, cu_q, ctx_lens, slots, num_requests, max_q_len,
                            num_heads, scale, window, out):
     """tcgen05 attention of the first ``num_requests`` requests of the flat batch."""
-    from gllm_b200 import ops
-
     num_pages, _, hkv, block_size, d = cache_layer.shape
     code = _prefill_tmem_fn()[0](
         q.data_ptr(), q_stride, out.data_ptr(), out.stride(0), cache_layer.data_ptr(), block_table.data_ptr(),
@@ -83,8 +83,6 @@ def prefill_attention(q, q_stride, cache_layer, block_table, cu_q, ctx_lens, slo
                       num_heads, scale, window, out):
     """Tensor-core attention of the first ``num_requests`` requests of the
     flat batch (portions of prompts)."""
-    from gllm_b200 import ops
-
     num_pages, _, hkv, block_size, d = cache_layer.shape
     code = _prefill_fn()(
         q.data_ptr(), q_stride, out.data_ptr(), out.stride(0), cache_layer.data_ptr(), block_table.data_ptr(),
@@ -139,6 +137,11 @@ def decode_stream_parts(head_dim: int, num_heads: int, num_kv_heads: int, block_
     or 32 tokens, 16-byte aligned operands)."""
     if head_dim not in (64, 128) or q.data_ptr() % 16 or cache_layer.data_ptr() % 16 or q.stride(0) % 8:
         return 0
+    return _stream_parts(head_dim, num_heads, num_kv_heads, block_size)
+
+
+@functools.lru_cache(maxsize=1024)
+def _stream_parts(head_dim: int, num_heads: int, num_kv_heads: int, block_size: int) -> int:
     return int(_decode_stream_fn()[1](head_dim, num_heads, num_kv_heads, block_size))
 
 
@@ -178,8 +181,6 @@ def decode_attention(q, q_stride, cache_layer, block_table, positions, token_row
     """Split-KV attention of ``positions.numel()`` single query tokens.  ``kernel``: "split" (one
     CTA per chunk of keys and kv head), "stream" (one persistent CTA per SM, TMA) or "auto" (stream
     when the step has enough keys to keep every SM's stream busy)."""
-    from gllm_b200 import ops
-
     num_pages, _, hkv, block_size, d = cache_layer.shape
     n = positions.numel()
     parts = decode_stream_parts(d, num_heads, hkv, block_size, q, cache_layer) if kernel != "split" else 0
@@ -213,8 +214,6 @@ def decode_attention(q, q_stride, cache_layer, block_table, positions, token_row
 
 
 def paged_attention_bf16(qkv, cache_layer, block_table, positions, token_row, num_heads, scale, window, batch, out):
-    from gllm_b200 import ops
-
     n = qkv.shape[0]
     n_pf = batch.num_prefill_tokens
     d, block_size = cache_layer.shape[4], cache_layer.shape[3]

@@ -8,6 +8,8 @@ from ctypes import c_float, c_int, c_int64, c_void_p
 
 import torch
 
+import gllm_b200.ops as ops
+from gllm_b200.ops.attention_bf16 import visible_spans
 from gllm_b200.ops.build import load_module
 
 P = c_void_p
@@ -41,9 +43,6 @@ def takes(qkv: torch.Tensor, cache_layer: torch.Tensor, num_heads: int, batch, o
 
 
 def paged_attention_f32(qkv, cache_layer, block_table, positions, token_row, num_heads, scale, window, batch, out):
-    from gllm_b200 import ops
-    from gllm_b200.ops.attention_bf16 import visible_spans
-
     portions, singles, chunk = _functions()
     num_pages, _, hkv, block_size, d = cache_layer.shape
     n, n_pf = qkv.shape[0], batch.num_prefill_tokens

@@ -18,7 +18,7 @@ def _joined(p: DepthPending, resid: torch.Tensor, dtype: torch.dtype, staged_row
         raise ValueError("resid must be [tokens, width]")
     n, width = resid.shape
     value = p.value
-    if isinstance(value, SplitSum) and (value.parts.shape[0] > 16 or 4 * staged_rows * width > STAGED_BYTES):
+    if isinstance(value, SplitSum) and (value.count > 16 or 4 * staged_rows * width > STAGED_BYTES):
         value = value.tensor()
     parts_ptr, n_parts, part_stride = _parts_args(value)
     if value is not None:

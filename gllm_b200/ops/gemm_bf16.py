@@ -11,11 +11,13 @@ which is what the reference uses for every projection
 
 from __future__ import annotations
 
+import functools
 import os
 from ctypes import c_float, c_int, c_int64, c_void_p
 
 import torch
 
+import gllm_b200.ops as ops
 from gllm_b200.ops.build import load_module
 
 P = c_void_p
@@ -90,8 +92,7 @@ def linear_grouped(x: torch.Tensor, weight: torch.Tensor, group_of_tile: torch.T
                       P, P]
         f.restype = c_int
         _grouped = f
-    from gllm_b200.ops import _check, _ptr, _stream, status_word
-
+    _check, _ptr, _stream, status_word = ops._check, ops._ptr, ops._stream, ops.status_word
     rows, k = x.shape
     groups, n, _ = weight.shape
     shape = (rows, n // 2) if gated else (rows, n) if splits == 1 else (splits, rows, n)
@@ -188,8 +189,6 @@ def linear_pair(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, gated:
                 act: tuple = (1.0, 0.0, 0.0)) -> torch.Tensor:
     """``out = x @ weight.T`` (or its gated form, see ``linear_gated``) by the kernel in which two CTAs
     of a cluster share every 256x256 tile.  Any number of tokens is right; few are slow."""
-    from gllm_b200 import ops
-
     m, k = x.shape
     code = _pair_fn()(x.data_ptr(), weight.data_ptr(), out.data_ptr(), int(out.dtype == torch.float32), int(gated), m,
                       weight.shape[0], k, x.stride(0), weight.stride(0), out.stride(0), *act,
@@ -199,18 +198,23 @@ def linear_pair(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, gated:
 
 
 def tensor_core_kernel_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
-    k = x.shape[1]
-    return (k % 8 == 0 and x.stride(1) == 1 and weight.stride(1) == 1 and x.stride(0) % 8 == 0
-            and weight.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
+    rows_x, cols_x = x.stride()
+    rows_w, cols_w = weight.stride()
+    return (x.shape[1] % 8 == 0 and cols_x == 1 and cols_w == 1 and rows_x % 8 == 0 and rows_w % 8 == 0
+            and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
+
+
+@functools.lru_cache(maxsize=4096)
+def _splits(m: int, n: int, k: int) -> int:
+    """Ranges of K that the one-CTA kernel cuts a product into: a function of the sizes alone."""
+    return _umma_fns()[1](m, n, k)
 
 
 def linear_tcgen05(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-    from gllm_b200 import ops
-
-    f, splits_of, tiles_of = _umma_fns()[:3]
+    f, _, tiles_of = _umma_fns()[:3]
     m, k = x.shape
     n = weight.shape[0]
-    splits = splits_of(m, n, k)
+    splits = _splits(m, n, k)
     if splits == 1 and pair_kernel_pays(x, n):
         return linear_pair(x, weight, out)
     partial, tickets = _device_scratch(x.device, splits * m * n if splits > 1 else 0, tiles_of(m, n))
@@ -220,8 +224,7 @@ def linear_tcgen05(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> 
                  weight.stride(0), n, splits, partial.data_ptr(), tickets.data_ptr(), 0,
                  ops.status_word(x.device).data_ptr(), ops._stream())
         ops._check(code, "gemm_bf16")
-        return ops.SplitSum(partial[: splits * m * n].view(splits, m, n), out.dtype,
-                            scratch_generation(x.device)).tensor(out)
+        return ops.SplitSum.in_scratch(partial, splits, m, n, out.dtype, scratch_generation(x.device)).tensor(out)
     code = f(x.data_ptr(), weight.data_ptr(), out.data_ptr(), int(out.dtype == torch.float32), m, n, k,
              x.stride(0), weight.stride(0), out.stride(0), splits, partial.data_ptr(), tickets.data_ptr(), 1,
              ops.status_word(x.device).data_ptr(), ops._stream())
@@ -229,17 +232,15 @@ def linear_tcgen05(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> 
     return out
 
 
-def linear_split(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype):
+def linear_split(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, takes: bool = False):
     """The product as a SplitSum when the kernel would cut it along K; None
-    when it would not (or does not take these operands)."""
-    from gllm_b200 import ops
-
-    if not tensor_core_kernel_takes(x, weight):
+    when it would not (or does not take these operands; ``takes``: it is known to)."""
+    if not takes and not tensor_core_kernel_takes(x, weight):
         return None
-    f, splits_of, tiles_of = _umma_fns()[:3]
+    f = _umma_fns()[0]
     m, k = x.shape
     n = weight.shape[0]
-    splits = splits_of(m, n, k)
+    splits = _splits(m, n, k)
     if splits <= 1:
         return None
     partial, tickets = _device_scratch(x.device, splits * m * n, 0)
@@ -247,7 +248,7 @@ def linear_split(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype):
              weight.stride(0), n, splits, partial.data_ptr(), tickets.data_ptr(), 0,
              ops.status_word(x.device).data_ptr(), ops._stream())
     ops._check(code, "gemm_bf16")
-    return ops.SplitSum(partial[: splits * m * n].view(splits, m, n), out_dtype, scratch_generation(x.device))
+    return ops.SplitSum.in_scratch(partial, splits, m, n, out_dtype, scratch_generation(x.device))
 
 
 def linear_bf16(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
@@ -267,15 +268,13 @@ def linear_gated(x: torch.Tensor, weight: torch.Tensor, slope: float = 1.0, limi
     product's epilogue (``a(g) = g * sigmoid(slope * g)``, gate capped at ``limit`` and up clamped to
     ``[-limit, limit]`` with ``limit``; the defaults are ``silu(gate) * up``); None when the kernel does not take
     these operands."""
-    from gllm_b200 import ops
-
     act = (float(slope), float(limit or 0.0), float(up_offset))
 
     n, k = weight.shape
     if not tensor_core_kernel_takes(x, weight) or n % 128:
         return None
     m = x.shape[0]
-    out = torch.empty((m, n // 2), dtype=torch.bfloat16, device=x.device)
+    out = x.new_empty((m, n // 2))
     if pair_kernel_pays(x, n):
         return linear_pair(x, weight, out, gated=True, act=act)
     g = _umma_fns()[3]
@@ -286,17 +285,15 @@ def linear_gated(x: torch.Tensor, weight: torch.Tensor, slope: float = 1.0, limi
 
 
 # ---- a product that adds itself into the residual stream
-def linear_accumulate(x: torch.Tensor, weight: torch.Tensor, acc: torch.Tensor) -> bool:
+def linear_accumulate(x: torch.Tensor, weight: torch.Tensor, acc: torch.Tensor, takes: bool = False) -> bool:
     """``acc += x @ weight.T`` (``acc`` fp32 ``[m, n]``) inside the product's epilogue, for up to 64
     tokens; False when the kernel does not take the operands (nothing was launched)."""
-    from gllm_b200 import ops
-
     m, k = x.shape
     n = weight.shape[0]
-    if (m > FEW_TOKENS or not tensor_core_kernel_takes(x, weight) or acc.dtype != torch.float32
+    if (m > FEW_TOKENS or not (takes or tensor_core_kernel_takes(x, weight)) or acc.dtype != torch.float32
             or tuple(acc.shape) != (m, n) or acc.stride(1) != 1):
         return False
-    splits = _umma_fns()[1](m, n, k)
+    splits = _splits(m, n, k)
     code = _accumulate_fn()(x.data_ptr(), weight.data_ptr(), acc.data_ptr(), m, n, k, x.stride(0), weight.stride(0),
                             acc.stride(0), splits, ops.status_word(x.device).data_ptr(), ops._stream())
     ops._check(code, "gemm_bf16_accumulate")
