@@ -81,7 +81,8 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
 
 // A grouped product: the tokens' rows come in tiles of 256 that each belong to one group, whose weight is rows
 // group_of_tile[tile] * group_rows .. of W; tiles behind num_tiles[0] do not exist.  row_scale (gated form, null or one
-// number per row): gate and up are multiplied by it first.  group_of_tile null: an ordinary product.
+// number per row): gate and up are multiplied by it first.  A form of its own (GROUPED), so that ordinary products don't
+// pay for its tests and factors.
 struct PairGroups {
   const int* group_of_tile;
   const int* num_tiles;
@@ -89,7 +90,7 @@ struct PairGroups {
   const float* row_scale;
 };
 
-template <typename OutT, bool GATED>
+template <typename OutT, bool GATED, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1)
 umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                       OutT* __restrict__ out, int M, int N, int K, int64_t ldo, int tiles_m, int num_items,
@@ -141,11 +142,11 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     const int tn = w / tiles_m, tm = w - tn * tiles_m;    // neighbouring pairs share a weight tile
     row_x = tm * 2 * BM + (int)rank * BM;
     row_w = tn * BN + (int)rank * BNH;
-    if (groups.group_of_tile != nullptr) row_w += groups.group_of_tile[tm] * groups.group_rows;
+    if (GROUPED) row_w += groups.group_of_tile[tm] * groups.group_rows;
   };
   // (which tiles there are, and whose weight they need, comes from the kernel before)
   auto count_tiles = [&]() {
-    if (groups.group_of_tile == nullptr) return;
+    if (!GROUPED) return;
     pdl_wait();
     tiles_m = min(tiles_m, groups.num_tiles[0]);
     num_items = tiles_m * ((N + BN - 1) / BN);
@@ -245,7 +246,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
       const uint32_t taddr = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
       const int m = row_x + row;
       float rs = 1.f;
-      if (GATED && groups.row_scale != nullptr && m < M) rs = groups.row_scale[m];
+      if (GROUPED && GATED && groups.row_scale != nullptr && m < M) rs = groups.row_scale[m];
       if (GATED) {
         // this thread's token row holds, per 128 columns, 64 gates then their 64 ups
         const int n_out = N / 2;
@@ -259,7 +260,8 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
           if (m < M && f0 < n_out) {
             float y[16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) y[i] = gate_act_bf16(g[i] * rs, u[i] * rs, act);
+            for (int i = 0; i < 16; ++i)
+              y[i] = GROUPED ? gate_act_bf16(g[i] * rs, u[i] * rs, act) : gate_act_bf16(g[i], u[i], act);
             OutT* dst = out + (int64_t)m * ldo + f0;
             if (f0 + 16 <= n_out && sizeof(OutT) == 2 && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
               uint4 p0, p1;
@@ -352,7 +354,7 @@ bool make_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t ld
 }
 int sm_count() { return gllm_sm_count(); }
 
-template <typename OutT, bool GATED>
+template <typename OutT, bool GATED, bool GROUPED = false>
 int pair_launch(const __nv_bfloat16* X, const __nv_bfloat16* W, OutT* out, int M, int N, int K, int64_t ldx,
                 int64_t ldw, int64_t ldo, int* status, cudaStream_t stream, GateAct act = GateAct{1.f, 0.f, 0.f},
                 PairGroups groups = PairGroups{nullptr, nullptr, 0, nullptr}, int w_rows = 0) {
@@ -361,7 +363,8 @@ int pair_launch(const __nv_bfloat16* X, const __nv_bfloat16* W, OutT* out, int M
   if (!make_map(&map_x, X, M, K, ldx, BM) || !make_map(&map_w, W, w_rows, K, ldw, BNH)) return (int)cudaErrorInvalidValue;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(umma_gemm_pair_kernel<OutT, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(umma_gemm_pair_kernel<OutT, GATED, GROUPED>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          SMEM);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
@@ -369,7 +372,7 @@ int pair_launch(const __nv_bfloat16* X, const __nv_bfloat16* W, OutT* out, int M
   const int tiles_m = (M + 2 * BM - 1) / (2 * BM), tiles_n = (N + BN - 1) / BN;
   const int num_items = tiles_m * tiles_n;
   const int pairs = num_items < sm_count() / 2 ? num_items : sm_count() / 2;
-  return gllm_launch_cluster(umma_gemm_pair_kernel<OutT, GATED>, dim3(2 * pairs), dim3(THREADS), (size_t)SMEM, stream,
+  return gllm_launch_cluster(umma_gemm_pair_kernel<OutT, GATED, GROUPED>, dim3(2 * pairs), dim3(THREADS), (size_t)SMEM, stream,
                              2u, map_x, map_w, out, M, N, K, ldo, tiles_m, num_items, status, act, groups);
 }
 }  // namespace
@@ -412,8 +415,8 @@ GLLM_API int gllm_gemm_bf16_pair_grouped(const __nv_bfloat16* X, const __nv_bflo
     return (int)cudaErrorInvalidValue;
   const PairGroups g{group_of_tile, num_tiles, N, row_scale};
   if (gated)
-    return pair_launch<__nv_bfloat16, true>(X, W, (__nv_bfloat16*)out, rows, N, K, K, K, N / 2, status, stream,
+    return pair_launch<__nv_bfloat16, true, true>(X, W, (__nv_bfloat16*)out, rows, N, K, K, K, N / 2, status, stream,
                                             GateAct{slope, limit, offset}, g, groups * N);
-  return pair_launch<float, false>(X, W, (float*)out, rows, N, K, K, K, N, status, stream, GateAct{1.f, 0.f, 0.f}, g,
+  return pair_launch<float, false, true>(X, W, (float*)out, rows, N, K, K, K, N, status, stream, GateAct{1.f, 0.f, 0.f}, g,
                                    groups * N);
 }
