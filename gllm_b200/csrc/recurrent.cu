@@ -28,15 +28,18 @@
 // heads of 64 x 128: y 9.7e-8, state 1.1e-7 (1.3e-7 and 1.1e-7 token by token); decays a hundred times slower 8.7e-8 and
 // 9.2e-8 (2.0e-7 and 6.4e-7).  With the tensor cores adding into long-lived accumulators they were 6.1e-7 and 2.5e-7.
 //
-// A block takes 32 value columns of one (request, head); eight warps.  Warp w owns rows 16 (w / 2) .. of the chunk
-// (half of its causal tiles of C B^T, then 16 of the 32 columns of y) and DK / 8 columns of the state.  The next chunk's
-// C, B and x are copied and its decays summed (by a ninth warp) while this one is computed.  What bounds it: the chain of a
-// chunk, 4.4 us of two barriers and about 1,200 instructions a warp with two warps a scheduler (tensor pipe 22 % busy),
-// times the chunks of the longest request; token by token a chunk is a chain of 64 steps, 23 us.  2,048 tokens of one
-// request, 64 heads of 64 x 128: 142 us against 727; four of 512: 147 against 672; 64: 17 against 28.
+// A block takes 32 value columns of one (request, head) with a warp for every 8 key channels (16 or 8 warps).  The warps
+// share each 16 rows of the chunk (its causal tiles of C B^T, then the columns of y) and each owns 8 columns of the state.
+// The next chunk's C, B and x are copied and its decays summed (by one more warp) while this one is computed.  What bounds
+// it: the chain of a chunk, 4.2 us of two barriers around products whose operands are read from shared memory (about
+// 510 KB a chunk: half of that time; tensor pipe 22 % busy), times the chunks of the longest request; token by token a chunk
+// is a chain of 64 steps, 23 us.  2,048 tokens of one request, 64 heads of 64 x 128: 135 us against 727 (142 with eight
+// warps of 16 state columns); with eight warps four of 512: 147 against 672; 64: 17 against 28.
 
 namespace ssd {
-constexpr int L = 64, COLS = 32, THREADS = 256;     // (and one warp more, for the decays)
+constexpr int L = 64, COLS = 32;
+// a warp for every 8 state columns, and one more for the decays
+template <int DK> constexpr int THREADS_OF = DK * 4;
 constexpr int XP = COLS + 8, MP = L + 8;            // rows padded by 16 bytes: ldmatrix without bank conflicts
 
 template <int DK> struct Smem {
@@ -63,7 +66,9 @@ __device__ __forceinline__ void mma_add(float (&sum)[4], const uint32_t (&a)[4],
 #pragma unroll
   for (int e = 0; e < 4; ++e) sum[e] += d[e];
 }
-__device__ __forceinline__ void block_barrier() { asm volatile("bar.sync 0, %0;" ::"n"(THREADS + 32) : "memory"); }
+template <int THREADS> __device__ __forceinline__ void block_barrier() {
+  asm volatile("bar.sync 0, %0;" ::"n"(THREADS + 32) : "memory");
+}
 
 __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -75,7 +80,7 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t&
 }
 
 template <int DK>
-__global__ void __launch_bounds__(THREADS + 32, 1)
+__global__ void __launch_bounds__(THREADS_OF<DK> + 32, 1)
 chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_bfloat16* __restrict__ k,
              int64_t k_stride, const __nv_bfloat16* __restrict__ v, int64_t v_stride, const float* __restrict__ gates,
              int64_t gates_stride, const float* __restrict__ gate_bias, const float* __restrict__ rate, float q_scale,
@@ -83,14 +88,16 @@ chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_b
              float* __restrict__ out, int64_t out_stride, int heads, int dv, int kv_div, int from) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem<DK>& sm = *reinterpret_cast<Smem<DK>*>(smem_raw);
-  constexpr int KS = DK / 16, NT = DK / 64;         // k steps of a product over DK; tiles of 8 state columns a warp owns
+  // k steps of a product over DK; warps that share 16 rows of a product; the tiles of 8 columns that one of them has at most
+  // in the causal matrix, and in the rest
+  constexpr int THREADS = THREADS_OF<DK>, KS = DK / 16, Q = THREADS / 128, NC = 8 / Q, NY = 4 / Q;
   pdl_trigger();
   pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * COLS;
   const int start = cu_q[r], end = cu_q[r + 1];
   if (start >= end || end - start < from) return;   // (shorter requests are another kernel's)
-  const int mt = warp >> 1, half = warp & 1, gr = lane >> 2, gc = (lane & 3) * 2;
+  const int mt = warp / Q, part = warp % Q, gr = lane >> 2, gc = (lane & 3) * 2;
   const float A = rate[h], bias = gate_bias[h];
   const __nv_bfloat16* q_src = q + (h / kv_div) * DK;
   const __nv_bfloat16* k_src = k + (h / kv_div) * DK;
@@ -105,25 +112,23 @@ chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_b
       cp_async16(smem_u32(&sm.c[buf][t][p]), q_src + tok * q_stride + p, t < nt);
       cp_async16(smem_u32(&sm.b[buf][t][p]), k_src + tok * k_stride + p, t < nt);
     }
-    {
+    if (tid < L * COLS / 8) {
       const int t = tid >> 2, p = (tid & 3) * 8;
       cp_async16(smem_u32(&sm.x[buf][t][p]), v_src + (int64_t)(t0 + min(t, nt - 1)) * v_stride + p, t < nt);
     }
     cp_async_commit();
   };
-  auto put_state = [&](const float (&S)[2][NT][4]) {
+  auto put_state = [&](const float (&S)[2][4]) {
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
-      for (int n = 0; n < NT; ++n)
+      for (int e = 0; e < 2; ++e) {
+        uint32_t parts[3];
+        split3(S[m][2 * e], S[m][2 * e + 1], parts[0], parts[1], parts[2]);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          uint32_t part[3];
-          split3(S[m][n][2 * e], S[m][n][2 * e + 1], part[0], part[1], part[2]);
-#pragma unroll
-          for (int p = 0; p < 3; ++p)
-            *reinterpret_cast<uint32_t*>(&sm.s[p][m * 16 + gr + 8 * e][(warp * NT + n) * 8 + gc]) = part[p];
-        }
+        for (int p = 0; p < 3; ++p)
+          *reinterpret_cast<uint32_t*>(&sm.s[p][m * 16 + gr + 8 * e][warp * 8 + gc]) = parts[p];
+      }
   };
 
   if (warp == THREADS / 32) {
@@ -163,39 +168,37 @@ chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_b
     fetch(start);
     scan(start, 0);
     for (int t0 = start, buf = 0; t0 < end; t0 += L, buf ^= 1) {
-      block_barrier();
+      block_barrier<THREADS>();
       if (t0 + L < end) scan(t0 + L, buf ^ 1);
-      block_barrier();
+      block_barrier<THREADS>();
     }
     return;
   }
   request(start, 0);
-  float S[2][NT][4];
-  float* sp = state + (((int64_t)state_slots[r] * heads + h) * dv + col0 + gr) * DK + warp * NT * 8 + gc;
+  float S[2][4];
+  float* sp = state + (((int64_t)state_slots[r] * heads + h) * dv + col0 + gr) * DK + warp * 8 + gc;
 #pragma unroll
   for (int m = 0; m < 2; ++m)
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const float2 x = *reinterpret_cast<const float2*>(sp + (int64_t)(m * 16 + 8 * e) * DK + n * 8);
-        S[m][n][2 * e] = x.x, S[m][n][2 * e + 1] = x.y;
-      }
+    for (int e = 0; e < 2; ++e) {
+      const float2 x = *reinterpret_cast<const float2*>(sp + (int64_t)(m * 16 + 8 * e) * DK);
+      S[m][2 * e] = x.x, S[m][2 * e + 1] = x.y;
+    }
   put_state(S);
 
   int buf = 0;
   for (int t0 = start; t0 < end; t0 += L, buf ^= 1) {
     cp_async_wait<0>();
-    block_barrier();                                // the chunk's operands and decays and the state's parts are there
+    block_barrier<THREADS>();                                // the chunk's operands and decays and the state's parts are there
     if (t0 + L < end) request(t0 + L, buf ^ 1);
     // C B^T of this warp's causal tiles, C S^T of its columns
-    float cb[4][4], y[2][4], y_low[2][4];           // (y_low: the products of the state's lower parts)
+    float cb[NC][4], y[NY][4], y_low[NY][4];           // (y_low: the products of the state's lower parts)
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
+    for (int n = 0; n < NC; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) cb[n][e] = 0.f;
 #pragma unroll
-    for (int n = 0; n < 2; ++n)
+    for (int n = 0; n < NY; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) y[n][e] = y_low[n][e] = 0.f;
 #pragma unroll
@@ -205,10 +208,10 @@ chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_b
       ldmatrix_x4(a0, smem_u32(a_row + ks * 16));
       ldmatrix_x4(a1, smem_u32(a_row + ks * 16 + 16));
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        if (n <= mt) {
+      for (int n = 0; n < NC; ++n) {
+        if (part + Q * n < 2 * (mt + 1)) {
           uint32_t bb[4];
-          ldmatrix_x4(bb, smem_u32(&sm.b[buf][(half * (mt + 1) + n) * 8 + (lane & 7)][ks * 16 + (lane >> 3) * 8]));
+          ldmatrix_x4(bb, smem_u32(&sm.b[buf][(part + Q * n) * 8 + (lane & 7)][ks * 16 + (lane >> 3) * 8]));
           mma_add(cb[n], a0, bb[0], bb[1]);
           mma_add(cb[n], a1, bb[2], bb[3]);
         }
@@ -216,9 +219,9 @@ chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_b
 #pragma unroll
       for (int p = 0; p < 3; ++p)
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
+        for (int n = 0; n < NY; ++n) {
           uint32_t bb[4];
-          ldmatrix_x4(bb, smem_u32(&sm.s[p][half * 16 + n * 8 + (lane & 7)][ks * 16 + (lane >> 3) * 8]));
+          ldmatrix_x4(bb, smem_u32(&sm.s[p][(part * NY + n) * 8 + (lane & 7)][ks * 16 + (lane >> 3) * 8]));
           if (p == 0) {
             mma_add(y[n], a0, bb[0], bb[1]);
             mma_add(y[n], a1, bb[2], bb[3]);
@@ -232,7 +235,7 @@ chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_b
     {
       const float e0 = sm.eg[buf][row], e1 = sm.eg[buf][row + 8];
 #pragma unroll
-      for (int n = 0; n < 2; ++n)
+      for (int n = 0; n < NY; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           y[n][e] = (y[n][e] + y_low[n][e]) * (e < 2 ? e0 : e1);
@@ -240,9 +243,9 @@ chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_b
         }
       const float h0 = sm.g_hi[buf][row], l0 = sm.g_lo[buf][row], h1 = sm.g_hi[buf][row + 8], l1 = sm.g_lo[buf][row + 8];
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        if (n <= mt) {
-          const int c = (half * (mt + 1) + n) * 8 + gc;
+      for (int n = 0; n < NC; ++n) {
+        if (part + Q * n < 2 * (mt + 1)) {
+          const int c = (part + Q * n) * 8 + gc;
           float val[4];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
@@ -252,44 +255,52 @@ chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_b
           }
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            uint32_t part[3];
-            split3(val[2 * e], val[2 * e + 1], part[0], part[1], part[2]);
+            uint32_t parts[3];
+            split3(val[2 * e], val[2 * e + 1], parts[0], parts[1], parts[2]);
 #pragma unroll
-            for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(&sm.m[p][row + 8 * e][c]) = part[p];
+            for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(&sm.m[p][row + 8 * e][c]) = parts[p];
           }
         }
       }
-      const int t = tid >> 2, p0 = (tid & 3) * 8;
-      const float w = sm.w[buf][t];
-      uint4 raw = *reinterpret_cast<const uint4*>(&sm.x[buf][t][p0]);
-      const uint32_t in[4] = {raw.x, raw.y, raw.z, raw.w};
-      uint32_t parts[3][4];
+      if (tid < L * COLS / 8) {                     // (with 16 warps: those with the fewer causal tiles)
+        const int t = tid >> 2, p0 = (tid & 3) * 8;
+        const float w = sm.w[buf][t];
+        uint4 raw = *reinterpret_cast<const uint4*>(&sm.x[buf][t][p0]);
+        const uint32_t in[4] = {raw.x, raw.y, raw.z, raw.w};
+        uint32_t parts[3][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const __nv_bfloat162 two = *reinterpret_cast<const __nv_bfloat162*>(&in[i]);
-        split3(__low2float(two) * w, __high2float(two) * w, parts[0][i], parts[1][i], parts[2][i]);
+        for (int i = 0; i < 4; ++i) {
+          const __nv_bfloat162 two = *reinterpret_cast<const __nv_bfloat162*>(&in[i]);
+          split3(__low2float(two) * w, __high2float(two) * w, parts[0][i], parts[1][i], parts[2][i]);
+        }
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+          *reinterpret_cast<uint4*>(&sm.xw[p][t][p0]) = make_uint4(parts[p][0], parts[p][1], parts[p][2], parts[p][3]);
       }
-#pragma unroll
-      for (int p = 0; p < 3; ++p)
-        *reinterpret_cast<uint4*>(&sm.xw[p][t][p0]) = make_uint4(parts[p][0], parts[p][1], parts[p][2], parts[p][3]);
     }
     const float loss = sm.loss[buf], keep = sm.keep[buf];
-    block_barrier();                                // M and the weighted x are there; nobody reads the state's parts any more
+    block_barrier<THREADS>();                                // M and the weighted x are there; nobody reads the state's parts any more
 #pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
-      if (ks <= mt) {
-        uint32_t bb[4];
-        ldmatrix_x4_trans(bb, smem_u32(&sm.x[buf][ks * 16 + (lane & 15)][half * 16 + (lane >> 4) * 8]));
+    for (int ks = 0; ks < 4; ks += 2) {
+      if (ks > mt) break;
+      uint32_t bb[2][NY][2];                        // [k step][tile]
+#pragma unroll
+      for (int n = 0; n < NY; ++n) {
+        uint32_t both[4];
+        ldmatrix_x4_trans(both, smem_u32(&sm.x[buf][ks * 16 + lane][(part * NY + n) * 8]));
+        bb[0][n][0] = both[0], bb[0][n][1] = both[1], bb[1][n][0] = both[2], bb[1][n][1] = both[3];
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (ks + j > mt) break;
 #pragma unroll
         for (int p = 0; p < 3; ++p) {
           uint32_t a[4];
-          ldmatrix_x4(a, smem_u32(&sm.m[p][mt * 16 + (lane & 15)][ks * 16 + (lane >> 4) * 8]));
-          if (p == 0) {
-            mma_add(y[0], a, bb[0], bb[1]);
-            mma_add(y[1], a, bb[2], bb[3]);
-          } else {
-            mma_bf16(y_low[0], a, bb[0], bb[1]);
-            mma_bf16(y_low[1], a, bb[2], bb[3]);
+          ldmatrix_x4(a, smem_u32(&sm.m[p][mt * 16 + (lane & 15)][(ks + j) * 16 + (lane >> 4) * 8]));
+#pragma unroll
+          for (int n = 0; n < NY; ++n) {
+            if (p == 0) mma_add(y[n], a, bb[j][n][0], bb[j][n][1]);
+            else mma_bf16(y_low[n], a, bb[j][n][0], bb[j][n][1]);
           }
         }
       }
@@ -298,32 +309,22 @@ chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_b
     for (int e = 0; e < 2; ++e) {
       const int t = t0 + row + 8 * e;
       if (t < end) {
-        float* dst = out + (int64_t)t * out_stride + (int64_t)h * dv + col0 + half * 16 + gc;
+        float* dst = out + (int64_t)t * out_stride + (int64_t)h * dv + col0 + part * NY * 8 + gc;
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
-          *reinterpret_cast<float2*>(dst + n * 8) = make_float2((y[n][2 * e] + y_low[n][2 * e]) * q_scale, (y[n][2 * e + 1] + y_low[n][2 * e + 1]) * q_scale);
+        for (int n = 0; n < NY; ++n)
+          *reinterpret_cast<float2*>(dst + n * 8) = make_float2((y[n][2 * e] + y_low[n][2 * e]) * q_scale,
+                                                                (y[n][2 * e + 1] + y_low[n][2 * e + 1]) * q_scale);
       }
     }
-    float add[2][NT][4], add_low[2][NT][4];
+    float add[2][4], add_low[2][4];
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
-      for (int n = 0; n < NT; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) add[m][n][e] = add_low[m][n][e] = 0.f;
+      for (int e = 0; e < 4; ++e) add[m][e] = add_low[m][e] = 0.f;
 #pragma unroll
     for (int ks = 0; ks < 4; ks += 2) {
-      uint32_t bb[2][4];                            // tiles of B: [k step][tile 0: two, tile 1: two]
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        if (NT == 2) {
-          ldmatrix_x4_trans(bb[j], smem_u32(&sm.b[buf][(ks + j) * 16 + (lane & 15)][warp * 16 + (lane >> 4) * 8]));
-        } else if (j == 0) {
-          uint32_t both[4];
-          ldmatrix_x4_trans(both, smem_u32(&sm.b[buf][ks * 16 + lane][warp * 8]));
-          bb[0][0] = both[0], bb[0][1] = both[1], bb[1][0] = both[2], bb[1][1] = both[3];
-        }
-      }
+      uint32_t bb[4];                               // this warp's columns of B: [k step: two]
+      ldmatrix_x4_trans(bb, smem_u32(&sm.b[buf][ks * 16 + lane][warp * 8]));
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -332,32 +333,25 @@ chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_b
           for (int m = 0; m < 2; ++m) {
             uint32_t a[4];
             ldmatrix_x4_trans(a, smem_u32(&sm.xw[p][(ks + j) * 16 + (lane >> 4) * 8 + (lane & 7)][m * 16 + ((lane >> 3) & 1) * 8]));
-#pragma unroll
-            for (int n = 0; n < NT; ++n) {
-              if (p == 0) mma_add(add[m][n], a, bb[j][2 * n], bb[j][2 * n + 1]);
-              else mma_bf16(add_low[m][n], a, bb[j][2 * n], bb[j][2 * n + 1]);
-            }
+            if (p == 0) mma_add(add[m], a, bb[2 * j], bb[2 * j + 1]);
+            else mma_bf16(add_low[m], a, bb[2 * j], bb[2 * j + 1]);
           }
     }
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
-      for (int n = 0; n < NT; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float sum = add[m][n][e] + add_low[m][n][e];
-          // (a slow state loses little and is changed by that little; a fast one is mostly replaced)
-          S[m][n][e] = loss < 0.5f ? S[m][n][e] + fmaf(-loss, S[m][n][e], sum) : fmaf(keep, S[m][n][e], sum);
-        }
+      for (int e = 0; e < 4; ++e) {
+        const float sum = add[m][e] + add_low[m][e];
+        // (a slow state loses little and is changed by that little; a fast one is mostly replaced)
+        S[m][e] = loss < 0.5f ? S[m][e] + fmaf(-loss, S[m][e], sum) : fmaf(keep, S[m][e], sum);
+      }
     if (t0 + L < end) put_state(S);
   }
 #pragma unroll
   for (int m = 0; m < 2; ++m)
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-        *reinterpret_cast<float2*>(sp + (int64_t)(m * 16 + 8 * e) * DK + n * 8) = make_float2(S[m][n][2 * e], S[m][n][2 * e + 1]);
+    for (int e = 0; e < 2; ++e)
+      *reinterpret_cast<float2*>(sp + (int64_t)(m * 16 + 8 * e) * DK) = make_float2(S[m][2 * e], S[m][2 * e + 1]);
 }
 
 // Whether chunk_kernel takes these operands: bfloat16 rows on 16-byte boundaries, 64 or 128 key channels, value columns
@@ -378,7 +372,7 @@ inline int launch(const __nv_bfloat16* q, int64_t q_stride, const __nv_bfloat16*
   const size_t smem = dk == 64 ? sizeof(Smem<64>) : sizeof(Smem<128>);
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  return gllm_launch(kernel, dim3(dv / COLS, heads, requests), dim3(THREADS + 32), smem, stream, q, q_stride, k, k_stride, v,
+  return gllm_launch(kernel, dim3(dv / COLS, heads, requests), dim3(dk * 4 + 32), smem, stream, q, q_stride, k, k_stride, v,
                      v_stride, gates, gates_stride, gate_bias, rate, q_scale, state, cu_q, state_slots, out, out_stride,
                      heads, dv, kv_div, from);
 }
