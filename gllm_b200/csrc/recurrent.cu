@@ -28,17 +28,18 @@
 // heads of 64 x 128: y 9.7e-8, state 1.1e-7 (1.3e-7 and 1.1e-7 token by token); decays a hundred times slower 8.7e-8 and
 // 9.2e-8 (2.0e-7 and 6.4e-7).  With the tensor cores adding into long-lived accumulators they were 6.1e-7 and 2.5e-7.
 //
-// A block takes 32 value columns of one (request, head) with a warp for every 8 key channels (16 or 8 warps).  The warps
-// share each 16 rows of the chunk (its causal tiles of C B^T, then the columns of y) and each owns 8 columns of the state.
-// The next chunk's C, B and x are copied and its decays summed (by one more warp) while this one is computed.  What bounds
-// it: the chain of a chunk, 4.2 us of two barriers around products whose operands are read from shared memory (about
-// 510 KB a chunk: half of that time; tensor pipe 22 % busy), times the chunks of the longest request; token by token a chunk
-// is a chain of 64 steps, 23 us.  2,048 tokens of one request, 64 heads of 64 x 128: 135 us against 727 (142 with eight
-// warps of 16 state columns); with eight warps four of 512: 147 against 672; 64: 17 against 28.
+// A block takes 32 value columns of one (request, head) with two warps for every 16 key channels (16 or 8 warps).  The
+// warps share each 16 rows of the chunk (its causal tiles of C B^T, then the columns of y) and each owns 16 x 16 of the
+// state.  The next chunk's C, B and x are copied and its decays summed (by one more warp) while this one is computed.
+// What bounds it: the chain of a chunk, 3.9 us of two barriers around products whose operands come from shared memory
+// (430 KB a chunk, whose reads keep that pipe busy half of the time), times the chunks of the longest request; token by
+// token a chunk is a chain of 64 steps, 23 us.  2,048 tokens of one request, 64 heads of 64 x 128: 125 us against 727
+// (142 with eight warps; 135 with sixteen that read the weighted x, in three parts, as the operand of 16 x 8 tiles: here
+// B is, which has one part).  With eight warps four requests of 512: 147 against 672; 64: 17 against 28.
 
 namespace ssd {
 constexpr int L = 64, COLS = 32;
-// a warp for every 8 state columns, and one more for the decays
+// two warps for every 16 key channels, and one more for the decays
 template <int DK> constexpr int THREADS_OF = DK * 4;
 constexpr int XP = COLS + 8, MP = L + 8;            // rows padded by 16 bytes: ldmatrix without bank conflicts
 
@@ -77,6 +78,13 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t&
   const __nv_bfloat162 l = __floats2bfloat162_rn(ra - __low2float(m), rb - __high2float(m));
   hi = *reinterpret_cast<const uint32_t*>(&h), mid = *reinterpret_cast<const uint32_t*>(&m),
   lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// Four 8 x 8 tiles of packed pairs to shared memory, each transposed; every lane gives the address of one stored row.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, const uint32_t (&r)[4]) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3])
+               : "memory");
 }
 
 template <int DK>
@@ -118,17 +126,19 @@ chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_b
     }
     cp_async_commit();
   };
+  // This warp's state: key channels dk0 + gr (+ 8), value columns c0 + 8 n + gc (+ 1).  It goes to shared memory column by
+  // column: a tile's rows are key channels here and value columns there.
+  const int dk0 = (warp >> 1) * 16, c0 = (warp & 1) * 16;
   auto put_state = [&](const float (&S)[2][4]) {
+    uint32_t parts[3][4];                           // [part][tile n, rows gr or gr + 8]
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        uint32_t parts[3];
-        split3(S[m][2 * e], S[m][2 * e + 1], parts[0], parts[1], parts[2]);
+      for (int e = 0; e < 2; ++e)
+        split3(S[n][2 * e], S[n][2 * e + 1], parts[0][2 * n + e], parts[1][2 * n + e], parts[2][2 * n + e]);
 #pragma unroll
-        for (int p = 0; p < 3; ++p)
-          *reinterpret_cast<uint32_t*>(&sm.s[p][m * 16 + gr + 8 * e][warp * 8 + gc]) = parts[p];
-      }
+    for (int p = 0; p < 3; ++p)
+      stmatrix_x4_trans(smem_u32(&sm.s[p][c0 + (lane >> 4) * 8 + (lane & 7)][dk0 + ((lane >> 3) & 1) * 8]), parts[p]);
   };
 
   if (warp == THREADS / 32) {
@@ -176,14 +186,11 @@ chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_b
   }
   request(start, 0);
   float S[2][4];
-  float* sp = state + (((int64_t)state_slots[r] * heads + h) * dv + col0 + gr) * DK + warp * 8 + gc;
+  float* sp = state + (((int64_t)state_slots[r] * heads + h) * dv + col0 + c0 + gc) * DK + dk0 + gr;
 #pragma unroll
-  for (int m = 0; m < 2; ++m)
+  for (int n = 0; n < 2; ++n)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const float2 x = *reinterpret_cast<const float2*>(sp + (int64_t)(m * 16 + 8 * e) * DK);
-      S[m][2 * e] = x.x, S[m][2 * e + 1] = x.y;
-    }
+    for (int e = 0; e < 4; ++e) S[n][e] = sp[(n * 8 + (e & 1)) * DK + (e >> 1) * 8];
   put_state(S);
 
   int buf = 0;
@@ -318,40 +325,38 @@ chunk_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_b
     }
     float add[2][4], add_low[2][4];
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) add[m][e] = add_low[m][e] = 0.f;
+      for (int e = 0; e < 4; ++e) add[n][e] = add_low[n][e] = 0.f;
 #pragma unroll
-    for (int ks = 0; ks < 4; ks += 2) {
-      uint32_t bb[4];                               // this warp's columns of B: [k step: two]
-      ldmatrix_x4_trans(bb, smem_u32(&sm.b[buf][ks * 16 + lane][warp * 8]));
+    for (int ks = 0; ks < 4; ++ks) {                // B^T (16 key channels) times the weighted x (16 columns)
+      uint32_t a[4];
+      ldmatrix_x4_trans(a, smem_u32(&sm.b[buf][ks * 16 + (lane >> 4) * 8 + (lane & 7)][dk0 + ((lane >> 3) & 1) * 8]));
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
+      for (int p = 0; p < 3; ++p) {
+        uint32_t bb[4];
+        ldmatrix_x4_trans(bb, smem_u32(&sm.xw[p][ks * 16 + (lane & 15)][c0 + (lane >> 4) * 8]));
 #pragma unroll
-        for (int p = 0; p < 3; ++p)
-#pragma unroll
-          for (int m = 0; m < 2; ++m) {
-            uint32_t a[4];
-            ldmatrix_x4_trans(a, smem_u32(&sm.xw[p][(ks + j) * 16 + (lane >> 4) * 8 + (lane & 7)][m * 16 + ((lane >> 3) & 1) * 8]));
-            if (p == 0) mma_add(add[m], a, bb[2 * j], bb[2 * j + 1]);
-            else mma_bf16(add_low[m], a, bb[2 * j], bb[2 * j + 1]);
-          }
+        for (int n = 0; n < 2; ++n) {
+          if (p == 0) mma_add(add[n], a, bb[2 * n], bb[2 * n + 1]);
+          else mma_bf16(add_low[n], a, bb[2 * n], bb[2 * n + 1]);
+        }
+      }
     }
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float sum = add[m][e] + add_low[m][e];
+        const float sum = add[n][e] + add_low[n][e];
         // (a slow state loses little and is changed by that little; a fast one is mostly replaced)
-        S[m][e] = loss < 0.5f ? S[m][e] + fmaf(-loss, S[m][e], sum) : fmaf(keep, S[m][e], sum);
+        S[n][e] = loss < 0.5f ? S[n][e] + fmaf(-loss, S[n][e], sum) : fmaf(keep, S[n][e], sum);
       }
     if (t0 + L < end) put_state(S);
   }
 #pragma unroll
-  for (int m = 0; m < 2; ++m)
+  for (int n = 0; n < 2; ++n)
 #pragma unroll
-    for (int e = 0; e < 2; ++e)
-      *reinterpret_cast<float2*>(sp + (int64_t)(m * 16 + 8 * e) * DK) = make_float2(S[m][2 * e], S[m][2 * e + 1]);
+    for (int e = 0; e < 4; ++e) sp[(n * 8 + (e & 1)) * DK + (e >> 1) * 8] = S[n][e];
 }
 
 // Whether chunk_kernel takes these operands: bfloat16 rows on 16-byte boundaries, 64 or 128 key channels, value columns
