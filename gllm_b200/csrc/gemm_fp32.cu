@@ -1,25 +1,31 @@
-// True 32-bit matrix product on the CUDA cores: C[M,N] = A[M,K] * B[N,K]^T,
-// the `x @ W.T` of gllm/model/layers/linear.py:20 with W stored [out, in].
+// True 32-bit matrix product C[M,N] = X[M,K] * W[N,K]^T, the `x @ W.T` of
+// gllm/model/layers/linear.py:20 with W stored [out, in].  This is the path
+// that shows faults bf16 hides: no operand is rounded.
 //
-// No tensor-core mode of any kind (no TF32): every product is a 32-bit fused
-// multiply-add.  Each output element is accumulated by one thread in an order
-// that does not depend on M, so a token's result does not depend on the batch
-// it is in.  This is the reference path that shows faults bf16 hides.  Two
-// kernels: tiles of 16 x 16 to 64 x 64 outputs on packed multiply-adds with
-// asynchronous copies (rows 16-byte aligned, K a multiple of 4), and a plain
-// 64 x 64 tile for everything else (k = 0..K-1 in ascending order).
+// Two kernels.  Rows on 16-byte boundaries and K a multiple of 4 run on the
+// tensor cores with every 32-bit number cut into three bfloat16 whose sum it
+// is (8 bits of its significand each, rounded to nearest, so nothing is lost):
+//   x = x0 + x1 + x2,  w = w0 + w1 + w2,
+//   x w = w0 x0 + (w0 x1 + w1 x0 + w0 x2 + w1 x1 + w2 x0) + terms below 2^-26 |x w|.
+// Everything else runs a plain 64 x 64 tile of 32-bit multiply-adds.
 //
-// What bounds the packed kernel: the multiply-add pipe (74 TFLOP/s at 128 a
-// clock and SM; a loop of nothing but packed multiply-adds reaches 105 a
-// clock) and the latency from one multiply-add to the next with few warps; the
-// shared-memory loads keep their pipe half busy.  2,048 x 8,192 x 2,048:
-// 1,413 us = 48.6 TFLOP/s, 1,909 us = 36.0 with a 128 x 128 tile of scalar
-// multiply-adds and one k-tile in flight; 700 x 2,048 x 8,192: 626 against
-// 1,097 us; 8 x 16,384 x 2,048: 64 against 381.  Error against 64 bits at
-// K = 2,048: 5.7e-7 (two partial sums) against 8.1e-7.
-#include "common.cuh"
+// The tensor cores' own additions truncate.  The leading products' accumulator
+// is therefore taken out of tensor memory every 256 of K (16 additions) and
+// added to 32-bit sums in registers, rounded to nearest; the other five
+// products are 2^-8 of it and stay in theirs for a whole range of K.
+//
+// K is cut into ranges that depend on (N, K) alone.  A work item is a tile of
+// 128 weight rows x BT tokens times one range (few tokens: the unsummed parts
+// go to scratch) or all ranges one after the other; the ranges' sums are added
+// in ascending order either way, so a token's result does not depend on the
+// batch it is in.
+//
+// A result that is not finite is computed again with 32-bit multiply-adds from
+// the operands themselves: the parts of an infinity are not its sum.
+#include "umma_utils.cuh"
 
 namespace {
+// ------------------------------------------------------------------ plain tile
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;  // 256 threads
 
 __global__ void __launch_bounds__(256)
@@ -76,161 +82,536 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
   }
 }
 
-// ---- tiles whose rows lie in shared memory as they do in memory, [row][k], filled by cp.async several k-tiles ahead.
-// A thread owns TM x TN outputs (rows and columns TY and TX apart).  Four k at a time it reads 16 bytes of each of its
-// rows and multiplies them as two packed pairs (fma.rn.f32x2), so an output is kept as two sums, of the products with
-// even and with odd k, each in ascending order; they are added at the end.
-constexpr int PK = 32, PITCH = PK + 4;   // (a pitch of 9 sixteen-byte pieces: eight neighbouring rows on eight bank groups)
+// ------------------------------------------------------------------ three parts a number, on the tensor cores
+namespace parts3 {
+constexpr int ROWS = 128;           // weight rows of a tile (MMA M)
+constexpr int KB = 32;              // k per block: 32 floats = one 128-byte swizzle row, 32 bf16 = one of 64 bytes
+constexpr int CHUNK = 8;            // blocks between two visits to the leading accumulator
+constexpr int WORKERS = 16;         // warps that cut operands into parts and keep the sums
+constexpr int GROUPS = 4;           // of workers, that take turns with the blocks
+constexpr int CUT = 4;              // blocks of parts in flight (no fewer than GROUPS: a group waits for one phase of a stage)
+constexpr int THREADS = (WORKERS + 2) * 32;
+constexpr int RANGE_BLOCKS = 64;    // longest range of K (2,048), as long as there are at most 16 of them
+constexpr int MOST_RANGES = 16;
+constexpr int A_COLS = 3 * KB / 2;  // tensor-memory columns of one block of the weight's parts
 
-template <int BM_, int BN_, int TM_, int TN_, int STAGES, int UNROLL>
-__global__ void __launch_bounds__((BM_ / TM_) * (BN_ / TN_))
-gemm_f32_pairs_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M, int N,
-                      int K, int64_t lda, int64_t ldb, int64_t ldc) {
-  constexpr int TY = BM_ / TM_, TX = BN_ / TN_, THREADS = TX * TY, ROWS = BM_ + BN_;
-  static_assert(TX % 8 == 0 && TY % 4 == 0, "a warp's threads lie 4 by 8");
-  extern __shared__ __align__(16) float tiles[];          // [STAGES][BM_ + BN_][PITCH]
-  pdl_trigger();
-  // A warp's threads lie 4 rows by 8 columns, a half warp 4 by 4: a 16-byte load is served a half warp at a time when
-  // its addresses fit one pass over the banks, so neither operand's load takes more than two.
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tx = (warp % (TX / 8)) * 8 + (lane & 3) + (lane >> 4) * 4, ty = (warp / (TX / 8)) * 4 + ((lane >> 2) & 3);
-  const int m0 = blockIdx.y * BM_, n0 = blockIdx.x * BN_;
-  // a thread copies piece `piece` of the rows row0, row0 + STEP, ...: of A's first, of B's behind them
-  constexpr int PIECES = PK / 4, STEP = THREADS / PIECES, COPIES = ROWS / STEP;
-  static_assert(THREADS % PIECES == 0 && BM_ % STEP == 0 && BN_ % STEP == 0, "whole rows per round of copies");
-  const int piece = tid % PIECES, row0 = tid / PIECES;
-  const float* a_src = A + (int64_t)(m0 + row0) * lda + piece * 4;
-  const float* b_src = B + (int64_t)(n0 + row0) * ldb + piece * 4;
-  const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(tiles) + (uint32_t)((row0 * PITCH + piece * 4) * sizeof(float));
-  auto request = [&](int k0, int stage) {
-    const bool k_in = k0 + piece * 4 < K;
-    const uint32_t dst = dst0 + (uint32_t)(stage * ROWS * PITCH * sizeof(float));
+template <int BT>
+struct Shape {
+  static constexpr int RAW = (ROWS + BT) * KB * 4;
+  static constexpr int PARTS = ((3 * BT * KB * 2 + 1023) / 1024) * 1024;
+  static constexpr int STAGES_ = (216 * 1024 - CUT * PARTS) / RAW;
+  static constexpr int STAGES = STAGES_ > 8 ? 8 : STAGES_;                 // raw blocks in flight
+  static constexpr int CROSS = BT <= 64 ? 2 : 1;                           // accumulators of the five smaller products
+  static constexpr int COLS = (2 + CROSS) * BT + CUT * A_COLS;
+  static constexpr int TMEM_COLS = COLS <= 256 ? 256 : 512;
+  static constexpr int SMEM = STAGES * RAW + CUT * PARTS + 1024;
+  static_assert(COLS <= 512 && STAGES >= GROUPS, "fits");
+};
+
+// Shared-memory descriptor of a K-major tile with rows of 64 bytes, 64-byte swizzle, 8-row groups 512 bytes apart.
+__device__ __forceinline__ uint64_t desc64(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) | ((uint64_t)1 << 46) |
+         ((uint64_t)4 << 61);
+}
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t (&r)[4]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld4_nowait(uint32_t taddr, float* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, float* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "r"(taddr));
+}
+// sum[i] += the accumulator's columns taddr + i of this thread's row
+template <int C>
+__device__ __forceinline__ void add_columns(uint32_t taddr, float (&sum)[C]) {
+  constexpr int STEP = C % 8 == 0 ? 8 : 4;
 #pragma unroll
-    for (int c = 0; c < COPIES; ++c) {
-      const bool is_a = c < BM_ / STEP;
-      const int r = is_a ? c * STEP : c * STEP - BM_;
-      const bool in = k_in && (is_a ? m0 + row0 + r < M : n0 + row0 + r < N);
-      const float* src = is_a ? a_src + k0 + r * lda : b_src + k0 + r * ldb;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)(c * STEP * PITCH * sizeof(float))),
-                   "l"(in ? src : A), "r"(in ? 16 : 0) : "memory");
+  for (int c = 0; c < C; c += STEP) {
+    float v[STEP];
+    if constexpr (STEP == 8) tmem_ld8_nowait(taddr + (uint32_t)c, v);
+    else tmem_ld4_nowait(taddr + (uint32_t)c, v);
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < STEP; ++i) {
+      asm volatile("" : "+f"(v[i])::"memory");             // (not read ahead of the wait)
+      sum[c + i] += v[i];
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  unsigned long long acc[TM_][TN_];
-#pragma unroll
-  for (int i = 0; i < TM_; ++i)
-#pragma unroll
-    for (int j = 0; j < TN_; ++j) acc[i][j] = 0ull;
-  const int k_tiles = (K + PK - 1) / PK;
-  pdl_wait();
-#pragma unroll
-  for (int t = 0; t < STAGES - 1; ++t) {
-    if (t < k_tiles) request(t * PK, t);
-    else asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  int stage = 0;
-  for (int t = 0; t < k_tiles; ++t) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-    __syncthreads();                                       // tile t is there, and nobody reads tile t - 1 any more
-    const int ahead = t + STAGES - 1;
-    if (ahead < k_tiles) request(ahead * PK, stage == 0 ? STAGES - 1 : stage - 1);
-    else asm volatile("cp.async.commit_group;" ::: "memory");
-    const float* a_s = tiles + (stage * ROWS + ty) * PITCH;
-    const float* b_s = tiles + (stage * ROWS + BM_ + tx) * PITCH;
-#pragma unroll UNROLL
-    for (int kk = 0; kk < PK; kk += 4) {
-      ulonglong2 a[TM_];
+}
+
+__device__ __forceinline__ uint32_t pack2(float low, float high) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(low, high);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+// Eight numbers as three parts each, two to a word.
+__device__ __forceinline__ void cut8(const float4& a, const float4& b, uint32_t (&p)[3][4]) {
+  float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-      for (int i = 0; i < TM_; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(a_s + i * TY * PITCH + kk);
+  for (int i = 0; i < 4; ++i) {
+    float lo = x[2 * i], hi = x[2 * i + 1];
 #pragma unroll
-      for (int j = 0; j < TN_; ++j) {
-        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(b_s + j * TX * PITCH + kk);
+    for (int part = 0; part < 3; ++part) {
+      const uint32_t w = pack2(lo, hi);
+      p[part][i] = w;
+      lo -= __uint_as_float(w << 16);                      // (exact: what is left has no more bits than the number had)
+      hi -= __uint_as_float(w & 0xffff0000u);
+    }
+  }
+}
+
+struct Cut {                        // how the work is laid out
+  int tiles_n, tiles_m;             // tiles of weight rows, of tokens
+  int ranges, range_blocks, blocks; // of K
+  int split;                        // 1: an item is one range of a tile; 0: all of them
+};
+
+// Item w: neighbouring CTAs share a tile of weight rows (or take the ranges of one).
+template <int BT>
+__device__ __forceinline__ void place(const Cut& cut, int w, int& n0, int& m0, int& kb_begin, int& kb_end, int& range) {
+  range = 0;
+  if (cut.split) {
+    range = w % cut.ranges;
+    w /= cut.ranges;
+  }
+  const int tn = w / cut.tiles_m, tm = w - tn * cut.tiles_m;
+  n0 = tn * ROWS, m0 = tm * BT;
+  kb_begin = cut.split ? range * cut.range_blocks : 0;
+  kb_end = cut.split ? min(cut.blocks, kb_begin + cut.range_blocks) : cut.blocks;
+}
+
+// Results of an item that are not finite, once more with 32-bit multiply-adds: token m's, weight row n's at dst[0], of the
+// next tokens behind it.
+__device__ __noinline__ void again(float* dst, int64_t ldo, int tokens, const float* __restrict__ x, int64_t ldx,
+                                   const float* __restrict__ w, int k0, int k1) {
+  for (int i = 0; i < tokens; ++i, dst += ldo, x += ldx) {
+    if ((__float_as_uint(__ldcg(dst)) & 0x7f800000u) != 0x7f800000u) continue;
+    float s = 0.f;
+    for (int k = k0; k < k1; k += 4) {
+      const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
+      s = fmaf(a.x, b.x, s), s = fmaf(a.y, b.y, s), s = fmaf(a.z, b.z, s), s = fmaf(a.w, b.w, s);
+    }
+    *dst = s;
+  }
+}
+// The sum of a range of an item, columns c0 .. of one of its rows: behind the item's first range it joins what this thread
+// has written of the ranges before.
+template <int BT, int COLS>
+__device__ __forceinline__ void put_range(const Cut& cut, int item, int end, int row, int c0, const float (&acc)[COLS],
+                                          const float* __restrict__ X, const float* __restrict__ W, float* out, int M, int N,
+                                          int K, int64_t ldx, int64_t ldw, int64_t ldo, bool& broken) {
+  int n0, m0, kb_begin, kb_end, range;
+  place<BT>(cut, item, n0, m0, kb_begin, kb_end, range);
+  const int n = n0 + row, m = m0 + c0, tokens = min(COLS, M - m);
+  if (n >= N || tokens <= 0) return;
+  float* const dst = out + (int64_t)range * M * N + (int64_t)m * ldo + n;
+  const bool joins = end - kb_begin > cut.range_blocks;
 #pragma unroll
-        for (int i = 0; i < TM_; ++i) fma2(acc[i][j], a[i].x, b.x);
-#pragma unroll
-        for (int i = 0; i < TM_; ++i) fma2(acc[i][j], a[i].y, b.y);
+  for (int i = 0; i < COLS; ++i) {
+    if (i < tokens) {
+      const float v = acc[i];
+      broken = broken || (__float_as_uint(v) & 0x7f800000u) == 0x7f800000u;
+      if (joins) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + i * ldo), "f"(v) : "memory");   // (nothing to wait for)
+      else dst[i * ldo] = v;
+    }
+  }
+  if (end != kb_end) return;
+  if (broken)
+    again(dst, ldo, tokens, X + (int64_t)m * ldx, ldx, W + (int64_t)n * ldw, kb_begin * KB, min(K, kb_end * KB));
+  broken = false;
+}
+
+// Warps 0..15 cut the operands into parts (the weight's into tensor memory, the MMA's A operand; the tokens' into shared
+// memory, its B operand) and keep the sums: warp w the tile's rows 32 (w % 4) .. and a quarter of its columns.  Warp 16
+// requests the operands by TMA, warp 17 issues the products.  Weight parts in tensor memory: a product of 16 tokens
+// then takes 16 cycles, with both operands in shared memory 40; of 96 tokens 49 cycles for 3 KB of shared memory instead of 7, and
+// what is left of the 128 bytes a cycle is needed for the cutting.
+template <int BT>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                      const float* __restrict__ X, const float* __restrict__ W, float* __restrict__ out, int M, int N, int K,
+                      int64_t ldx, int64_t ldw, int64_t ldo, Cut cut, int num_items, int* __restrict__ status) {
+  using S = Shape<BT>;
+  constexpr int COLS = BT / 4;      // columns of a worker
+  extern __shared__ unsigned char smem_dyn[];
+  __shared__ __align__(8) uint64_t raw_full[S::STAGES], raw_empty[S::STAGES], cut_full[CUT], cut_empty[CUT], main_full[2],
+      main_empty[2], cross_empty[S::CROSS];
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ int abort_flag;
+
+  pdl_trigger();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t raw_base = (smem_addr(smem_dyn) + 1023u) & ~1023u, parts_base = raw_base + S::STAGES * S::RAW;
+  unsigned char* raw_ptr = smem_dyn + (raw_base - smem_addr(smem_dyn));
+  unsigned char* parts_ptr = raw_ptr + S::STAGES * S::RAW;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S::STAGES; ++s) mbar_init(smem_addr(&raw_full[s]), 1), mbar_init(smem_addr(&raw_empty[s]), WORKERS / GROUPS);
+    for (int s = 0; s < CUT; ++s) mbar_init(smem_addr(&cut_full[s]), WORKERS / GROUPS), mbar_init(smem_addr(&cut_empty[s]), 1);
+    for (int b = 0; b < 2; ++b) mbar_init(smem_addr(&main_full[b]), 1), mbar_init(smem_addr(&main_empty[b]), WORKERS);
+    for (int b = 0; b < S::CROSS; ++b) mbar_init(smem_addr(&cross_empty[b]), WORKERS);
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == WORKERS + 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_slot)),
+                 "r"((uint32_t)S::TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_main = tmem_base_slot, tmem_cross = tmem_main + 2 * BT, tmem_parts = tmem_cross + S::CROSS * BT;
+
+  if (warp == WORKERS) {
+    // ------------------------------------------------------------ operands by TMA
+    if (lane == 0) {
+      uint32_t it = 0;
+      bool ok = true;
+      // pass 0: the weight blocks of the first STAGES stages, which no kernel before this one writes; pass 1: their tokens,
+      // then both operands of every later block as stages come free
+      for (int pass = 0; pass < 2 && ok; ++pass) {
+        if (pass == 1) pdl_wait();
+        it = 0;
+        bool more = true;
+        for (int w = blockIdx.x; w < num_items && ok && more; w += gridDim.x) {
+          int n0, m0, kb_begin, kb_end, range;
+          place<BT>(cut, w, n0, m0, kb_begin, kb_end, range);
+          for (int kb = kb_begin; kb < kb_end; ++kb, ++it) {
+            const uint32_t s = it % S::STAGES, round = it / S::STAGES, bar = smem_addr(&raw_full[s]);
+            const uint32_t dst = raw_base + s * S::RAW;
+            if (pass == 0) {
+              if (round > 0) { more = false; break; }
+              mbar_expect_tx(bar, (uint32_t)S::RAW);
+              tma_load_2d(dst, &map_w, kb * KB, n0, bar);
+            } else {
+              if (round > 0) {
+                ok = mbar_wait(smem_addr(&raw_empty[s]), (round & 1u) ^ 1u, status, &abort_flag);
+                if (!ok) break;
+                mbar_expect_tx(bar, (uint32_t)S::RAW);
+                tma_load_2d(dst, &map_w, kb * KB, n0, bar);
+              }
+              tma_load_2d(dst + ROWS * KB * 4, &map_x, kb * KB, m0, bar);
+            }
+          }
+        }
+      }
+      if (abort_flag) {
+        // let the copies already issued land before the CTA leaves (bounded)
+        const uint32_t first = it > (uint32_t)S::STAGES ? it - S::STAGES : 0u;
+        for (uint32_t i = first; i < it; ++i) {
+          const unsigned long long t0 = global_timer();
+          while (!mbar_try_wait(smem_addr(&raw_full[i % S::STAGES]), (i / S::STAGES) & 1u)) {
+            if (global_timer() - t0 > UMMA_WAIT_LIMIT_NS) break;
+          }
+        }
       }
     }
-    stage = stage + 1 == STAGES ? 0 : stage + 1;
-  }
-  asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (warp == WORKERS + 1) {
+    // ------------------------------------------------------------ products (the whole warp converged, one elected thread)
+    const bool leader = elect_one();
+    auto wait_u = [&](uint64_t* bar, uint32_t parity) -> bool {
+      return __all_sync(0xffffffffu, mbar_wait(smem_addr(bar), parity, status, &abort_flag)) != 0;
+    };
+    constexpr uint32_t idesc = umma_idesc(ROWS, BT);
+    uint32_t it = 0, chunks = 0, segments = 0;
+    bool ok = true;
+    for (int w = blockIdx.x; w < num_items && ok; w += gridDim.x) {
+      int n0, m0, kb_begin, kb_end, range;
+      place<BT>(cut, w, n0, m0, kb_begin, kb_end, range);
+      for (int r0 = kb_begin; r0 < kb_end && ok; r0 += cut.range_blocks, ++segments) {
+        const int r1 = min(kb_end, r0 + cut.range_blocks);
+        const uint32_t cb = segments % S::CROSS;
+        ok = wait_u(&cross_empty[cb], ((segments / S::CROSS) & 1u) ^ 1u);
+        if (!ok) break;
+        const uint32_t d_cross = tmem_cross + cb * BT;
+        for (int kb = r0; kb < r1; ++kb, ++it) {
+          const bool chunk_first = (kb - r0) % CHUNK == 0, chunk_last = (kb - r0) % CHUNK == CHUNK - 1 || kb + 1 == r1;
+          const uint32_t mb = chunks & 1u, d_main = tmem_main + mb * BT;
+          if (chunk_first) {
+            ok = wait_u(&main_empty[mb], ((chunks >> 1) & 1u) ^ 1u);
+            if (!ok) break;
+          }
+          const uint32_t s = it % CUT;
+          ok = wait_u(&cut_full[s], (it / CUT) & 1u);
+          if (!ok) break;
+          const uint32_t a0 = tmem_parts + s * A_COLS;
+          const uint64_t b0 = desc64(parts_base + s * S::PARTS);
+          constexpr uint64_t PART = (BT * KB * 2) >> 4;    // from one part of the tokens to the next
+          if (leader) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < TM_; ++i) {
-    const int m = m0 + ty + i * TY;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < TN_; ++j) {
-      const int n = n0 + tx + j * TX;
-      if (n < N)
-        C[(int64_t)m * ldc + n] = pair_sum(acc[i][j]);
+            for (int k = 0; k < KB / 16; ++k) {
+              const uint32_t a = a0 + k * 8;
+              const uint64_t b = b0 + (uint64_t)((k * 32) >> 4);
+              umma_bf16_ts(d_main, a, b, idesc, (!chunk_first || k > 0) ? 1u : 0u);
+              umma_bf16_ts(d_cross, a, b + PART, idesc, (kb > r0 || k > 0) ? 1u : 0u);
+              umma_bf16_ts(d_cross, a + KB / 2, b, idesc, 1u);
+              umma_bf16_ts(d_cross, a, b + 2 * PART, idesc, 1u);
+              umma_bf16_ts(d_cross, a + KB / 2, b + PART, idesc, 1u);
+              umma_bf16_ts(d_cross, a + KB, b, idesc, 1u);
+            }
+            umma_commit(smem_addr(&cut_empty[s]));
+            if (chunk_last) umma_commit(smem_addr(&main_full[mb]));
+          }
+          __syncwarp();
+          if (chunk_last) ++chunks;
+        }
+      }
     }
+  } else {
+    // ------------------------------------------------------------ parts and sums
+    pdl_wait();                                            // nothing is written before the previous kernel is done
+    // the sums: this warp's rows 32 * quarter .., columns side * COLS ..
+    const int quarter = warp & 3, side = warp >> 2;
+    const int row = quarter * 32 + lane;
+    const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+    // the parts: blocks are taken in turn by GROUPS groups of warps; of a block, a thread cuts A_K of its weight row's 32 k
+    // and B_PIECES times eight k of a token's row
+    constexpr int SIDES = WORKERS / GROUPS / 4, A_K = KB / SIDES;
+    constexpr int GROUP_THREADS = WORKERS / GROUPS * 32;
+    constexpr int B_PIECES = 4 * BT <= GROUP_THREADS ? 1 : 4 * BT <= 2 * GROUP_THREADS ? 2 : 4;
+    const uint32_t group = (uint32_t)side / SIDES;
+    const int a_side = side % SIDES;
+    const int g_tid = (int)threadIdx.x - (int)group * GROUP_THREADS;
+    const int b_row = g_tid / (4 / B_PIECES), b_piece = g_tid % (4 / B_PIECES) * B_PIECES;
+    const bool has_b = b_row < BT;                         // (whole warps)
+    float acc[COLS];
+#pragma unroll
+    for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
+    uint32_t it = 0, chunks = 0, segments = 0;
+    bool ok = true;
+    auto wait_u = [&](uint64_t* bar, uint32_t parity) -> bool {
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_addr(bar), parity, status, &abort_flag)) != 0;
+      return ok;
+    };
+    // the chunk that waits to be added: of which item; where its range ends, if with it
+    bool pending = false, broken = false;                  // (broken: a sum of this item was not finite)
+    int p_item = 0, p_end = 0, behind = 0;                 // (behind: blocks between its end and the block in hand)
+    int item = (int)blockIdx.x - (int)gridDim.x, n0, m0, kb = 0, r0 = 0, r1 = 0, kb_begin, kb_end = 0, range;
+    while (true) {
+      bool more = true;
+      if (kb == kb_end) {
+        item += gridDim.x;
+        more = item < num_items;
+        if (more) {
+          place<BT>(cut, item, n0, m0, kb_begin, kb_end, range);
+          kb = r0 = kb_begin, r1 = min(kb_end, r0 + cut.range_blocks);
+        }
+      } else if (kb == r1) {
+        r0 = r1, r1 = min(kb_end, r0 + cut.range_blocks);
+      }
+      const bool mine = more && it % GROUPS == group;
+      if (mine) {
+        const uint32_t rs = it % S::STAGES, cs = it % CUT;
+        if (!wait_u(&raw_full[rs], (it / S::STAGES) & 1u)) break;
+        const unsigned char* raw = raw_ptr + rs * S::RAW;
+        float4 a[A_K / 4];
+#pragma unroll
+        for (int j = 0; j < A_K / 4; ++j)
+          a[j] = *reinterpret_cast<const float4*>(raw + row * 128 + (((a_side * (A_K / 4) + j) ^ (row & 7)) << 4));
+        if (!wait_u(&cut_empty[cs], ((it / CUT) & 1u) ^ 1u)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t ta = tmem_parts + cs * A_COLS + lanes + a_side * (A_K / 2);
+#pragma unroll
+        for (int j = 0; j < A_K / 8; ++j) {
+          uint32_t parts[3][4];
+          cut8(a[2 * j], a[2 * j + 1], parts);
+#pragma unroll
+          for (int p = 0; p < 3; ++p) tmem_st4(ta + p * (KB / 2) + j * 4, parts[p]);
+        }
+        if (has_b) {
+          const unsigned char* b_raw = raw + ROWS * 128 + b_row * 128;
+          unsigned char* b_parts = parts_ptr + cs * S::PARTS + b_row * 64;
+#pragma unroll
+          for (int j = 0; j < B_PIECES; ++j) {
+            const int e = b_piece + j;
+            const float4 lo = *reinterpret_cast<const float4*>(b_raw + (((2 * e) ^ (b_row & 7)) << 4));
+            const float4 hi = *reinterpret_cast<const float4*>(b_raw + (((2 * e + 1) ^ (b_row & 7)) << 4));
+            uint32_t parts[3][4];
+            cut8(lo, hi, parts);
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+              *reinterpret_cast<uint4*>(b_parts + p * (BT * KB * 2) + ((e ^ ((b_row >> 1) & 3)) << 4)) =
+                  make_uint4(parts[p][0], parts[p][1], parts[p][2], parts[p][3]);
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        tmem_wait_st();
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(smem_addr(&raw_empty[rs]));
+          mbar_arrive(smem_addr(&cut_full[cs]));
+        }
+      }
+      // The chunk before is added while the products of this block run: by the CUT-th block behind it, as the stage after
+      // that comes free only behind products that may wait for these sums to be taken.
+      const bool chunk_last = more && ((kb - r0) % CHUNK == CHUNK - 1 || kb + 1 == r1);
+      if (pending && (mine || behind >= CUT - 1 || chunk_last || !more)) {
+        const uint32_t mb = chunks & 1u, cb = segments % S::CROSS;
+        if (!wait_u(&main_full[mb], (chunks >> 1) & 1u)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        add_columns<COLS>(tmem_main + mb * BT + lanes + side * COLS, acc);
+        if (p_end) add_columns<COLS>(tmem_cross + cb * BT + lanes + side * COLS, acc);
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(smem_addr(&main_empty[mb]));
+          if (p_end) mbar_arrive(smem_addr(&cross_empty[cb]));
+        }
+        ++chunks;
+        pending = false;
+        if (p_end) {
+          ++segments;
+          put_range<BT, COLS>(cut, p_item, p_end, row, side * COLS, acc, X, W, out, M, N, K, ldx, ldw, ldo, broken);
+#pragma unroll
+          for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
+        }
+      }
+      if (!more) break;
+      if (chunk_last) {
+        pending = true;
+        behind = 0;
+        p_item = item;
+        p_end = kb + 1 == r1 ? r1 : 0;
+      } else {
+        ++behind;
+      }
+      ++kb, ++it;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  }
+  __syncthreads();
+  if (warp == WORKERS + 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_main), "r"((uint32_t)S::TMEM_COLS)
+                 : "memory");
   }
 }
 
-template <int BM_, int BN_, int TM_, int TN_, int STAGES, int UNROLL>
-int gemm_f32_pairs(const float* A, const float* B, float* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
-                   cudaStream_t stream) {
-  constexpr size_t smem = sizeof(float) * STAGES * (BM_ + BN_) * PITCH;
-  auto kernel = gemm_f32_pairs_kernel<BM_, BN_, TM_, TN_, STAGES, UNROLL>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-  if (e != cudaSuccess) return (int)e;
-  // (tiles of rows lie along y, at most 65,535 a launch)
-  for (int m0 = 0; m0 < M; m0 += 65535 * BM_) {
-    const int rows = M - m0 < 65535 * BM_ ? M - m0 : 65535 * BM_;
-    const dim3 grid((N + BN_ - 1) / BN_, (rows + BM_ - 1) / BM_);
-    // Blocks that start while the kernel before them drains land wherever a place frees first.  Asking for a share of an
-    // SM's shared memory that lets no SM take more than its even share of the blocks keeps them spread.
-    const int64_t per_sm = ((int64_t)grid.x * grid.y + gllm_sm_count() - 1) / gllm_sm_count();
-    const int64_t share = 228 * 1024 / per_sm - 1024;            // (1 KB of every block's share is the system's)
-    const size_t ask = share > (int64_t)smem ? (size_t)(share < 227 * 1024 ? share : 227 * 1024) : smem;
-    const int rc = gllm_launch(kernel, grid, dim3((BM_ / TM_) * (BN_ / TN_)), ask, stream, A + (int64_t)m0 * lda, B,
-                               C + (int64_t)m0 * ldc, rows, N, K, lda, ldb, ldc);
-    if (rc != 0) return rc;
-  }
-  return 0;
-}
-}  // namespace
+// ------------------------------------------------------------------ host side
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// Which tile: the one whose fullest SM ends first.  A tile's time per k is `chain` (ns) while it has an SM to itself and
-// `work` times the tiles of the SM once they fill it; tiles of two warps count in pairs (an SM has four schedulers).
-// Measured per tile at K = 8,192 and 148 SMs (one tile an SM; 10 and more): the larger a tile the less it reads per
-// product, the smaller the better it spreads.  Steps of up to 16 tokens take the smallest tile, which streams the
-// weight best (16,384 x 2,048: 64 us against 95 with 32 x 32).
-static int pairs_tile_of(int M, int N) {
-  struct Tile { int m, n, pairs; float chain, work; };
-  static const Tile tiles[] = {{16, 16, 1, 10.4f, 3.66f}, {32, 16, 1, 13.2f, 5.2f}, {32, 32, 1, 19.4f, 7.4f},
-                               {64, 32, 1, 30.f, 13.8f}, {64, 64, 0, 33.7f, 26.4f}, {64, 64, 1, 56.4f, 25.f}};
-  if (M <= 16) return 0;
-  int best = 0;
+// A [rows, cols] fp32 matrix with `ld` elements between rows; boxes of KB columns x box_rows rows.
+bool make_map(CUtensorMap* map, const float* base, int rows, int cols, int64_t ld, int box_rows) {
+  static const EncodeTiledFn fn = []() -> EncodeTiledFn {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const bool found = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                       q == cudaDriverEntryPointSuccess;
+    return found ? (EncodeTiledFn)p : nullptr;
+  }();
+  if (!fn) return false;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+  cuuint32_t box[2] = {(cuuint32_t)KB, (cuuint32_t)box_rows};
+  cuuint32_t elem[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, elem,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Ranges of K: a function of (N, K) alone.  As many as give every SM at most one item of a one-tile step, each at least
+// eight blocks long, and enough that none is longer than RANGE_BLOCKS.
+void ranges_of(int N, int K, int& ranges, int& range_blocks) {
+  const int blocks = (K + KB - 1) / KB, tiles = (N + ROWS - 1) / ROWS, sms = gllm_sm_count();
+  int want = tiles < sms ? sms / tiles : 1;
+  if (want > blocks / 8) want = blocks / 8;
+  const int least = (blocks + RANGE_BLOCKS - 1) / RANGE_BLOCKS;
+  if (want < least) want = least;
+  if (want > MOST_RANGES) want = MOST_RANGES;
+  if (want < 1) want = 1;
+  range_blocks = (blocks + want - 1) / want;
+  ranges = (blocks + range_blocks - 1) / range_blocks;     // (none is empty)
+}
+
+// Tokens per tile and whether an item is one range: the layout whose fullest SM ends first.
+struct Plan { int bt, split; };
+Plan plan_of(int M, int N, int K) {
+  int ranges, range_blocks;
+  ranges_of(N, K, ranges, range_blocks);
+  const int64_t blocks = (K + KB - 1) / KB, tiles_n = (N + ROWS - 1) / ROWS, sms = gllm_sm_count();
+  // a block's time, in ns: up to 64 tokens the cutting of the weight's 128 rows, beyond the tokens' as well
+  static const int widths[] = {16, 32, 64, 96};
+  static const float block_ns[] = {500.f, 505.f, 520.f, 640.f};
+  Plan best{96, 0};
   float best_time = 0.f;
-  for (int i = 0; i < 6; ++i) {
-    const Tile& t = tiles[i];
-    int64_t per_sm = ((int64_t)((M + t.m - 1) / t.m) * ((N + t.n - 1) / t.n) + gllm_sm_count() - 1) / gllm_sm_count();
-    if (t.pairs) per_sm = (per_sm + 1) & ~(int64_t)1;
-    const float work = t.work * (float)per_sm, time = work > t.chain ? work : t.chain;
-    if (i == 0 || time < best_time) best = i, best_time = time;
+  for (int i = 0; i < 4; ++i) {
+    const int64_t tiles = tiles_n * ((M + widths[i] - 1) / widths[i]);
+    for (int split = 0; split < 2; ++split) {
+      if (split && (ranges == 1 || (int64_t)ranges * M * N > (int64_t)1 << 26)) continue;
+      const int64_t items = split ? tiles * ranges : tiles, waves = (items + sms - 1) / sms;
+      float time = (float)waves * (float)(split ? range_blocks : blocks) * block_ns[i];
+      if (split) time += 3000.f + (float)ranges * (float)M * (float)N * 8.f / 5000.f;     // written, read and summed
+      if (best_time == 0.f || time < best_time) best = Plan{widths[i], split}, best_time = time;
+    }
   }
   return best;
 }
 
-GLLM_API int gllm_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, int64_t lda,
-                           int64_t ldb, int64_t ldc, cudaStream_t stream) {
+template <int BT>
+int launch(const float* X, const float* W, float* out, float* partial, int M, int N, int K, int64_t ldx, int64_t ldw,
+           int64_t ldo, int split, int* status, cudaStream_t stream) {
+  CUtensorMap map_w, map_x;
+  if (!make_map(&map_w, W, N, K, ldw, ROWS) || !make_map(&map_x, X, M, K, ldx, BT)) return (int)cudaErrorInvalidValue;
+  Cut cut;
+  ranges_of(N, K, cut.ranges, cut.range_blocks);
+  cut.blocks = (K + KB - 1) / KB;
+  cut.tiles_n = (N + ROWS - 1) / ROWS, cut.tiles_m = (M + BT - 1) / BT;
+  cut.split = split;
+  const int64_t items = (int64_t)cut.tiles_n * cut.tiles_m * (split ? cut.ranges : 1);
+  if (items > 0x7fffffff - 4096) return (int)cudaErrorInvalidValue;
+  auto kernel = gemm_f32_parts_kernel<BT>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<BT>::SMEM);
+  if (e != cudaSuccess) return (int)e;
+  const int grid = items < gllm_sm_count() ? (int)items : gllm_sm_count();
+  return gllm_launch(kernel, dim3(grid), dim3(THREADS), (size_t)Shape<BT>::SMEM, stream, map_w, map_x, X, W,
+                     split ? partial : out, M, N, K, ldx, ldw, split ? (int64_t)N : ldo, cut, (int)items, status);
+}
+}  // namespace parts3
+
+bool on_vectors(const float* X, const float* W, int K, int64_t ldx, int64_t ldw) {
+  return K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0 &&
+         (reinterpret_cast<uintptr_t>(W) & 15) == 0;
+}
+}  // namespace
+
+// How many unsummed parts [parts][M][N] the product of these operands leaves in `partial` (0: none, it writes C itself).
+GLLM_API int gllm_gemm_f32_parts(const float* X, const float* W, int M, int N, int K, int64_t ldx, int64_t ldw) {
+  if (M <= 0 || N <= 0 || K <= 0 || !on_vectors(X, W, K, ldx, ldw)) return 0;
+  if (!parts3::plan_of(M, N, K).split) return 0;
+  int ranges, range_blocks;
+  parts3::ranges_of(N, K, ranges, range_blocks);
+  return ranges;
+}
+
+// partial: what gllm_gemm_f32_parts says, to be summed in ascending order by the caller's next kernel; C is then not written.
+GLLM_API int gllm_gemm_f32(const float* X, const float* W, float* C, float* partial, int M, int N, int K, int64_t ldx,
+                           int64_t ldw, int64_t ldc, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return (int)cudaErrorInvalidValue;
-  const bool vectors = K % 4 == 0 && lda % 4 == 0 && ldb % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 &&
-                       (reinterpret_cast<uintptr_t>(B) & 15) == 0;
-  if (vectors) {
+  if (on_vectors(X, W, K, ldx, ldw)) {
     if (M > 128 * 65535) return (int)cudaErrorInvalidValue;
-    switch (pairs_tile_of(M, N)) {
-      case 0: return gemm_f32_pairs<16, 16, 2, 2, 6, 8>(A, B, C, M, N, K, lda, ldb, ldc, stream);
-      case 1: return gemm_f32_pairs<32, 16, 4, 2, 6, 8>(A, B, C, M, N, K, lda, ldb, ldc, stream);
-      case 2: return gemm_f32_pairs<32, 32, 4, 4, 4, 8>(A, B, C, M, N, K, lda, ldb, ldc, stream);
-      case 3: return gemm_f32_pairs<64, 32, 8, 4, 4, 8>(A, B, C, M, N, K, lda, ldb, ldc, stream);
-      case 4: return gemm_f32_pairs<64, 64, 8, 4, 3, 8>(A, B, C, M, N, K, lda, ldb, ldc, stream);
-      default: return gemm_f32_pairs<64, 64, 8, 8, 3, 1>(A, B, C, M, N, K, lda, ldb, ldc, stream);
+    const parts3::Plan plan = parts3::plan_of(M, N, K);
+    if (plan.split && partial == nullptr) return (int)cudaErrorInvalidValue;
+    switch (plan.bt) {
+      case 16: return parts3::launch<16>(X, W, C, partial, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
+      case 32: return parts3::launch<32>(X, W, C, partial, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
+      case 64: return parts3::launch<64>(X, W, C, partial, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
+      default: return parts3::launch<96>(X, W, C, partial, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
     }
   }
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   if (grid.y > 65535) return (int)cudaErrorInvalidValue;
-  return gllm_launch(gemm_f32_kernel, grid, dim3(256), 0, stream, A, B, C, M, N, K, lda, ldb, ldc);
+  return gllm_launch(gemm_f32_kernel, grid, dim3(256), 0, stream, X, W, C, M, N, K, ldx, ldw, ldc);
 }

@@ -77,7 +77,8 @@ _SIGNATURES = {
                                 c_int, P, P],
     },
     "gemm_fp32": {
-        "gllm_gemm_f32": [P, P, P, c_int, c_int, c_int, c_int64, c_int64, c_int64, P],
+        "gllm_gemm_f32": [P, P, P, P, c_int, c_int, c_int, c_int64, c_int64, c_int64, P, P],
+        "gllm_gemm_f32_parts": [P, P, c_int, c_int, c_int, c_int64, c_int64],
     },
     "sampling": {
         "gllm_sample": [P, c_int64, c_int, c_int, P, P, P, P, P, P, c_int, P, P, P, P, P, P, P],
@@ -931,8 +932,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
            out: torch.Tensor | None = None, split_ok: bool = False, add_into: torch.Tensor | None = None,
            bias: torch.Tensor | None = None):
     """``x @ weight.T`` with ``weight`` stored ``[out, in]``
-    (gllm/model/layers/linear.py:20).  fp32 inputs run the FFMA kernel (no
-    tensor-core mode); bf16 inputs run the tensor-core kernels with fp32
+    (gllm/model/layers/linear.py:20).  fp32 inputs run a true 32-bit product
+    (``csrc/gemm_fp32.cu``); bf16 inputs run the tensor-core kernels with fp32
     accumulation.  With ``split_ok`` the result may be a SplitSum (for callers
     that hand it to ``add_rmsnorm`` or ``rope_store``).  With ``add_into``
     (fp32 ``[m, n]``, the residual stream) the product may add itself there
@@ -965,9 +966,12 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
     if x.dtype == torch.float32:
         if out_dtype != torch.float32:
             raise TypeError("the fp32 product writes fp32")
+        count = _fn("gemm_fp32", "gllm_gemm_f32_parts")(x.data_ptr(), weight.data_ptr(), m, n, k, x.stride(0), k)
+        parts = x.new_empty((count, m, n)) if count else None
         f = _fn("gemm_fp32", "gllm_gemm_f32")
-        _check(f(x.data_ptr(), weight.data_ptr(), out.data_ptr(), m, n, k, x.stride(0), k, n, _stream()), "gemm_f32")
-        return out
+        _check(f(x.data_ptr(), weight.data_ptr(), out.data_ptr(), _ptr(parts), m, n, k, x.stride(0), k, n,
+                 status_word(x.device).data_ptr(), _stream()), "gemm_f32")
+        return SplitSum(parts, torch.float32).tensor(out) if count else out
     return gemm_bf16.linear_bf16(x, weight, out)
 
 

@@ -1,0 +1,67 @@
+"""The 32-bit product on the tensor cores (three bfloat16 parts a number): widths of its token tiles, ends of blocks, chunks and
+ranges of K, magnitudes, and operands that are not finite."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _bound(a, b):
+    """Per element: the leading accumulator truncates at most 16 times a chunk of 256, a chunk's and a range's sum round once
+    each, what the cut leaves out is under 2^-24 of a product, and the smaller products' accumulator is 2^-7 of the leading one
+    with up to 640 truncations (2,048 of K, five products of 16 a time)."""
+    k = a.shape[1]
+    steps = 2.0 * (16 + 640 / 128) + (k / 256 + k / 2048 + 4)
+    return steps * 2.0 ** -24 * (a.double().abs() @ b.double().abs().T) + 1e-37
+
+
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 64, 65, 97, 200])
+@pytest.mark.parametrize("n,k", [(1, 32), (127, 36), (129, 256), (300, 260), (2048, 2080), (257, 4100)])
+def test_sizes(m, n, k):
+    from gllm_b200 import ops
+
+    g = torch.Generator().manual_seed(m * n + k)
+    a, b = torch.randn(m, k, generator=g).cuda(), torch.randn(n, k, generator=g).cuda()
+    got = ops.linear(a, b)
+    want = a.double() @ b.double().T
+    assert bool(((got.double() - want).abs() <= _bound(a, b)).all())
+    assert torch.equal(ops.linear(a[m // 2:m // 2 + 1].contiguous(), b)[0], got[m // 2])
+    assert int(ops.status_word(a.device)[0]) == 0
+
+
+@pytest.mark.parametrize("scale_a,scale_b", [(1e30, 1e-30), (1e-18, 1e-12), (1e18, 1e18), (3e-30, 1.0)])
+def test_magnitudes(scale_a, scale_b):
+    from gllm_b200 import ops
+
+    g = torch.Generator().manual_seed(3)
+    a = (torch.randn(70, 520, generator=g) * scale_a).cuda()
+    b = (torch.randn(130, 520, generator=g) * scale_b).cuda()
+    a[:, ::7] *= 1e-6                                    # very different numbers in one row
+    got = ops.linear(a, b)
+    want = a.double() @ b.double().T
+    assert bool(((got.double() - want).abs() <= _bound(a, b)).all())
+
+
+@pytest.mark.parametrize("m", [3, 90, 200])
+def test_not_finite(m):
+    """As the sum of 32-bit products has it: an infinity stays one, and what does not meet it stays as it is."""
+    from gllm_b200 import ops
+
+    g = torch.Generator().manual_seed(m)
+    a, b = torch.randn(m, 2100, generator=g).cuda(), torch.randn(260, 2100, generator=g).cuda()
+    clean = ops.linear(a, b)
+    a[1, 2099], a[2, 5] = float("inf"), float("nan")
+    a[0, 7] = 3.4e38                                     # finite, and an infinity once rounded to bfloat16
+    b[200, 40] = float("-inf")
+    b[:, 7] = 0.25
+    got, want = ops.linear(a, b), a.double() @ b.double().T
+    finite = want.isfinite() & (want.abs() < 3.4e38)
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got[~finite & ~want.isnan()].double(), want[~finite & ~want.isnan()])
+    assert bool(((got.double() - want).abs()[finite] <= (1.1 * 2100 * 2.0 ** -24 * (a.double().abs() @ b.double().abs().T))[finite]).all())
+    rows = torch.arange(m, device="cuda") > 2
+    cols = torch.arange(260, device="cuda") != 200
+    b2 = b.clone()
+    assert torch.equal(ops.linear(a[rows], b2)[:, cols], got[rows][:, cols])
+    assert clean.isfinite().all()
