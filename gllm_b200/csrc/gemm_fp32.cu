@@ -2,9 +2,10 @@
 // gllm/model/layers/linear.py:20 with W stored [out, in].  This is the path
 // that shows faults bf16 hides: no operand is rounded.
 //
-// Two kernels.  Rows on 16-byte boundaries and K a multiple of 4 run on the
-// tensor cores with every 32-bit number cut into three bfloat16 whose sum it
-// is (8 bits of its significand each, rounded to nearest, so nothing is lost):
+// Two kernels.  Rows on 16-byte boundaries and K a multiple of 4, 32 or more,
+// run on the tensor cores with every 32-bit number cut into three bfloat16
+// whose sum it is (8 bits of its significand each, rounded to nearest, so
+// nothing is lost):
 //   x = x0 + x1 + x2,  w = w0 + w1 + w2,
 //   x w = w0 x0 + (w0 x1 + w1 x0 + w0 x2 + w1 x1 + w2 x0) + terms below 2^-26 |x w|.
 // Everything else runs a plain 64 x 64 tile of 32-bit multiply-adds.
@@ -15,10 +16,10 @@
 // products are 2^-8 of it and stay in theirs for a whole range of K.
 //
 // K is cut into ranges that depend on (N, K) alone.  A work item is a tile of
-// 128 weight rows x BT tokens times one range (few tokens: the unsummed parts
-// go to scratch) or all ranges one after the other; the ranges' sums are added
-// in ascending order either way, so a token's result does not depend on the
-// batch it is in.
+// 128 weight rows x BT tokens times one range (few tokens: the blocks of a
+// tile's ranges are a cluster and add up through shared memory) or all ranges
+// one after the other; the ranges' sums are added in ascending order either
+// way, so a token's result does not depend on the batch it is in.
 //
 // A result that is not finite is computed again with 32-bit multiply-adds from
 // the operands themselves: the parts of an infinity are not its sum.
@@ -38,11 +39,11 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
   const int tid = threadIdx.x;
   const int tx = tid % 16, ty = tid / 16;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[TM][TN];
+  float acc[2][TM][TN];            // of the products with even and with odd k
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN; ++j) acc[0][i][j] = acc[1][i][j] = 0.f;
 
   // each thread loads 4 elements of A and 4 of B per k-tile
   const int lrow = tid / 4;        // 0..63
@@ -66,7 +67,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        for (int j = 0; j < TN; ++j) acc[kk & 1][i][j] = fmaf(a[i], b[j], acc[kk & 1][i][j]);
     }
     __syncthreads();
   }
@@ -77,7 +78,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       const int n = n0 + tx * TN + j;
-      if (n < N) C[(int64_t)m * ldc + n] = acc[i][j];
+      if (n < N) C[(int64_t)m * ldc + n] = acc[0][i][j] + acc[1][i][j];
     }
   }
 }
@@ -89,17 +90,20 @@ constexpr int KB = 32;              // k per block: 32 floats = one 128-byte swi
 constexpr int CHUNK = 8;            // blocks between two visits to the leading accumulator
 constexpr int WORKERS = 16;         // warps that cut operands into parts and keep the sums
 constexpr int GROUPS = 4;           // of workers, that take turns with the blocks
-constexpr int CUT = 4;              // blocks of parts in flight (no fewer than GROUPS: a group waits for one phase of a stage)
 constexpr int THREADS = (WORKERS + 2) * 32;
 constexpr int RANGE_BLOCKS = 64;    // longest range of K (2,048), as long as there are at most 16 of them
-constexpr int MOST_RANGES = 16;
+constexpr int MOST_RANGES = 16;     // (eight where they are a cluster's blocks)
+constexpr int MOST_BLOCKS = 8;
 constexpr int A_COLS = 3 * KB / 2;  // tensor-memory columns of one block of the weight's parts
 
 template <int BT>
 struct Shape {
   static constexpr int RAW = (ROWS + BT) * KB * 4;
+  // blocks of parts in flight: no fewer than GROUPS (a group waits for one phase of a stage), more where tensor memory has room,
+  // so that the groups do not fall into step with the products
+  static constexpr int CUT = BT <= 32 ? 8 : 4;
   static constexpr int PARTS = ((3 * BT * KB * 2 + 1023) / 1024) * 1024;
-  static constexpr int STAGES_ = (216 * 1024 - CUT * PARTS) / RAW;
+  static constexpr int STAGES_ = (224 * 1024 - CUT * PARTS) / RAW;
   static constexpr int STAGES = STAGES_ > 8 ? 8 : STAGES_;                 // raw blocks in flight
   static constexpr int CROSS = BT <= 64 ? 2 : 1;                           // accumulators of the five smaller products
   static constexpr int COLS = (2 + CROSS) * BT + CUT * A_COLS;
@@ -169,7 +173,7 @@ __device__ __forceinline__ void cut8(const float4& a, const float4& b, uint32_t 
 struct Cut {                        // how the work is laid out
   int tiles_n, tiles_m;             // tiles of weight rows, of tokens
   int ranges, range_blocks, blocks; // of K
-  int split;                        // 1: an item is one range of a tile; 0: all of them
+  int split;                        // 1: an item is one range of a tile, a block each, a cluster a tile; 0: all of them
 };
 
 // Item w: neighbouring CTAs share a tile of weight rows (or take the ranges of one).
@@ -186,22 +190,22 @@ __device__ __forceinline__ void place(const Cut& cut, int w, int& n0, int& m0, i
   kb_end = cut.split ? min(cut.blocks, kb_begin + cut.range_blocks) : cut.blocks;
 }
 
-// Results of an item that are not finite, once more with 32-bit multiply-adds: token m's, weight row n's at dst[0], of the
-// next tokens behind it.
-__device__ __noinline__ void again(float* dst, int64_t ldo, int tokens, const float* __restrict__ x, int64_t ldx,
-                                   const float* __restrict__ w, int k0, int k1) {
-  for (int i = 0; i < tokens; ++i, dst += ldo, x += ldx) {
-    if ((__float_as_uint(__ldcg(dst)) & 0x7f800000u) != 0x7f800000u) continue;
-    float s = 0.f;
-    for (int k = k0; k < k1; k += 4) {
-      const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
-      s = fmaf(a.x, b.x, s), s = fmaf(a.y, b.y, s), s = fmaf(a.z, b.z, s), s = fmaf(a.w, b.w, s);
-    }
-    *dst = s;
+// A result once more, with 32-bit multiply-adds.
+__device__ __noinline__ float again(const float* __restrict__ x, const float* __restrict__ w, int K) {
+  float s = 0.f;
+  for (int k = 0; k < K; k += 4) {
+    const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
+    s = fmaf(a.x, b.x, s), s = fmaf(a.y, b.y, s), s = fmaf(a.z, b.z, s), s = fmaf(a.w, b.w, s);
   }
+  return s;
 }
+__device__ __forceinline__ bool is_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
 // The sum of a range of an item, columns c0 .. of one of its rows: behind the item's first range it joins what this thread
-// has written of the ranges before.
+// has written of the ranges before.  `broken`: some sum of the item was not finite.
 template <int BT, int COLS>
 __device__ __forceinline__ void put_range(const Cut& cut, int item, int end, int row, int c0, const float (&acc)[COLS],
                                           const float* __restrict__ X, const float* __restrict__ W, float* out, int M, int N,
@@ -210,20 +214,21 @@ __device__ __forceinline__ void put_range(const Cut& cut, int item, int end, int
   place<BT>(cut, item, n0, m0, kb_begin, kb_end, range);
   const int n = n0 + row, m = m0 + c0, tokens = min(COLS, M - m);
   if (n >= N || tokens <= 0) return;
-  float* const dst = out + (int64_t)range * M * N + (int64_t)m * ldo + n;
-  const bool joins = end - kb_begin > cut.range_blocks;
+  float* const dst = out + (int64_t)m * ldo + n;
+  const bool joins = end > cut.range_blocks;
 #pragma unroll
   for (int i = 0; i < COLS; ++i) {
     if (i < tokens) {
       const float v = acc[i];
-      broken = broken || (__float_as_uint(v) & 0x7f800000u) == 0x7f800000u;
+      broken = broken || !is_finite(v);
       if (joins) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + i * ldo), "f"(v) : "memory");   // (nothing to wait for)
       else dst[i * ldo] = v;
     }
   }
   if (end != kb_end) return;
   if (broken)
-    again(dst, ldo, tokens, X + (int64_t)m * ldx, ldx, W + (int64_t)n * ldw, kb_begin * KB, min(K, kb_end * KB));
+    for (int i = 0; i < tokens; ++i)
+      if (!is_finite(__ldcg(dst + i * ldo))) dst[i * ldo] = again(X + (int64_t)(m + i) * ldx, W + (int64_t)n * ldw, K);
   broken = false;
 }
 
@@ -240,7 +245,7 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
   using S = Shape<BT>;
   constexpr int COLS = BT / 4;      // columns of a worker
   extern __shared__ unsigned char smem_dyn[];
-  __shared__ __align__(8) uint64_t raw_full[S::STAGES], raw_empty[S::STAGES], cut_full[CUT], cut_empty[CUT], main_full[2],
+  __shared__ __align__(8) uint64_t raw_full[S::STAGES], raw_empty[S::STAGES], cut_full[S::CUT], cut_empty[S::CUT], main_full[2],
       main_empty[2], cross_empty[S::CROSS];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
@@ -253,7 +258,7 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::STAGES; ++s) mbar_init(smem_addr(&raw_full[s]), 1), mbar_init(smem_addr(&raw_empty[s]), WORKERS / GROUPS);
-    for (int s = 0; s < CUT; ++s) mbar_init(smem_addr(&cut_full[s]), WORKERS / GROUPS), mbar_init(smem_addr(&cut_empty[s]), 1);
+    for (int s = 0; s < S::CUT; ++s) mbar_init(smem_addr(&cut_full[s]), WORKERS / GROUPS), mbar_init(smem_addr(&cut_empty[s]), 1);
     for (int b = 0; b < 2; ++b) mbar_init(smem_addr(&main_full[b]), 1), mbar_init(smem_addr(&main_empty[b]), WORKERS);
     for (int b = 0; b < S::CROSS; ++b) mbar_init(smem_addr(&cross_empty[b]), WORKERS);
     abort_flag = 0;
@@ -314,6 +319,8 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         }
       }
     }
+    __syncwarp();
+    if (cut.split) cluster_barrier(), cluster_barrier();
   } else if (warp == WORKERS + 1) {
     // ------------------------------------------------------------ products (the whole warp converged, one elected thread)
     const bool leader = elect_one();
@@ -339,8 +346,8 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             ok = wait_u(&main_empty[mb], ((chunks >> 1) & 1u) ^ 1u);
             if (!ok) break;
           }
-          const uint32_t s = it % CUT;
-          ok = wait_u(&cut_full[s], (it / CUT) & 1u);
+          const uint32_t s = it % S::CUT;
+          ok = wait_u(&cut_full[s], (it / S::CUT) & 1u);
           if (!ok) break;
           const uint32_t a0 = tmem_parts + s * A_COLS;
           const uint64_t b0 = desc64(parts_base + s * S::PARTS);
@@ -366,6 +373,7 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         }
       }
     }
+    if (cut.split) cluster_barrier(), cluster_barrier();
   } else {
     // ------------------------------------------------------------ parts and sums
     pdl_wait();                                            // nothing is written before the previous kernel is done
@@ -394,98 +402,117 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     };
     // the chunk that waits to be added: of which item; where its range ends, if with it
     bool pending = false, broken = false;                  // (broken: a sum of this item was not finite)
-    int p_item = 0, p_end = 0, behind = 0;                 // (behind: blocks between its end and the block in hand)
-    int item = (int)blockIdx.x - (int)gridDim.x, n0, m0, kb = 0, r0 = 0, r1 = 0, kb_begin, kb_end = 0, range;
-    while (true) {
-      bool more = true;
-      if (kb == kb_end) {
-        item += gridDim.x;
-        more = item < num_items;
-        if (more) {
-          place<BT>(cut, item, n0, m0, kb_begin, kb_end, range);
-          kb = r0 = kb_begin, r1 = min(kb_end, r0 + cut.range_blocks);
-        }
-      } else if (kb == r1) {
-        r0 = r1, r1 = min(kb_end, r0 + cut.range_blocks);
-      }
-      const bool mine = more && it % GROUPS == group;
-      if (mine) {
-        const uint32_t rs = it % S::STAGES, cs = it % CUT;
-        if (!wait_u(&raw_full[rs], (it / S::STAGES) & 1u)) break;
-        const unsigned char* raw = raw_ptr + rs * S::RAW;
-        float4 a[A_K / 4];
+    int p_item = 0, p_end = 0;
+    for (int item = blockIdx.x; ok; item += gridDim.x) {
+      int n0, m0, kb_begin = 0, kb_end = 1, range;
+      const bool more = item < num_items;                  // (behind the last item the pending chunk is left)
+      if (more) place<BT>(cut, item, n0, m0, kb_begin, kb_end, range);
+      for (int r0 = kb_begin; r0 < kb_end && ok; r0 += cut.range_blocks) {
+        const int r1 = min(kb_end, r0 + cut.range_blocks);
+        for (int c0 = r0; c0 < r1 && ok; c0 += CHUNK) {
+          const int blocks = more ? min(CHUNK, r1 - c0) : 0;
+          // this group's blocks of the chunk
+          for (int j = (group - it) % GROUPS; ok; j += GROUPS) {
+            if (j < blocks) {
+              const uint32_t at = it + j, rs = at % S::STAGES, cs = at % S::CUT;
+              if (!wait_u(&cut_empty[cs], ((at / S::CUT) & 1u) ^ 1u) || !wait_u(&raw_full[rs], (at / S::STAGES) & 1u)) break;
+              const unsigned char* raw = raw_ptr + rs * S::RAW;
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              const uint32_t ta = tmem_parts + cs * A_COLS + lanes + a_side * (A_K / 2);
 #pragma unroll
-        for (int j = 0; j < A_K / 4; ++j)
-          a[j] = *reinterpret_cast<const float4*>(raw + row * 128 + (((a_side * (A_K / 4) + j) ^ (row & 7)) << 4));
-        if (!wait_u(&cut_empty[cs], ((it / CUT) & 1u) ^ 1u)) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t ta = tmem_parts + cs * A_COLS + lanes + a_side * (A_K / 2);
+              for (int i = 0; i < A_K / 8; ++i) {
+                const int e = a_side * (A_K / 4) + 2 * i;
+                const float4 lo = *reinterpret_cast<const float4*>(raw + row * 128 + ((e ^ (row & 7)) << 4));
+                const float4 hi = *reinterpret_cast<const float4*>(raw + row * 128 + (((e + 1) ^ (row & 7)) << 4));
+                uint32_t parts[3][4];
+                cut8(lo, hi, parts);
 #pragma unroll
-        for (int j = 0; j < A_K / 8; ++j) {
-          uint32_t parts[3][4];
-          cut8(a[2 * j], a[2 * j + 1], parts);
+                for (int p = 0; p < 3; ++p) tmem_st4(ta + p * (KB / 2) + i * 4, parts[p]);
+              }
+              if (has_b) {
+                const unsigned char* b_raw = raw + ROWS * 128 + b_row * 128;
+                unsigned char* b_parts = parts_ptr + cs * S::PARTS + b_row * 64;
 #pragma unroll
-          for (int p = 0; p < 3; ++p) tmem_st4(ta + p * (KB / 2) + j * 4, parts[p]);
-        }
-        if (has_b) {
-          const unsigned char* b_raw = raw + ROWS * 128 + b_row * 128;
-          unsigned char* b_parts = parts_ptr + cs * S::PARTS + b_row * 64;
+                for (int i = 0; i < B_PIECES; ++i) {
+                  const int e = b_piece + i;
+                  const float4 lo = *reinterpret_cast<const float4*>(b_raw + (((2 * e) ^ (b_row & 7)) << 4));
+                  const float4 hi = *reinterpret_cast<const float4*>(b_raw + (((2 * e + 1) ^ (b_row & 7)) << 4));
+                  uint32_t parts[3][4];
+                  cut8(lo, hi, parts);
 #pragma unroll
-          for (int j = 0; j < B_PIECES; ++j) {
-            const int e = b_piece + j;
-            const float4 lo = *reinterpret_cast<const float4*>(b_raw + (((2 * e) ^ (b_row & 7)) << 4));
-            const float4 hi = *reinterpret_cast<const float4*>(b_raw + (((2 * e + 1) ^ (b_row & 7)) << 4));
-            uint32_t parts[3][4];
-            cut8(lo, hi, parts);
+                  for (int p = 0; p < 3; ++p)
+                    *reinterpret_cast<uint4*>(b_parts + p * (BT * KB * 2) + ((e ^ ((b_row >> 1) & 3)) << 4)) =
+                        make_uint4(parts[p][0], parts[p][1], parts[p][2], parts[p][3]);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+              }
+              tmem_wait_st();
+              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+              __syncwarp();
+              if (lane == 0) {
+                mbar_arrive(smem_addr(&raw_empty[rs]));
+                mbar_arrive(smem_addr(&cut_full[cs]));
+              }
+            }
+            // The chunk before is added while the products of this block run: ahead of the next of the group's, as that stage
+            // comes free only behind products that may wait for these sums to be taken.
+            if (pending) {
+              const uint32_t mb = chunks & 1u, cb = segments % S::CROSS;
+              if (!wait_u(&main_full[mb], (chunks >> 1) & 1u)) break;
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              add_columns<COLS>(tmem_main + mb * BT + lanes + side * COLS, acc);
+              if (p_end) add_columns<COLS>(tmem_cross + cb * BT + lanes + side * COLS, acc);
+              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+              __syncwarp();
+              if (lane == 0) {
+                mbar_arrive(smem_addr(&main_empty[mb]));
+                if (p_end) mbar_arrive(smem_addr(&cross_empty[cb]));
+              }
+              ++chunks;
+              pending = false;
+              if (p_end) {
+                ++segments;
+                if (cut.split) break;                      // (the block's only item and range; `more` is false)
+                put_range<BT, COLS>(cut, p_item, p_end, row, side * COLS, acc, X, W, out, M, N, K, ldx, ldw, ldo, broken);
 #pragma unroll
-            for (int p = 0; p < 3; ++p)
-              *reinterpret_cast<uint4*>(b_parts + p * (BT * KB * 2) + ((e ^ ((b_row >> 1) & 3)) << 4)) =
-                  make_uint4(parts[p][0], parts[p][1], parts[p][2], parts[p][3]);
+                for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
+              }
+            }
+            if (j + GROUPS >= blocks) break;
           }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        }
-        tmem_wait_st();
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(smem_addr(&raw_empty[rs]));
-          mbar_arrive(smem_addr(&cut_full[cs]));
-        }
-      }
-      // The chunk before is added while the products of this block run: by the CUT-th block behind it, as the stage after
-      // that comes free only behind products that may wait for these sums to be taken.
-      const bool chunk_last = more && ((kb - r0) % CHUNK == CHUNK - 1 || kb + 1 == r1);
-      if (pending && (mine || behind >= CUT - 1 || chunk_last || !more)) {
-        const uint32_t mb = chunks & 1u, cb = segments % S::CROSS;
-        if (!wait_u(&main_full[mb], (chunks >> 1) & 1u)) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        add_columns<COLS>(tmem_main + mb * BT + lanes + side * COLS, acc);
-        if (p_end) add_columns<COLS>(tmem_cross + cb * BT + lanes + side * COLS, acc);
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(smem_addr(&main_empty[mb]));
-          if (p_end) mbar_arrive(smem_addr(&cross_empty[cb]));
-        }
-        ++chunks;
-        pending = false;
-        if (p_end) {
-          ++segments;
-          put_range<BT, COLS>(cut, p_item, p_end, row, side * COLS, acc, X, W, out, M, N, K, ldx, ldw, ldo, broken);
-#pragma unroll
-          for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
+          it += blocks;
+          pending = true;
+          p_item = item;
+          p_end = c0 + CHUNK >= r1 ? r1 : 0;
         }
       }
       if (!more) break;
-      if (chunk_last) {
-        pending = true;
-        behind = 0;
-        p_item = item;
-        p_end = kb + 1 == r1 ? r1 : 0;
-      } else {
-        ++behind;
+    }
+    if (cut.split) {
+      // Every block's sums to the blocks of the cluster, 1/ranges of the tile's rows to each, where they lie [range][column]
+      // [row]: over the raw stages, which every block is done with behind the first barrier.
+      const int each = (ROWS + cut.ranges - 1) / cut.ranges, owner = row / each;
+      const uint32_t mine = (uint32_t)(blockIdx.x % (unsigned)cut.ranges);
+      cluster_barrier();
+      uint32_t dst;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                   : "=r"(dst)
+                   : "r"(raw_base + ((mine * BT + side * COLS) * each + row - owner * each) * 4u), "r"(owner));
+#pragma unroll
+      for (int i = 0; i < COLS; ++i)
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + (uint32_t)(i * each) * 4u), "f"(acc[i]) : "memory");
+      cluster_barrier();
+      int n0, m0, kb_begin, kb_end, range;
+      place<BT>(cut, blockIdx.x, n0, m0, kb_begin, kb_end, range);
+      const float* parts = reinterpret_cast<const float*>(raw_ptr);
+      for (int i = threadIdx.x; i < BT * each; i += WORKERS * 32) {
+        const int c = i / each, r = (int)mine * each + i - c * each, m = m0 + c, n = n0 + r;
+        if (r >= ROWS || m >= M || n >= N) continue;
+        float v = 0.f;
+        for (int j = 0; j < cut.ranges; ++j) v += parts[j * BT * each + i];
+        if (!is_finite(v)) v = again(X + (int64_t)m * ldx, W + (int64_t)n * ldw, K);
+        out[(int64_t)m * ldo + n] = v;
       }
-      ++kb, ++it;
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
@@ -521,11 +548,36 @@ bool make_map(CUtensorMap* map, const float* base, int rows, int cols, int64_t l
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Ranges of K: a function of (N, K) alone.  As many as give every SM at most one item of a one-tile step, each at least
-// eight blocks long, and enough that none is longer than RANGE_BLOCKS.
+// How many clusters of `blocks` blocks run at once, one block an SM (clusters do not reach across the SMs' groups: 148 SMs hold
+// 22 clusters of six but 15 of seven or eight).
+int clusters_of(int blocks) {
+  static const struct Table {
+    int count[MOST_BLOCKS + 1] = {};
+    Table() {
+      if (cudaFuncSetAttribute(gemm_f32_parts_kernel<96>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<96>::SMEM) != cudaSuccess)
+        return;
+      for (int c = 2; c <= MOST_BLOCKS; ++c) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(c), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = Shape<96>::SMEM;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = c, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr, cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, gemm_f32_parts_kernel<96>, &cfg) == cudaSuccess) count[c] = n;
+      }
+    }
+  } table;
+  return table.count[blocks];
+}
+
+// Ranges of K: a function of (N, K) alone.  As many blocks to a cluster as leave all tiles of one step of few tokens running at
+// once, each range at least eight blocks of K long, and enough that none is longer than RANGE_BLOCKS.
 void ranges_of(int N, int K, int& ranges, int& range_blocks) {
-  const int blocks = (K + KB - 1) / KB, tiles = (N + ROWS - 1) / ROWS, sms = gllm_sm_count();
-  int want = tiles < sms ? sms / tiles : 1;
+  const int blocks = (K + KB - 1) / KB, tiles = (N + ROWS - 1) / ROWS;
+  int want = 1;
+  for (int c = 2; c <= MOST_BLOCKS; ++c)
+    if (clusters_of(c) >= tiles) want = c;
   if (want > blocks / 8) want = blocks / 8;
   const int least = (blocks + RANGE_BLOCKS - 1) / RANGE_BLOCKS;
   if (want < least) want = least;
@@ -543,16 +595,17 @@ Plan plan_of(int M, int N, int K) {
   const int64_t blocks = (K + KB - 1) / KB, tiles_n = (N + ROWS - 1) / ROWS, sms = gllm_sm_count();
   // a block's time, in ns: up to 64 tokens the cutting of the weight's 128 rows, beyond the tokens' as well
   static const int widths[] = {16, 32, 64, 96};
-  static const float block_ns[] = {500.f, 505.f, 520.f, 640.f};
+  static const float block_ns[] = {445.f, 450.f, 455.f, 560.f};
   Plan best{96, 0};
   float best_time = 0.f;
   for (int i = 0; i < 4; ++i) {
     const int64_t tiles = tiles_n * ((M + widths[i] - 1) / widths[i]);
     for (int split = 0; split < 2; ++split) {
-      if (split && (ranges == 1 || (int64_t)ranges * M * N > (int64_t)1 << 26)) continue;
-      const int64_t items = split ? tiles * ranges : tiles, waves = (items + sms - 1) / sms;
-      float time = (float)waves * (float)(split ? range_blocks : blocks) * block_ns[i];
-      if (split) time += 3000.f + (float)ranges * (float)M * (float)N * 8.f / 5000.f;     // written, read and summed
+      const int64_t at_once = !split ? sms : ranges > 1 && ranges <= MOST_BLOCKS ? clusters_of(ranges) : 0;
+      if (at_once <= 0) continue;
+      const int64_t waves = (tiles + at_once - 1) / at_once;
+      // (a range's start and the sum through shared memory: measured 3 us)
+      const float time = (float)waves * ((float)(split ? range_blocks : blocks) * block_ns[i] + (split ? 3000.f : 0.f));
       if (best_time == 0.f || time < best_time) best = Plan{widths[i], split}, best_time = time;
     }
   }
@@ -560,8 +613,8 @@ Plan plan_of(int M, int N, int K) {
 }
 
 template <int BT>
-int launch(const float* X, const float* W, float* out, float* partial, int M, int N, int K, int64_t ldx, int64_t ldw,
-           int64_t ldo, int split, int* status, cudaStream_t stream) {
+int launch(const float* X, const float* W, float* out, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo, int split,
+           int* status, cudaStream_t stream) {
   CUtensorMap map_w, map_x;
   if (!make_map(&map_w, W, N, K, ldw, ROWS) || !make_map(&map_x, X, M, K, ldx, BT)) return (int)cudaErrorInvalidValue;
   Cut cut;
@@ -572,11 +625,14 @@ int launch(const float* X, const float* W, float* out, float* partial, int M, in
   const int64_t items = (int64_t)cut.tiles_n * cut.tiles_m * (split ? cut.ranges : 1);
   if (items > 0x7fffffff - 4096) return (int)cudaErrorInvalidValue;
   auto kernel = gemm_f32_parts_kernel<BT>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<BT>::SMEM);
+  static const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<BT>::SMEM);
   if (e != cudaSuccess) return (int)e;
+  if (split)
+    return gllm_launch_cluster(kernel, dim3((unsigned)items), dim3(THREADS), (size_t)Shape<BT>::SMEM, stream,
+                               (unsigned)cut.ranges, map_w, map_x, X, W, out, M, N, K, ldx, ldw, ldo, cut, (int)items, status);
   const int grid = items < gllm_sm_count() ? (int)items : gllm_sm_count();
-  return gllm_launch(kernel, dim3(grid), dim3(THREADS), (size_t)Shape<BT>::SMEM, stream, map_w, map_x, X, W,
-                     split ? partial : out, M, N, K, ldx, ldw, split ? (int64_t)N : ldo, cut, (int)items, status);
+  return gllm_launch(kernel, dim3(grid), dim3(THREADS), (size_t)Shape<BT>::SMEM, stream, map_w, map_x, X, W, out, M, N, K, ldx,
+                     ldw, ldo, cut, (int)items, status);
 }
 }  // namespace parts3
 
@@ -584,34 +640,31 @@ bool on_vectors(const float* X, const float* W, int K, int64_t ldx, int64_t ldw)
   return K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0 &&
          (reinterpret_cast<uintptr_t>(W) & 15) == 0;
 }
+// Whether the tensor-core kernel takes them: short of one block of K most of its work would be padding.
+bool in_parts(const float* X, const float* W, int K, int64_t ldx, int64_t ldw) {
+  return K >= parts3::KB && on_vectors(X, W, K, ldx, ldw);
+}
 }  // namespace
 
-// How many unsummed parts [parts][M][N] the product of these operands leaves in `partial` (0: none, it writes C itself).
-GLLM_API int gllm_gemm_f32_parts(const float* X, const float* W, int M, int N, int K, int64_t ldx, int64_t ldw) {
-  if (M <= 0 || N <= 0 || K <= 0 || !on_vectors(X, W, K, ldx, ldw)) return 0;
-  if (!parts3::plan_of(M, N, K).split) return 0;
-  int ranges, range_blocks;
-  parts3::ranges_of(N, K, ranges, range_blocks);
-  return ranges;
-}
-
-// partial: what gllm_gemm_f32_parts says, to be summed in ascending order by the caller's next kernel; C is then not written.
-GLLM_API int gllm_gemm_f32(const float* X, const float* W, float* C, float* partial, int M, int N, int K, int64_t ldx,
-                           int64_t ldw, int64_t ldc, int* status, cudaStream_t stream) {
+GLLM_API int gllm_gemm_f32(const float* X, const float* W, float* C, int M, int N, int K, int64_t ldx, int64_t ldw,
+                           int64_t ldc, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return (int)cudaErrorInvalidValue;
-  if (on_vectors(X, W, K, ldx, ldw)) {
-    if (M > 128 * 65535) return (int)cudaErrorInvalidValue;
+  if (M > (on_vectors(X, W, K, ldx, ldw) ? 128 : BM) * 65535) return (int)cudaErrorInvalidValue;
+  if (in_parts(X, W, K, ldx, ldw)) {
     const parts3::Plan plan = parts3::plan_of(M, N, K);
-    if (plan.split && partial == nullptr) return (int)cudaErrorInvalidValue;
     switch (plan.bt) {
-      case 16: return parts3::launch<16>(X, W, C, partial, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
-      case 32: return parts3::launch<32>(X, W, C, partial, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
-      case 64: return parts3::launch<64>(X, W, C, partial, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
-      default: return parts3::launch<96>(X, W, C, partial, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
+      case 16: return parts3::launch<16>(X, W, C, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
+      case 32: return parts3::launch<32>(X, W, C, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
+      case 64: return parts3::launch<64>(X, W, C, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
+      default: return parts3::launch<96>(X, W, C, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
     }
   }
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  if (grid.y > 65535) return (int)cudaErrorInvalidValue;
-  return gllm_launch(gemm_f32_kernel, grid, dim3(256), 0, stream, X, W, C, M, N, K, ldx, ldw, ldc);
+  for (int m0 = 0; m0 < M; m0 += BM * 65535) {               // (tiles of rows lie along y, at most 65,535 a launch)
+    const int rows = M - m0 < BM * 65535 ? M - m0 : BM * 65535;
+    const int rc = gllm_launch(gemm_f32_kernel, dim3((N + BN - 1) / BN, (rows + BM - 1) / BM), dim3(256), 0, stream,
+                               X + (int64_t)m0 * ldx, W, C + (int64_t)m0 * ldc, rows, N, K, ldx, ldw, ldc);
+    if (rc != 0) return rc;
+  }
+  return 0;
 }

@@ -77,8 +77,7 @@ _SIGNATURES = {
                                 c_int, P, P],
     },
     "gemm_fp32": {
-        "gllm_gemm_f32": [P, P, P, P, c_int, c_int, c_int, c_int64, c_int64, c_int64, P, P],
-        "gllm_gemm_f32_parts": [P, P, c_int, c_int, c_int, c_int64, c_int64],
+        "gllm_gemm_f32": [P, P, P, c_int, c_int, c_int, c_int64, c_int64, c_int64, P, P],
     },
     "sampling": {
         "gllm_sample": [P, c_int64, c_int, c_int, P, P, P, P, P, P, c_int, P, P, P, P, P, P, P],
@@ -966,12 +965,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
     if x.dtype == torch.float32:
         if out_dtype != torch.float32:
             raise TypeError("the fp32 product writes fp32")
-        count = _fn("gemm_fp32", "gllm_gemm_f32_parts")(x.data_ptr(), weight.data_ptr(), m, n, k, x.stride(0), k)
-        parts = x.new_empty((count, m, n)) if count else None
         f = _fn("gemm_fp32", "gllm_gemm_f32")
-        _check(f(x.data_ptr(), weight.data_ptr(), out.data_ptr(), _ptr(parts), m, n, k, x.stride(0), k, n,
+        _check(f(x.data_ptr(), weight.data_ptr(), out.data_ptr(), m, n, k, x.stride(0), k, n,
                  status_word(x.device).data_ptr(), _stream()), "gemm_f32")
-        return SplitSum(parts, torch.float32).tensor(out) if count else out
+        return out
     return gemm_bf16.linear_bf16(x, weight, out)
 
 
