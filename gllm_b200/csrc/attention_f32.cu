@@ -17,7 +17,7 @@ __device__ __forceinline__ unsigned long long twice(float x) {
 // ---- portions.  A block takes 64 rows (tokens x the query heads of one kv head) of one request and walks its keys in
 // tiles of 64: S = Q K^T and O += P V, each thread 4 rows x 8 keys and 4 rows x D/8 columns.
 // What bounds it: the latency of the shared-memory loads that feed the multiply-adds (12 sixteen-byte loads per 64 packed
-// ones in S, as many and 16 register pairs in P V) with two warps a scheduler; a half warp is 4 x 4 threads, so a load takes
+// ones in S, as many and 16 register pairs in P V) with three warps a scheduler (head size 64; two took 3 us more); a half warp is 4 x 4 threads, so a load takes
 // no more than two passes over the banks.  The warp-per-token kernel read every key row once per token and head, 32 rows
 // side by side: 2,515 us for 512 and 200 (over 300) tokens beside 8 single ones (about 1,000 keys), 32 heads of 64 over 8;
 // this kernel takes 128 us for the portions (10 of them for the look at broken values below), the split one 19 and its
@@ -33,7 +33,7 @@ template <int D> struct PortionSmem {
 };
 
 template <int D>
-__global__ void __launch_bounds__(PF_THREADS)
+__global__ void __launch_bounds__(PF_THREADS, D == 64 ? 3 : 1)
 attention_f32_portion_kernel(const float* __restrict__ q, int64_t q_stride, float* __restrict__ out, int64_t out_stride,
                              const float* __restrict__ cache, const int* __restrict__ block_table, int bt_stride,
                              const int* __restrict__ cu_q, const int* __restrict__ ctx_lens,

@@ -105,7 +105,7 @@ struct Shape {
   static constexpr int PARTS = ((3 * BT * KB * 2 + 1023) / 1024) * 1024;
   static constexpr int STAGES_ = (224 * 1024 - CUT * PARTS) / RAW;
   static constexpr int STAGES = STAGES_ > 8 ? 8 : STAGES_;                 // raw blocks in flight
-  static constexpr int CROSS = BT <= 64 ? 2 : 1;                           // accumulators of the five smaller products
+  static constexpr int CROSS = BT <= 80 ? 2 : 1;                           // accumulators of the five smaller products
   static constexpr int COLS = (2 + CROSS) * BT + CUT * A_COLS;
   static constexpr int TMEM_COLS = COLS <= 256 ? 256 : 512;
   static constexpr int SMEM = STAGES * RAW + CUT * PARTS + 1024;
@@ -390,7 +390,7 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     const int a_side = side % SIDES;
     const int g_tid = (int)threadIdx.x - (int)group * GROUP_THREADS;
     const int b_row = g_tid / (4 / B_PIECES), b_piece = g_tid % (4 / B_PIECES) * B_PIECES;
-    const bool has_b = b_row < BT;                         // (whole warps)
+    const bool has_b = b_row < BT;
     float acc[COLS];
 #pragma unroll
     for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
@@ -446,6 +446,7 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
               }
+              __syncwarp();
               tmem_wait_st();
               asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
               __syncwarp();
@@ -594,18 +595,19 @@ Plan plan_of(int M, int N, int K) {
   ranges_of(N, K, ranges, range_blocks);
   const int64_t blocks = (K + KB - 1) / KB, tiles_n = (N + ROWS - 1) / ROWS, sms = gllm_sm_count();
   // a block's time, in ns: up to 64 tokens the cutting of the weight's 128 rows, beyond the tokens' as well
-  static const int widths[] = {16, 32, 64, 96};
-  static const float block_ns[] = {445.f, 450.f, 455.f, 560.f};
+  // and what a range's end costs where all are one item's (96 columns have one accumulator of the smaller products)
+  static const int widths[] = {16, 32, 64, 80, 96};
+  static const float block_ns[] = {445.f, 450.f, 455.f, 530.f, 565.f}, end_ns[] = {1000.f, 1000.f, 1000.f, 1000.f, 2500.f};
   Plan best{96, 0};
   float best_time = 0.f;
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < 5; ++i) {
     const int64_t tiles = tiles_n * ((M + widths[i] - 1) / widths[i]);
     for (int split = 0; split < 2; ++split) {
       const int64_t at_once = !split ? sms : ranges > 1 && ranges <= MOST_BLOCKS ? clusters_of(ranges) : 0;
       if (at_once <= 0) continue;
       const int64_t waves = (tiles + at_once - 1) / at_once;
       // (a range's start and the sum through shared memory: measured 3 us)
-      const float time = (float)waves * ((float)(split ? range_blocks : blocks) * block_ns[i] + (split ? 3000.f : 0.f));
+      const float time = (float)waves * ((float)(split ? range_blocks : blocks) * block_ns[i] + (split ? 3000.f : end_ns[i] * (float)ranges));
       if (best_time == 0.f || time < best_time) best = Plan{widths[i], split}, best_time = time;
     }
   }
@@ -657,6 +659,7 @@ GLLM_API int gllm_gemm_f32(const float* X, const float* W, float* C, int M, int 
       case 16: return parts3::launch<16>(X, W, C, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
       case 32: return parts3::launch<32>(X, W, C, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
       case 64: return parts3::launch<64>(X, W, C, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
+      case 80: return parts3::launch<80>(X, W, C, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
       default: return parts3::launch<96>(X, W, C, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
     }
   }
