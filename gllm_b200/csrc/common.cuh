@@ -215,6 +215,19 @@ static inline bool gllm_pdl_enabled() {
   return on != 0;
 }
 
+// Launches `kernel` on `stream` behind all of the kernel before it: for grids of unequal blocks that share SMs, longest first.
+// Started early they pile up on the SMs that the kernel before leaves first.
+template <typename... KArgs, typename... Args>
+static inline int gllm_launch_in_order(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                       Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // Launches `kernel` on `stream` with programmatic stream serialization allowed (see above);
 // returns the cudaError_t as an int.
 template <typename... KArgs, typename... Args>
