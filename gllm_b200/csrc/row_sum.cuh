@@ -12,35 +12,46 @@ struct RowSum {
   const float* weights;
   int top;
 
+  template <int VEC> static __device__ __forceinline__ void load(const float* p, float (&v)[VEC]) {
+    static_assert(VEC == 4 || VEC == 1, "one load");
+    if constexpr (VEC == 4) {
+      const float4 x = __ldcg(reinterpret_cast<const float4*>(p));
+      v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+    } else {
+      v[0] = __ldcg(p);
+    }
+  }
+
   // columns c .. c + VEC - 1 of token t (VEC 4: 16-byte aligned); the rows of four slots are requested together
   template <int VEC> __device__ __forceinline__ void sum(int64_t t, int c, int width, float (&acc)[VEC]) const {
 #pragma unroll
     for (int e = 0; e < VEC; ++e) acc[e] = 0.f;
     for (int s0 = 0; s0 < top; s0 += 4) {
-      float v[4][VEC];
+      // (rows and weights, then the first part of every slot: nothing waits for the slot before it)
+      const float* p[4];
+      float w[4], v[4][VEC];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) v[q][e] = 0.f;
-        if (s0 + q < top) {
-          const int64_t row = row_of_pair ? (int64_t)row_of_pair[t * top + s0 + q] : t * top + s0 + q;
-          const float* p = y + row * width + c;
-          for (int k = 0; k < n_parts; ++k, p += part_stride) {
-            if (VEC == 4) {
-              const float4 x = __ldcg(reinterpret_cast<const float4*>(p));
-              v[q][0] += x.x, v[q][VEC > 1 ? 1 : 0] += x.y, v[q][VEC > 2 ? 2 : 0] += x.z, v[q][VEC > 3 ? 3 : 0] += x.w;
-            } else {
-              v[q][0] += __ldcg(p);
-            }
-          }
-        }
+        const bool in = s0 + q < top;
+        const int64_t slot = t * top + (in ? s0 + q : s0);
+        p[q] = y + (row_of_pair ? (int64_t)row_of_pair[slot] : slot) * width + c;
+        w[q] = weights ? weights[slot] : 1.f;
       }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) load<VEC>(p[q], v[q]);
+      for (int k = 1; k < n_parts; ++k)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float x[VEC];
+          load<VEC>(p[q] + k * part_stride, x);
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) v[q][e] += x[e];
+        }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         if (s0 + q >= top) break;
-        const float w = weights ? weights[t * top + s0 + q] : 1.f;
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) acc[e] = fmaf(w, v[q][e], acc[e]);
+        for (int e = 0; e < VEC; ++e) acc[e] = fmaf(w[q], v[q][e], acc[e]);
       }
     }
   }
