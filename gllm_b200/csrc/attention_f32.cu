@@ -20,7 +20,7 @@ __device__ __forceinline__ unsigned long long twice(float x) {
 // ones in S, as many and 16 register pairs in P V) with three warps a scheduler (head size 64; two took 3 us more); a half warp is 4 x 4 threads, so a load takes
 // no more than two passes over the banks.  The warp-per-token kernel read every key row once per token and head, 32 rows
 // side by side: 2,515 us for 512 and 200 (over 300) tokens beside 8 single ones (about 1,000 keys), 32 heads of 64 over 8;
-// this kernel takes 128 us for the portions (10 of them for the look at broken values below), the split one 19 and its
+// this kernel takes 105 us for the portions (10 of them for the look at broken values below), the split one 19 and its
 // merge 5 for the single tokens.
 constexpr int ROWS = 64, KEYS = 64, PF_THREADS = 128, P_PITCH = KEYS + 4;
 
