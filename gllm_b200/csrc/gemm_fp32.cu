@@ -636,7 +636,7 @@ int launch(const float* X, const float* W, float* out, int M, int N, int K, int6
   const int64_t items = (int64_t)cut.tiles_n * cut.tiles_m * (split ? cut.ranges : 1);
   if (items > 0x7fffffff - 4096) return (int)cudaErrorInvalidValue;
   auto kernel = gemm_f32_parts_kernel<BT>;
-  static const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<BT>::SMEM);
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<BT>::SMEM);
   if (e != cudaSuccess) return (int)e;
   if (split)
     return gllm_launch_cluster(kernel, dim3((unsigned)items), dim3(THREADS), (size_t)Shape<BT>::SMEM, stream,
