@@ -289,32 +289,20 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
-      // pass 0: the weight blocks of the first STAGES stages, which no kernel before this one writes; pass 1: their tokens,
-      // then both operands of every later block as stages come free
-      for (int pass = 0; pass < 2 && ok; ++pass) {
-        if (pass == 1) pdl_wait();
-        it = 0;
-        bool more = true;
-        for (int w = blockIdx.x; w < num_items && ok && more; w += gridDim.x) {
-          int n0, m0, kb_begin, kb_end, range;
-          place<BT>(cut, w, n0, m0, kb_begin, kb_end, range);
-          for (int kb = kb_begin; kb < kb_end; ++kb, ++it) {
-            const uint32_t s = it % S::STAGES, round = it / S::STAGES, bar = smem_addr(&raw_full[s]);
-            const uint32_t dst = raw_base + s * S::RAW;
-            if (pass == 0) {
-              if (round > 0) { more = false; break; }
-              mbar_expect_tx(bar, (uint32_t)S::RAW);
-              tma_load_2d(dst, &map_w, kb * KB, n0, bar);
-            } else {
-              if (round > 0) {
-                ok = mbar_wait(smem_addr(&raw_empty[s]), (round & 1u) ^ 1u, status, &abort_flag);
-                if (!ok) break;
-                mbar_expect_tx(bar, (uint32_t)S::RAW);
-                tma_load_2d(dst, &map_w, kb * KB, n0, bar);
-              }
-              tma_load_2d(dst + ROWS * KB * 4, &map_x, kb * KB, m0, bar);
-            }
+      pdl_wait();                                          // (either operand may be what the kernel before writes)
+      for (int w = blockIdx.x; w < num_items && ok; w += gridDim.x) {
+        int n0, m0, kb_begin, kb_end, range;
+        place<BT>(cut, w, n0, m0, kb_begin, kb_end, range);
+        for (int kb = kb_begin; kb < kb_end; ++kb, ++it) {
+          const uint32_t s = it % S::STAGES, round = it / S::STAGES, bar = smem_addr(&raw_full[s]);
+          const uint32_t dst = raw_base + s * S::RAW;
+          if (round > 0) {
+            ok = mbar_wait(smem_addr(&raw_empty[s]), (round & 1u) ^ 1u, status, &abort_flag);
+            if (!ok) break;
           }
+          mbar_expect_tx(bar, (uint32_t)S::RAW);
+          tma_load_2d(dst, &map_w, kb * KB, n0, bar);
+          tma_load_2d(dst + ROWS * KB * 4, &map_x, kb * KB, m0, bar);
         }
       }
       if (abort_flag) {

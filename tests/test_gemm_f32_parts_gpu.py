@@ -65,3 +65,23 @@ def test_not_finite(m):
     b2 = b.clone()
     assert torch.equal(ops.linear(a[rows], b2)[:, cols], got[rows][:, cols])
     assert clean.isfinite().all()
+
+
+@pytest.mark.parametrize("m", [3, 90])
+@pytest.mark.parametrize("k", [64, 600])
+def test_weight_that_the_kernel_before_writes(m, k):
+    """Either operand may be the result of the product right before, in memory that held another one's: nothing waits in between."""
+    from gllm_b200 import ops
+
+    g = torch.Generator().manual_seed(m)
+    a, b, x = (torch.randn(*shape, generator=g).cuda() for shape in ((200, k), (600, k), (m, 600)))
+    held = torch.empty(200, 600, device="cuda")
+    for factor in (1.0, -1.0, 2.0, 0.0, 0.5):
+        first = factor * a
+        torch.cuda.synchronize()
+        y = ops.linear(first, b, out=held)
+        of_weight, of_both = ops.linear(x, y), ops.linear(y, y)
+        torch.cuda.synchronize()
+        want = first.double() @ b.double().T
+        for got, right in ((y, want), (of_weight, x.double() @ want.T), (of_both, want @ want.T)):
+            assert bool(((got.double() - right).abs() <= 1e-5 * right.abs().max()).all())
