@@ -2,13 +2,15 @@
 // gllm/model/layers/linear.py:20 with W stored [out, in].  This is the path
 // that shows faults bf16 hides: no operand is rounded.
 //
-// Two kernels.  Rows on 16-byte boundaries and K a multiple of 4, 32 or more,
-// run on the tensor cores with every 32-bit number cut into three bfloat16
+// Three kernels.  Rows on 16-byte boundaries and K a multiple of 4 run, up to
+// K = 512, on packed 32-bit multiply-adds (tiles of 16 x 16 to 64 x 64), and
+// beyond on the tensor cores with every 32-bit number cut into three bfloat16
 // whose sum it is (8 bits of its significand each, rounded to nearest, so
 // nothing is lost):
 //   x = x0 + x1 + x2,  w = w0 + w1 + w2,
 //   x w = w0 x0 + (w0 x1 + w1 x0 + w0 x2 + w1 x1 + w2 x0) + terms below 2^-26 |x w|.
-// Everything else runs a plain 64 x 64 tile of 32-bit multiply-adds.
+// Everything else runs a plain 64 x 64 tile of 32-bit multiply-adds.  In both
+// multiply-add kernels an output is two sums, of even and of odd k.
 //
 // The tensor cores' own additions truncate.  The leading products' accumulator
 // is therefore taken out of tensor memory every 256 of K (16 additions) and
@@ -90,6 +92,142 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
       if (n < N) C[(int64_t)m * ldc + n] = acc[0][i][j] + acc[1][i][j];
     }
   }
+}
+
+// ------------------------------------------------------------------ packed multiply-adds
+// Rows lie in shared memory as they do in memory, [row][k], filled by cp.async several k-tiles ahead.
+// A thread owns TM x TN outputs (rows and columns TY and TX apart).  Four k at a time it reads 16 bytes of each of its
+// rows and multiplies them as two packed pairs (fma.rn.f32x2), so an output is kept as two sums, of the products with
+// even and with odd k, each in ascending order; they are added at the end.
+constexpr int PK = 32, PITCH = PK + 4;   // (a pitch of 9 sixteen-byte pieces: eight neighbouring rows on eight bank groups)
+
+template <int BM_, int BN_, int TM_, int TN_, int STAGES, int UNROLL>
+__global__ void __launch_bounds__((BM_ / TM_) * (BN_ / TN_))
+gemm_f32_pairs_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M, int N,
+                      int K, int64_t lda, int64_t ldb, int64_t ldc) {
+  constexpr int TY = BM_ / TM_, TX = BN_ / TN_, THREADS = TX * TY, ROWS = BM_ + BN_;
+  static_assert(TX % 8 == 0 && TY % 4 == 0, "a warp's threads lie 4 by 8");
+  extern __shared__ __align__(16) float tiles[];          // [STAGES][BM_ + BN_][PITCH]
+  pdl_trigger();
+  // A warp's threads lie 4 rows by 8 columns, a half warp 4 by 4: a 16-byte load is served a half warp at a time when
+  // its addresses fit one pass over the banks, so neither operand's load takes more than two.
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tx = (warp % (TX / 8)) * 8 + (lane & 3) + (lane >> 4) * 4, ty = (warp / (TX / 8)) * 4 + ((lane >> 2) & 3);
+  const int m0 = blockIdx.y * BM_, n0 = blockIdx.x * BN_;
+  // a thread copies piece `piece` of the rows row0, row0 + STEP, ...: of A's first, of B's behind them
+  constexpr int PIECES = PK / 4, STEP = THREADS / PIECES, COPIES = ROWS / STEP;
+  static_assert(THREADS % PIECES == 0 && BM_ % STEP == 0 && BN_ % STEP == 0, "whole rows per round of copies");
+  const int piece = tid % PIECES, row0 = tid / PIECES;
+  const float* a_src = A + (int64_t)(m0 + row0) * lda + piece * 4;
+  const float* b_src = B + (int64_t)(n0 + row0) * ldb + piece * 4;
+  const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(tiles) + (uint32_t)((row0 * PITCH + piece * 4) * sizeof(float));
+  auto request = [&](int k0, int stage) {
+    const bool k_in = k0 + piece * 4 < K;
+    const uint32_t dst = dst0 + (uint32_t)(stage * ROWS * PITCH * sizeof(float));
+#pragma unroll
+    for (int c = 0; c < COPIES; ++c) {
+      const bool is_a = c < BM_ / STEP;
+      const int r = is_a ? c * STEP : c * STEP - BM_;
+      const bool in = k_in && (is_a ? m0 + row0 + r < M : n0 + row0 + r < N);
+      const float* src = is_a ? a_src + k0 + r * lda : b_src + k0 + r * ldb;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)(c * STEP * PITCH * sizeof(float))),
+                   "l"(in ? src : A), "r"(in ? 16 : 0) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  unsigned long long acc[TM_][TN_];
+#pragma unroll
+  for (int i = 0; i < TM_; ++i)
+#pragma unroll
+    for (int j = 0; j < TN_; ++j) acc[i][j] = 0ull;
+  const int k_tiles = (K + PK - 1) / PK;
+  pdl_wait();
+#pragma unroll
+  for (int t = 0; t < STAGES - 1; ++t) {
+    if (t < k_tiles) request(t * PK, t);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  int stage = 0;
+  for (int t = 0; t < k_tiles; ++t) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();                                       // tile t is there, and nobody reads tile t - 1 any more
+    const int ahead = t + STAGES - 1;
+    if (ahead < k_tiles) request(ahead * PK, stage == 0 ? STAGES - 1 : stage - 1);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* a_s = tiles + (stage * ROWS + ty) * PITCH;
+    const float* b_s = tiles + (stage * ROWS + BM_ + tx) * PITCH;
+#pragma unroll UNROLL
+    for (int kk = 0; kk < PK; kk += 4) {
+      ulonglong2 a[TM_];
+#pragma unroll
+      for (int i = 0; i < TM_; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(a_s + i * TY * PITCH + kk);
+#pragma unroll
+      for (int j = 0; j < TN_; ++j) {
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(b_s + j * TX * PITCH + kk);
+#pragma unroll
+        for (int i = 0; i < TM_; ++i) fma2(acc[i][j], a[i].x, b.x);
+#pragma unroll
+        for (int i = 0; i < TM_; ++i) fma2(acc[i][j], a[i].y, b.y);
+      }
+    }
+    stage = stage + 1 == STAGES ? 0 : stage + 1;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < TM_; ++i) {
+    const int m = m0 + ty + i * TY;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < TN_; ++j) {
+      const int n = n0 + tx + j * TX;
+      if (n < N)
+        C[(int64_t)m * ldc + n] = pair_sum(acc[i][j]);
+    }
+  }
+}
+
+template <int BM_, int BN_, int TM_, int TN_, int STAGES, int UNROLL>
+int gemm_f32_pairs(const float* A, const float* B, float* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
+                   cudaStream_t stream) {
+  constexpr size_t smem = sizeof(float) * STAGES * (BM_ + BN_) * PITCH;
+  auto kernel = gemm_f32_pairs_kernel<BM_, BN_, TM_, TN_, STAGES, UNROLL>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  if (e != cudaSuccess) return (int)e;
+  // (tiles of rows lie along y, at most 65,535 a launch)
+  for (int m0 = 0; m0 < M; m0 += 65535 * BM_) {
+    const int rows = M - m0 < 65535 * BM_ ? M - m0 : 65535 * BM_;
+    const dim3 grid((N + BN_ - 1) / BN_, (rows + BM_ - 1) / BM_);
+    // Blocks that start while the kernel before them drains land wherever a place frees first.  Asking for a share of an
+    // SM's shared memory that lets no SM take more than its even share of the blocks keeps them spread.
+    const int64_t per_sm = ((int64_t)grid.x * grid.y + gllm_sm_count() - 1) / gllm_sm_count();
+    const int64_t share = 228 * 1024 / per_sm - 1024;            // (1 KB of every block's share is the system's)
+    const size_t ask = share > (int64_t)smem ? (size_t)(share < 227 * 1024 ? share : 227 * 1024) : smem;
+    const int rc = gllm_launch(kernel, grid, dim3((BM_ / TM_) * (BN_ / TN_)), ask, stream, A + (int64_t)m0 * lda, B,
+                               C + (int64_t)m0 * ldc, rows, N, K, lda, ldb, ldc);
+    if (rc != 0) return rc;
+  }
+  return 0;
+}
+// Which tile: the one whose fullest SM ends first.  A tile's time per k is `chain` (ns) while it has an SM to itself and
+// `work` times the tiles of the SM once they fill it; tiles of two warps count in pairs (an SM has four schedulers).
+// Measured per tile at K = 8,192 and 148 SMs (one tile an SM; 10 and more): the larger a tile the less it reads per
+// product, the smaller the better it spreads.  Steps of up to 16 tokens take the smallest tile, which streams the
+// weight best (16,384 x 2,048: 64 us against 95 with 32 x 32).
+int pairs_tile_of(int M, int N) {
+  struct Tile { int m, n, pairs; float chain, work; };
+  static const Tile tiles[] = {{16, 16, 1, 10.4f, 3.66f}, {32, 16, 1, 13.2f, 5.2f}, {32, 32, 1, 19.4f, 7.4f},
+                               {64, 32, 1, 30.f, 13.8f}, {64, 64, 0, 33.7f, 26.4f}, {64, 64, 1, 56.4f, 25.f}};
+  if (M <= 16) return 0;
+  int best = 0;
+  float best_time = 0.f;
+  for (int i = 0; i < 6; ++i) {
+    const Tile& t = tiles[i];
+    int64_t per_sm = ((int64_t)((M + t.m - 1) / t.m) * ((N + t.n - 1) / t.n) + gllm_sm_count() - 1) / gllm_sm_count();
+    if (t.pairs) per_sm = (per_sm + 1) & ~(int64_t)1;
+    const float work = t.work * (float)per_sm, time = work > t.chain ? work : t.chain;
+    if (i == 0 || time < best_time) best = i, best_time = time;
+  }
+  return best;
 }
 
 // ------------------------------------------------------------------ three parts a number, on the tensor cores
@@ -639,18 +777,30 @@ bool on_vectors(const float* X, const float* W, int K, int64_t ldx, int64_t ldw)
   return K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0 &&
          (reinterpret_cast<uintptr_t>(W) & 15) == 0;
 }
-// Whether the tensor-core kernel takes them: short of one block of K most of its work would be padding.
-bool in_parts(const float* X, const float* W, int K, int64_t ldx, int64_t ldw) {
-  return K >= parts3::KB && on_vectors(X, W, K, ldx, ldw);
-}
+// Sums of up to 512 products stay with multiply-adds: by K alone, as a token's result may not depend on its batch.  The
+// tensor-core kernel costs a start and an end of 4 us whatever K is (us, multiply-adds against parts: 8 x 1,024 x 256 3.9 against 6.3,
+// 8 x 512 x 512 6.4 : 7.4, 8 x 1,024 x 1,024 11.7 : 7.4); with many tokens it is ahead from K = 256 on (2,048 x 512 x 512 33 : 16),
+// which a decode step between two prompts does not get back.
+constexpr int SHORT_SUM = 512;
 }  // namespace
 
 GLLM_API int gllm_gemm_f32(const float* X, const float* W, float* C, int M, int N, int K, int64_t ldx, int64_t ldw,
                            int64_t ldc, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return (int)cudaErrorInvalidValue;
-  if (M > (on_vectors(X, W, K, ldx, ldw) ? 128 : BM) * 65535) return (int)cudaErrorInvalidValue;
-  if (in_parts(X, W, K, ldx, ldw)) {
+  const bool vectors = on_vectors(X, W, K, ldx, ldw);
+  if (M > (vectors ? 128 : BM) * 65535) return (int)cudaErrorInvalidValue;
+  if (vectors && K <= SHORT_SUM) {
+    switch (pairs_tile_of(M, N)) {
+      case 0: return gemm_f32_pairs<16, 16, 2, 2, 6, 8>(X, W, C, M, N, K, ldx, ldw, ldc, stream);
+      case 1: return gemm_f32_pairs<32, 16, 4, 2, 6, 8>(X, W, C, M, N, K, ldx, ldw, ldc, stream);
+      case 2: return gemm_f32_pairs<32, 32, 4, 4, 4, 8>(X, W, C, M, N, K, ldx, ldw, ldc, stream);
+      case 3: return gemm_f32_pairs<64, 32, 8, 4, 4, 8>(X, W, C, M, N, K, ldx, ldw, ldc, stream);
+      case 4: return gemm_f32_pairs<64, 64, 8, 4, 3, 8>(X, W, C, M, N, K, ldx, ldw, ldc, stream);
+      default: return gemm_f32_pairs<64, 64, 8, 8, 3, 1>(X, W, C, M, N, K, ldx, ldw, ldc, stream);
+    }
+  }
+  if (vectors) {
     const parts3::Plan plan = parts3::plan_of(M, N, K);
     switch (plan.bt) {
       case 16: return parts3::launch<16>(X, W, C, M, N, K, ldx, ldw, ldc, plan.split, status, stream);
