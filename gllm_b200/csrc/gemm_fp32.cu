@@ -13,7 +13,7 @@
 // multiply-add kernels an output is two sums, of even and of odd k.
 //
 // The tensor cores' own additions truncate.  The leading products' accumulator
-// is therefore taken out of tensor memory every 256 of K (16 additions) and
+// is therefore taken out of tensor memory every 128 .. 256 of K (chunk_of) and
 // added to 32-bit sums in registers, rounded to nearest; the other five
 // products are 2^-8 of it and stay in theirs for a whole range of K.
 //
@@ -234,7 +234,6 @@ int pairs_tile_of(int M, int N) {
 namespace parts3 {
 constexpr int ROWS = 128;           // weight rows of a tile (MMA M)
 constexpr int KB = 32;              // k per block: 32 floats = one 128-byte swizzle row, 32 bf16 = one of 64 bytes
-constexpr int CHUNK = 8;            // blocks between two visits to the leading accumulator
 constexpr int WORKERS = 16;         // warps that cut operands into parts and keep the sums
 constexpr int GROUPS = 4;           // of workers, that take turns with the blocks
 constexpr int THREADS = (WORKERS + 2) * 32;
@@ -320,6 +319,7 @@ __device__ __forceinline__ void cut8(const float4& a, const float4& b, uint32_t 
 struct Cut {                        // how the work is laid out
   int tiles_n, tiles_m;             // tiles of weight rows, of tokens
   int ranges, range_blocks, blocks; // of K
+  int chunk, extra;                 // blocks between two visits to the leading accumulator; more in a range's first
   int split;                        // 1: an item is one range of a tile, a block each, a cluster a tile; 0: all of them
 };
 
@@ -474,8 +474,8 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         ok = wait_u(&cross_empty[cb], ((segments / S::CROSS) & 1u) ^ 1u);
         if (!ok) break;
         const uint32_t d_cross = tmem_cross + cb * BT;
-        for (int kb = r0; kb < r1; ++kb, ++it) {
-          const bool chunk_first = (kb - r0) % CHUNK == 0, chunk_last = (kb - r0) % CHUNK == CHUNK - 1 || kb + 1 == r1;
+        for (int kb = r0, in_chunk = 0, len = cut.chunk + cut.extra; kb < r1; ++kb, ++it) {
+          const bool chunk_first = in_chunk == 0, chunk_last = in_chunk + 1 == len || kb + 1 == r1;
           const uint32_t mb = chunks & 1u, d_main = tmem_main + mb * BT;
           if (chunk_first) {
             ok = wait_u(&main_empty[mb], ((chunks >> 1) & 1u) ^ 1u);
@@ -504,7 +504,8 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             if (chunk_last) umma_commit(smem_addr(&main_full[mb]));
           }
           __syncwarp();
-          if (chunk_last) ++chunks;
+          if (chunk_last) ++chunks, in_chunk = 0, len = cut.chunk;
+          else ++in_chunk;
         }
       }
     }
@@ -544,8 +545,8 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
       if (more) place<BT>(cut, item, n0, m0, kb_begin, kb_end, range);
       for (int r0 = kb_begin; r0 < kb_end && ok; r0 += cut.range_blocks) {
         const int r1 = min(kb_end, r0 + cut.range_blocks);
-        for (int c0 = r0; c0 < r1 && ok; c0 += CHUNK) {
-          const int blocks = more ? min(CHUNK, r1 - c0) : 0;
+        for (int c0 = r0, len = cut.chunk + cut.extra; c0 < r1 && ok; c0 += len, len = cut.chunk) {
+          const int blocks = more ? min(len, r1 - c0) : 0;
           // this group's blocks of the chunk
           for (int j = (group - it) % GROUPS; ok; j += GROUPS) {
             if (j < blocks) {
@@ -619,7 +620,7 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
           it += blocks;
           pending = true;
           p_item = item;
-          p_end = c0 + CHUNK >= r1 ? r1 : 0;
+          p_end = c0 + len >= r1 ? r1 : 0;
         }
       }
       if (!more) break;
@@ -723,6 +724,12 @@ void ranges_of(int N, int K, int& ranges, int& range_blocks) {
   ranges = (blocks + range_blocks - 1) / range_blocks;     // (none is empty)
 }
 
+// Blocks between two visits to the leading accumulator.  Its truncations err to one side, so where all products have one sign a
+// sum errs by half a chunk's additions whatever K is (1.7e-7 with 4 blocks, 2.1e-7 with 6, 2.8e-7 with 7, 3.8e-7 with 8), while
+// the rounding of multiply-adds errs by the root of K (1.9e-7 at 640, 2.6e-7 at 1,280, 3.5e-7 at 2,048, 5.0e-7 at 4,096): no chunk
+// is longer than leaves such a sum as close to 64 bits as multiply-adds leave it.
+int chunk_of(int K) { return K < 1280 ? 4 : K < 2048 ? 6 : K < 4096 ? 7 : 8; }
+
 // Tokens per tile and whether an item is one range: the layout whose fullest SM ends first.
 struct Plan { int bt, split; };
 Plan plan_of(int M, int N, int K) {
@@ -759,6 +766,9 @@ int launch(const float* X, const float* W, float* out, int M, int N, int K, int6
   cut.blocks = (K + KB - 1) / KB;
   cut.tiles_n = (N + ROWS - 1) / ROWS, cut.tiles_m = (M + BT - 1) / BT;
   cut.split = split;
+  cut.chunk = chunk_of(K);
+  // (64 blocks as 8 + 7 + .. + 7: 3.0e-7, and a visit less: 700 x 16,384 x 2,048 264 us for 271)
+  cut.extra = cut.chunk == 7 && cut.range_blocks > 8 && cut.range_blocks % 7 == 1;
   const int64_t items = (int64_t)cut.tiles_n * cut.tiles_m * (split ? cut.ranges : 1);
   if (items > 0x7fffffff - 4096) return (int)cudaErrorInvalidValue;
   auto kernel = gemm_f32_parts_kernel<BT>;

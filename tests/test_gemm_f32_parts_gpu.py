@@ -91,7 +91,7 @@ def _off(got, want):
     return ((got.double() - want).norm() / want.norm()).item()
 
 
-@pytest.mark.parametrize("k", [32, 64, 96, 128, 256, 384, 512])
+@pytest.mark.parametrize("k", [32, 64, 96, 128, 256, 384, 512, 516, 640, 1024, 1280, 1792, 2048, 4096])
 @pytest.mark.parametrize("signs", ["both", "one"])
 def test_no_further_from_64_bits_than_multiply_adds(k, signs):
     """Rows off 16-byte boundaries run plain 32-bit multiply-adds, two sums a result; the others may not err by more.  (Each error is
