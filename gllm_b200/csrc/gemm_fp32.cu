@@ -5,10 +5,10 @@
 // Three kernels.  Rows on 16-byte boundaries and K a multiple of 4 run, up to
 // K = 512, on packed 32-bit multiply-adds (tiles of 16 x 16 to 64 x 64), and
 // beyond on the tensor cores with every 32-bit number cut into three bfloat16
-// whose sum it is (8 bits of its significand each, rounded to nearest, so
-// nothing is lost):
+// whose sum it is (8 bits of its significand each, rounded to nearest; times
+// 2^16 first, so that nothing is lost of the smallest numbers either):
 //   x = x0 + x1 + x2,  w = w0 + w1 + w2,
-//   x w = w0 x0 + (w0 x1 + w1 x0 + w0 x2 + w1 x1 + w2 x0) + terms below 2^-26 |x w|.
+//   x w = w0 x0 + (w0 x1 + w1 x0 + w0 x2 + w1 x1 + w2 x0) + terms of up to 2^-24 |x w|.
 // Everything else runs a plain 64 x 64 tile of 32-bit multiply-adds.  In both
 // multiply-add kernels an output is two sums, of even and of odd k.
 //
@@ -24,7 +24,9 @@
 // way, so a token's result does not depend on the batch it is in.
 //
 // A result that is not finite is computed again with 32-bit multiply-adds from
-// the operands themselves: the parts of an infinity are not its sum.
+// the operands themselves: the parts of an infinity are not its sum, and sums
+// that are 2^32 times too large may end where the result does not (from 2^96 on,
+// or with operands from 2^111 on).
 //
 // What bounds it: with many tokens the cutting (sixteen warps, about 400 issue
 // cycles for a block of 32 k) and shared memory (110 KB, 860 cycles), where the
@@ -241,6 +243,8 @@ constexpr int RANGE_BLOCKS = 64;    // longest range of K (2,048), as long as th
 constexpr int MOST_RANGES = 16;     // (eight where they are a cluster's blocks)
 constexpr int MOST_BLOCKS = 8;
 constexpr int A_COLS = 3 * KB / 2;  // tensor-memory columns of one block of the weight's parts
+constexpr float UP = 65536.f;       // operands are cut times 2^16: the last bit of the smallest number is then one bfloat16 has
+constexpr float DOWN = 1.f / (UP * UP);
 
 template <int BT>
 struct Shape {
@@ -300,18 +304,23 @@ __device__ __forceinline__ uint32_t pack2(float low, float high) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(low, high);
   return *reinterpret_cast<const uint32_t*>(&h);
 }
-// Eight numbers as three parts each, two to a word.
+__device__ __forceinline__ unsigned long long pair_of(float low, float high) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(low), "f"(high));
+  return v;
+}
+// Eight numbers, times 2^16, as three parts each, two to a word.
 __device__ __forceinline__ void cut8(const float4& a, const float4& b, uint32_t (&p)[3][4]) {
-  float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    float lo = x[2 * i], hi = x[2 * i + 1];
+    unsigned long long left = pair_of(x[2 * i], x[2 * i + 1]);
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(left) : "l"(pair_of(UP, UP)));
 #pragma unroll
     for (int part = 0; part < 3; ++part) {
-      const uint32_t w = pack2(lo, hi);
-      p[part][i] = w;
-      lo -= __uint_as_float(w << 16);                      // (exact: what is left has no more bits than the number had)
-      hi -= __uint_as_float(w & 0xffff0000u);
+      const uint32_t w = pack2(pair_low(left), pair_high(left));
+      p[part][i] = w;                                      // (exact: what is left has no more bits than the number had)
+      asm("sub.rn.f32x2 %0, %0, %1;" : "+l"(left) : "l"(pair_of(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u))));
     }
   }
 }
@@ -366,7 +375,7 @@ __device__ __forceinline__ void put_range(const Cut& cut, int item, int end, int
 #pragma unroll
   for (int i = 0; i < COLS; ++i) {
     if (i < tokens) {
-      const float v = acc[i];
+      const float v = acc[i] * DOWN;
       broken = broken || !is_finite(v);
       if (joins) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + i * ldo), "f"(v) : "memory");   // (nothing to wait for)
       else dst[i * ldo] = v;
@@ -646,7 +655,7 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         const int c = i / each, r = (int)mine * each + i - c * each, m = m0 + c, n = n0 + r;
         if (r >= ROWS || m >= M || n >= N) continue;
         float v = 0.f;
-        for (int j = 0; j < cut.ranges; ++j) v += parts[j * BT * each + i];
+        for (int j = 0; j < cut.ranges; ++j) v += parts[j * BT * each + i] * DOWN;
         if (!is_finite(v)) v = again(X + (int64_t)m * ldx, W + (int64_t)n * ldw, K);
         out[(int64_t)m * ldo + n] = v;
       }

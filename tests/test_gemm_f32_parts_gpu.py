@@ -105,3 +105,16 @@ def test_no_further_from_64_bits_than_multiply_adds(k, signs):
     a = wide[:, :k]
     want = a.double() @ b.double().T
     assert _off(ops.linear(a.contiguous(), b), want) <= 1.03 * _off(ops.linear(a, b), want)
+
+
+@pytest.mark.parametrize("scale_a,scale_b", [(1e-33, 1e30), (1e-35, 1e30), (1e-36, 1e30), (1e-37, 1e33), (1e30, 1e-37), (1e-39, 1e33)])
+@pytest.mark.parametrize("k", [260, 1032])
+def test_smallest_numbers_keep_their_bits(scale_a, scale_b, k):
+    """Operands down to the subnormal ones are what they are: the errors of 32-bit sums, relative to the result."""
+    from gllm_b200 import ops
+
+    g = torch.Generator().manual_seed(5)
+    a, b = (torch.randn(70, k, generator=g) * scale_a).cuda(), (torch.randn(130, k, generator=g) * scale_b).cuda()
+    want = a.double() @ b.double().T
+    # (5.7e-7 is what multiply-adds leave at K = 2,048; without the third part it would be 4e-6)
+    assert _off(ops.linear(a, b), want) <= 6e-7
