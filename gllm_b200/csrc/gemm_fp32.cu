@@ -356,6 +356,15 @@ __device__ __noinline__ float again(const float* __restrict__ x, const float* __
   return s;
 }
 __device__ __forceinline__ bool is_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+// The sum of one range of several, out of the accumulators.  Additions in memory take what is subnormal for zero.  Sums of 2^-102 and
+// more (and zeros) add up to nothing subnormal, as their last bits are 2^-125 and more; a smaller one becomes a NaN, and the
+// result is computed again.
+constexpr uint32_t LEAST = (uint32_t)(127 - 102) << 24;    // 2^-102, without its sign
+__device__ __forceinline__ float range_sum(float v) {
+  return (__float_as_uint(v) << 1) - 1u < LEAST - 1u ? __uint_as_float(0x7fffffffu) : v;
+}
+// 0xff000000 - LEAST and more: v is zero, smaller than 2^-102 or not finite.
+__device__ __forceinline__ uint32_t unusual(float v) { return (__float_as_uint(v) << 1) - LEAST; }
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
@@ -372,13 +381,25 @@ __device__ __forceinline__ void put_range(const Cut& cut, int item, int end, int
   if (n >= N || tokens <= 0) return;
   float* const dst = out + (int64_t)m * ldo + n;
   const bool joins = end > cut.range_blocks;
+  float v[COLS];
+  uint32_t most = 0;
+#pragma unroll
+  for (int i = 0; i < COLS; ++i) {
+    v[i] = acc[i] * DOWN;
+    most = max(most, unusual(v[i]));
+  }
+  if (most >= 0xff000000u - LEAST) {                       // (the columns behind the last token are zero: rare but there)
+#pragma unroll
+    for (int i = 0; i < COLS; ++i) {
+      if (cut.ranges > 1) v[i] = range_sum(v[i]);
+      broken = broken || !is_finite(v[i]);
+    }
+  }
 #pragma unroll
   for (int i = 0; i < COLS; ++i) {
     if (i < tokens) {
-      const float v = acc[i] * DOWN;
-      broken = broken || !is_finite(v);
-      if (joins) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + i * ldo), "f"(v) : "memory");   // (nothing to wait for)
-      else dst[i * ldo] = v;
+      if (joins) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + i * ldo), "f"(v[i]) : "memory");   // (nothing to wait for)
+      else dst[i * ldo] = v[i];
     }
   }
   if (end != kb_end) return;
@@ -655,7 +676,7 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         const int c = i / each, r = (int)mine * each + i - c * each, m = m0 + c, n = n0 + r;
         if (r >= ROWS || m >= M || n >= N) continue;
         float v = 0.f;
-        for (int j = 0; j < cut.ranges; ++j) v += parts[j * BT * each + i] * DOWN;
+        for (int j = 0; j < cut.ranges; ++j) v += range_sum(parts[j * BT * each + i] * DOWN);
         if (!is_finite(v)) v = again(X + (int64_t)m * ldx, W + (int64_t)n * ldw, K);
         out[(int64_t)m * ldo + n] = v;
       }

@@ -118,3 +118,17 @@ def test_smallest_numbers_keep_their_bits(scale_a, scale_b, k):
     want = a.double() @ b.double().T
     # (5.7e-7 is what multiply-adds leave at K = 2,048; without the third part it would be 4e-6)
     assert _off(ops.linear(a, b), want) <= 6e-7
+
+
+@pytest.mark.parametrize("m", [70, 300])
+def test_subnormal_results(m):
+    """To half a unit of the smallest number, and a fifth of that for the sums of some 40,000 units; and the same in a batch as alone."""
+    from gllm_b200 import ops
+
+    g = torch.Generator().manual_seed(m)
+    a, b = (torch.randn(m, 4100, generator=g) * 1e-21).cuda(), (torch.randn(2048, 4100, generator=g) * 1e-21).cuda()
+    got = ops.linear(a, b)
+    want = a.double() @ b.double().T
+    assert bool(((got.double() - want).abs() <= 1.2 * 2.0 ** -150).all())
+    for row in (0, m - 1):
+        assert torch.equal(ops.linear(a[row:row + 1].contiguous(), b)[0], got[row])
