@@ -715,8 +715,7 @@ bool make_map(CUtensorMap* map, const float* base, int rows, int cols, int64_t l
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// How many clusters of `blocks` blocks run at once, one block an SM (clusters do not reach across the SMs' groups: 148 SMs hold
-// 22 clusters of six but 15 of seven or eight).
+// How many clusters of `blocks` blocks this device runs at once, one block an SM (clusters do not reach across the SMs' groups).
 int clusters_of(int blocks) {
   static const struct Table {
     int count[MOST_BLOCKS + 1] = {};
@@ -738,13 +737,15 @@ int clusters_of(int blocks) {
   return table.count[blocks];
 }
 
-// Ranges of K: a function of (N, K) alone.  As many blocks to a cluster as leave all tiles of one step of few tokens running at
-// once, each range at least eight blocks of K long, and enough that none is longer than RANGE_BLOCKS.
+// Ranges of K: a function of (N, K) alone, also on a device that holds fewer clusters or none (there the ranges of a tile follow
+// one another; the order of the sums is the same).  As many blocks to a cluster as leave all tiles of one step of few tokens
+// running at once on a B200, each range at least eight blocks of K long, and enough that none is longer than RANGE_BLOCKS.
+constexpr int AT_ONCE[MOST_BLOCKS + 1] = {0, 0, 74, 45, 33, 26, 22, 15, 15};   // clusters_of() on 148 SMs
 void ranges_of(int N, int K, int& ranges, int& range_blocks) {
   const int blocks = (K + KB - 1) / KB, tiles = (N + ROWS - 1) / ROWS;
   int want = 1;
   for (int c = 2; c <= MOST_BLOCKS; ++c)
-    if (clusters_of(c) >= tiles) want = c;
+    if (AT_ONCE[c] >= tiles) want = c;
   if (want > blocks / 8) want = blocks / 8;
   const int least = (blocks + RANGE_BLOCKS - 1) / RANGE_BLOCKS;
   if (want < least) want = least;
@@ -823,6 +824,13 @@ bool on_vectors(const float* X, const float* W, int K, int64_t ldx, int64_t ldw)
 // which a decode step between two prompts does not get back.
 constexpr int SHORT_SUM = 512;
 }  // namespace
+
+// Blocks of 32 k in a range of a sum of K products on the tensor cores.
+GLLM_API int gllm_gemm_f32_range_blocks(int N, int K) {
+  int ranges, range_blocks;
+  parts3::ranges_of(N, K, ranges, range_blocks);
+  return range_blocks;
+}
 
 GLLM_API int gllm_gemm_f32(const float* X, const float* W, float* C, int M, int N, int K, int64_t ldx, int64_t ldw,
                            int64_t ldc, int* status, cudaStream_t stream) {
