@@ -346,16 +346,87 @@ __device__ __forceinline__ void place(const Cut& cut, int w, int& n0, int& m0, i
   kb_end = cut.split ? min(cut.blocks, kb_begin + cut.range_blocks) : cut.blocks;
 }
 
-// A result once more, with 32-bit multiply-adds.
-__device__ __noinline__ float again(const float* __restrict__ x, const float* __restrict__ w, int K) {
-  float s = 0.f;
-  for (int k = 0; k < K; k += 4) {
-    const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
-    s = fmaf(a.x, b.x, s), s = fmaf(a.y, b.y, s), s = fmaf(a.z, b.z, s), s = fmaf(a.w, b.w, s);
-  }
-  return s;
-}
 __device__ __forceinline__ bool is_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+__device__ __forceinline__ bool any_of_workers(bool mine) {          // (a barrier of theirs as well)
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(any)
+      : "r"(mine ? 1u : 0u), "n"(WORKERS * 32)
+      : "memory");
+  return any != 0;
+}
+// The results that are not finite, of the weight rows n0 .. n0 + rows and the tokens m0 .. m0 + BT, once more with 32-bit
+// multiply-adds (two sums each, of even and of odd k) by all workers, who are done with the stages: their memory holds the tiles.
+// A thread takes rows 32 and columns 16 apart; a warp's threads lie 4 rows by 8 columns, a half warp 4 by 4.  What bounds it: the
+// shared-memory loads.  700 x 16,384 x 2,048 with a NaN in one token 784 us, in every token 2,030; 669 and 34,400 when a thread
+// walked a weight row for each result, 1,020 where all of it is multiply-adds.
+template <int BT>
+__device__ __noinline__ void once_more(const float* __restrict__ X, const float* __restrict__ W, float* out, int M, int N, int K,
+                                       int64_t ldx, int64_t ldw, int64_t ldo, int n0, int rows, int m0) {
+  extern __shared__ unsigned char smem_dyn[];
+  constexpr int PITCH_ = KB + 4, COLS = BT / 16, LINES = ROWS + BT;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ty = (warp >> 1) * 4 + ((lane >> 2) & 3), tx = (warp & 1) * 8 + (lane & 3) + (lane >> 4) * 4;
+  const int count = min(rows, N - n0), tokens = min(BT, M - m0);
+  auto at = [&](int i, int j) { return out + (int64_t)(m0 + tx + 16 * j) * ldo + n0 + ty + 32 * i; };
+  uint32_t need = 0;                                       // the columns (of 16 apart) that this warp has to do
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < COLS; ++j)
+      if (ty + 32 * i < count && tx + 16 * j < tokens && !is_finite(__ldcg(at(i, j)))) need |= 1u << j;
+  need = __reduce_or_sync(0xffffffffu, need);
+  if (!any_of_workers(need != 0)) return;
+  const uint32_t base = (smem_addr(smem_dyn) + 15u) & ~15u;
+  const float* const tiles = reinterpret_cast<const float*>(smem_dyn + (base - smem_addr(smem_dyn)));
+  auto request = [&](int k0, int stage) {
+    for (int p = threadIdx.x; p < LINES * (KB / 4); p += WORKERS * 32) {
+      const int line = p / (KB / 4), k = k0 + p % (KB / 4) * 4;
+      const bool of_w = line < ROWS, in = k < K && (of_w ? line < count : line - ROWS < tokens);
+      const float* src = !in ? W : of_w ? W + (int64_t)(n0 + line) * ldw + k : X + (int64_t)(m0 + line - ROWS) * ldx + k;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + (uint32_t)((stage * LINES + line) * PITCH_ + k - k0) * 4u),
+                   "l"(src), "r"(in ? 16 : 0) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  unsigned long long sum[4][COLS];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < COLS; ++j) sum[i][j] = 0ull;
+  constexpr int AHEAD = 3;                                 // tiles in flight
+  static_assert((AHEAD + 1) * LINES * PITCH_ * 4 <= Shape<BT>::STAGES * Shape<BT>::RAW, "the stages' memory");
+  for (int t = 0; t < AHEAD; ++t) request(t * KB, t);
+  for (int k0 = 0, stage = 0; k0 < K; k0 += KB, stage = (stage + 1) & AHEAD) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD - 1) : "memory");
+    any_of_workers(false);                                 // the tile is there, and nobody reads the one before any more
+    request(k0 + AHEAD * KB, (stage + AHEAD) & AHEAD);
+    const float* w_s = tiles + (stage * LINES + ty) * PITCH_;
+    const float* x_s = tiles + (stage * LINES + ROWS + tx) * PITCH_;
+    if (!need) continue;
+#pragma unroll 2
+    for (int k = 0; k < KB; k += 4) {
+      ulonglong2 w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const ulonglong2*>(w_s + 32 * i * PITCH_ + k);
+#pragma unroll
+      for (int j = 0; j < COLS; ++j) {
+        if (!(need >> j & 1)) continue;
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(x_s + 16 * j * PITCH_ + k);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) fma2(sum[i][j], w[i].x, x.x), fma2(sum[i][j], w[i].y, x.y);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < COLS; ++j)
+      if (ty + 32 * i < count && tx + 16 * j < tokens && !is_finite(__ldcg(at(i, j)))) *at(i, j) = pair_sum(sum[i][j]);
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  any_of_workers(false);                                   // (the next tile goes over this one)
+}
 // The sum of one range of several, out of the accumulators.  Additions in memory take what is subnormal for zero.  Sums of 2^-102 and
 // more (and zeros) add up to nothing subnormal, as their last bits are 2^-125 and more; a smaller one becomes a NaN, and the
 // result is computed again.
@@ -370,11 +441,10 @@ __device__ __forceinline__ void cluster_barrier() {
 }
 
 // The sum of a range of an item, columns c0 .. of one of its rows: behind the item's first range it joins what this thread
-// has written of the ranges before.  `broken`: some sum of the item was not finite.
+// has written of the ranges before.  `broken`: some sum was not finite.
 template <int BT, int COLS>
 __device__ __forceinline__ void put_range(const Cut& cut, int item, int end, int row, int c0, const float (&acc)[COLS],
-                                          const float* __restrict__ X, const float* __restrict__ W, float* out, int M, int N,
-                                          int K, int64_t ldx, int64_t ldw, int64_t ldo, bool& broken) {
+                                          float* out, int M, int N, int64_t ldo, bool& broken) {
   int n0, m0, kb_begin, kb_end, range;
   place<BT>(cut, item, n0, m0, kb_begin, kb_end, range);
   const int n = n0 + row, m = m0 + c0, tokens = min(COLS, M - m);
@@ -402,11 +472,6 @@ __device__ __forceinline__ void put_range(const Cut& cut, int item, int end, int
       else dst[i * ldo] = v[i];
     }
   }
-  if (end != kb_end) return;
-  if (broken)
-    for (int i = 0; i < tokens; ++i)
-      if (!is_finite(__ldcg(dst + i * ldo))) dst[i * ldo] = again(X + (int64_t)(m + i) * ldx, W + (int64_t)n * ldw, K);
-  broken = false;
 }
 
 // Warps 0..15 cut the operands into parts (the weight's into tensor memory, the MMA's A operand; the tokens' into shared
@@ -567,7 +632,7 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
       return ok;
     };
     // the chunk that waits to be added: of which item; where its range ends, if with it
-    bool pending = false, broken = false;                  // (broken: a sum of this item was not finite)
+    bool pending = false, broken = false;                  // (broken: some sum was not finite)
     int p_item = 0, p_end = 0;
     for (int item = blockIdx.x; ok; item += gridDim.x) {
       int n0, m0, kb_begin = 0, kb_end = 1, range;
@@ -640,7 +705,7 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
               if (p_end) {
                 ++segments;
                 if (cut.split) break;                      // (the block's only item and range; `more` is false)
-                put_range<BT, COLS>(cut, p_item, p_end, row, side * COLS, acc, X, W, out, M, N, K, ldx, ldw, ldo, broken);
+                put_range<BT, COLS>(cut, p_item, p_end, row, side * COLS, acc, out, M, N, ldo, broken);
 #pragma unroll
                 for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
               }
@@ -677,10 +742,17 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         if (r >= ROWS || m >= M || n >= N) continue;
         float v = 0.f;
         for (int j = 0; j < cut.ranges; ++j) v += range_sum(parts[j * BT * each + i] * DOWN);
-        if (!is_finite(v)) v = again(X + (int64_t)m * ldx, W + (int64_t)n * ldw, K);
+        broken = broken || !is_finite(v);
         out[(int64_t)m * ldo + n] = v;
       }
     }
+    if (any_of_workers(broken))
+      for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
+        int n0, m0, kb_begin, kb_end, range;
+        place<BT>(cut, item, n0, m0, kb_begin, kb_end, range);
+        const int each = cut.split ? (ROWS + cut.ranges - 1) / cut.ranges : ROWS, first = cut.split ? range * each : 0;
+        once_more<BT>(X, W, out, M, N, K, ldx, ldw, ldo, n0 + first, min(each, ROWS - first), m0);
+      }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
   __syncthreads();

@@ -132,3 +132,22 @@ def test_subnormal_results(m):
     assert bool(((got.double() - want).abs() <= 1.2 * 2.0 ** -150).all())
     for row in (0, m - 1):
         assert torch.equal(ops.linear(a[row:row + 1].contiguous(), b)[0], got[row])
+
+
+@pytest.mark.parametrize("m", [1, 17, 90])
+@pytest.mark.parametrize("n,k", [(10001, 600), (2050, 2100), (700, 1100)])
+def test_broken_rows_of_either_operand(m, n, k):
+    """Results that are not finite, in tiles with a range each and with all: as multiply-adds have them; the others do not change."""
+    from gllm_b200 import ops
+
+    g = torch.Generator().manual_seed(m + n)
+    a, b = torch.randn(m, k, generator=g).cuda(), torch.randn(n, k, generator=g).cuda()
+    clean = ops.linear(a, b)
+    x, w = a.clone(), b.clone()
+    x[m - 1, k - 1], w[n - 1, 3], w[5, 0] = float("nan"), float("inf"), float("nan")
+    got, want = ops.linear(x, w), x.double() @ w.double().T
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[want.isinf()].double(), want[want.isinf()])
+    assert torch.equal(got[want.isfinite()], clean[want.isfinite()])
+    big = ops.linear(a * 1e34, b)                         # finite, and beyond what the parts' sums hold
+    assert _off(big / 1e34, a.double() @ b.double().T) <= 1e-6
