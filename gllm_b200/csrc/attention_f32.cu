@@ -32,8 +32,9 @@ template <int D> struct PortionSmem {
   int key_ok[2][KEYS];
 };
 
-template <int D>
-__global__ void __launch_bounds__(PF_THREADS, D == 64 ? 3 : 1)
+// PER_SM: blocks an SM has to hold (0: the compiler's choice)
+template <int D, int PER_SM>
+__global__ void __launch_bounds__(PF_THREADS, PER_SM)
 attention_f32_portion_kernel(const float* __restrict__ q, int64_t q_stride, float* __restrict__ out, int64_t out_stride,
                              const float* __restrict__ cache, const int* __restrict__ block_table, int bt_stride,
                              const int* __restrict__ cu_q, const int* __restrict__ ctx_lens,
@@ -381,18 +382,27 @@ int portions_launch(const float* q, int64_t q_stride, float* out, int64_t out_st
                     int requests, int max_q_len, int hq, int hkv, int block_size, int num_pages, float scale,
                     int window, int* status, cudaStream_t stream) {
   const int tokens = ROWS / (hq / hkv);
-  auto kernel = attention_f32_portion_kernel<D>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PortionSmem<D>));
-  if (e != cudaSuccess) return (int)e;
   const int64_t blocks = (int64_t)((max_q_len + tokens - 1) / tokens) * hkv * requests;
   if (blocks > 0x7fffffff) return (int)cudaErrorInvalidValue;
-  // (more blocks than SMs: 317 us with an early start, 282 without, for a layer over 512 and 200 (+300) tokens)
+  // Head size 64: a third block on an SM is paid for in registers, which only a grid that has it is to pay: 16 prompts of 16 tokens
+  // (128 blocks) 14.9 us with two, 17.1 with three, 4 of 130 (288) 31.9 and 31.4; 16 of 100 (896) 64 and 57, 2,000 tokens (1,000) 627
+  // and 569.  The other sizes are left to the compiler (asked for one block, head size 32 took 188 registers for 167 and lost its
+  // third one: 3 of 200 tokens behind 300 111 us for 86).
+  auto kernel = D != 64 ? attention_f32_portion_kernel<D, 0>
+                        : blocks > 2 * gllm_sm_count() ? attention_f32_portion_kernel<D, D == 64 ? 3 : 0>
+                                                       : attention_f32_portion_kernel<D, D == 64 ? 1 : 0>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PortionSmem<D>));
+  if (e != cudaSuccess) return (int)e;
+  // Blocks of unequal length that share SMs do not start early (gllm_launch_in_order): behind another kernel, head size 64, 300 tokens
+  // 64 us early and 49 in order, 3 of 200 behind 300 153 and 134, 4 of 130 45 and 35; but 8 of 128 39 and 43, 16 of 100 59 and 61.
+  // (With head size 128 a block has an SM to itself: 8 of 128 100 and 102, 1,024 tokens 394 and 396.)
+  const bool in_order = D < 128 && max_q_len > 2 * KEYS && blocks > gllm_sm_count();
   auto start = [&](auto launch) {
     return launch(kernel, dim3((unsigned)blocks), dim3(PF_THREADS), sizeof(PortionSmem<D>), stream, q, q_stride, out, out_stride,
                   cache, block_table, bt_stride, cu_q, ctx_lens, slots, requests, hq, hkv, block_size, num_pages, scale, window,
                   status);
   };
-  if (blocks > gllm_sm_count()) return start([](auto... a) { return gllm_launch_in_order(a...); });
+  if (in_order) return start([](auto... a) { return gllm_launch_in_order(a...); });
   return start([](auto... a) { return gllm_launch(a...); });
 }
 
