@@ -345,8 +345,10 @@ struct SharedParts {
 
 // A thread takes VEC neighbouring columns; the rows of up to four slots, and four parts of the shared expert's, are requested
 // together, and no thread takes a second stretch of columns: what bounds it is the one trip of 41 MB for 777 tokens of four slots
-// and two shared parts (2,048 columns), 9.7 us; with loads behind one another and two stretches a thread 15.9.
-template <typename T, int VEC>
+// and two shared parts (2,048 columns), 9.7 us; with loads behind one another and two stretches a thread 15.9.  SLOTS: rows requested
+// together; a token's only slot is one: the reads of three that are not there cost 2,048 tokens of 2,048 columns and three parts
+// 15.8 us for 9.0.
+template <typename T, int VEC, int SLOTS>
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(RowSum y, const T* __restrict__ shared, SharedParts parts, T* __restrict__ out, int width,
                    const float* __restrict__ shared_gate, int64_t shared_gate_stride) {
@@ -362,7 +364,7 @@ moe_combine_kernel(RowSum y, const T* __restrict__ shared, SharedParts parts, T*
 #pragma unroll
       for (int e = 0; e < VEC; ++e) sh[e] = to_float(from_float<T>(sh[e]));
     }
-    y.sum<VEC>(t, c, width, acc);
+    y.sum<VEC, SLOTS>(t, c, width, acc);
 #pragma unroll
     for (int e = 0; e < VEC; ++e) {
       if (parts.p) acc[e] = fmaf(sg, sh[e], acc[e]);
@@ -471,7 +473,8 @@ static int moe_combine_launch(const float* y, int n_parts, int64_t part_stride, 
   const bool vec = width % 4 == 0 && part_stride % 4 == 0 && shared_stride % 4 == 0 &&
                    ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(shared_parts)) & 15) == 0;
   const int blocks_y = (width + (vec ? 1024 : 256) - 1) / (vec ? 1024 : 256);
-  auto kernel = vec ? moe_combine_kernel<T, 4> : moe_combine_kernel<T, 1>;
+  auto kernel = top == 1 ? vec ? moe_combine_kernel<T, 4, 1> : moe_combine_kernel<T, 1, 1>
+                         : vec ? moe_combine_kernel<T, 4, 4> : moe_combine_kernel<T, 1, 4>;
   return gllm_launch(kernel, dim3(n_tokens, blocks_y), dim3(256), 0, stream, rows, shared, parts, out, width,
                      shared_gate, shared_gate_stride);
 }

@@ -53,3 +53,26 @@ def test_shared_parts_join_the_experts_as_their_sum_does(dtype, width, count, to
     want = want + (torch.sigmoid(logits.double())[:, None] if gate else 1.0) * shared
     # three products of numbers of a few units, then one rounding to the type
     torch.testing.assert_close(got.double(), want, rtol=2.0 ** -8 if dtype == torch.bfloat16 else 1e-6, atol=2e-6)
+
+
+@pytest.mark.parametrize("top", [1, 2, 3, 5])
+@pytest.mark.parametrize("parts", [1, 2, 3])
+@pytest.mark.parametrize("width", [66, 1028])
+@pytest.mark.parametrize("rows", [False, True])
+def test_sum_over_slots(top, parts, width, rows):
+    """Parts in ascending order, then slots in ascending order by fused multiply-adds; a token's only slot has a kernel of its own."""
+    from gllm_b200.ops import moe
+
+    g = torch.Generator().manual_seed(top)
+    tokens = 70
+    y, weights = torch.randn(parts, tokens * top, width, generator=g).cuda(), torch.rand(tokens, top, generator=g).cuda()
+    at = torch.randperm(tokens * top, generator=g) if rows else torch.arange(tokens * top)
+    got = moe.combine(y, weights, None, torch.float32, row_of_pair=at.int().cuda() if rows else None)
+    each = _in_order(y)[at.cuda()].view(tokens, top, width)
+    want = torch.zeros(tokens, width, device="cuda", dtype=torch.float64)
+    size = torch.zeros_like(want)
+    for s in range(top):
+        want += weights[:, s:s + 1].double() * each[:, s].double()
+        size += (weights[:, s:s + 1] * each[:, s]).abs().double()
+    # one rounding a slot, of a sum no larger than the magnitudes'
+    assert bool(((got.double() - want).abs() <= top * 2.0 ** -24 * size + 1e-37).all())
