@@ -832,6 +832,14 @@ void ranges_of(int N, int K, int& ranges, int& range_blocks) {
 // the rounding of multiply-adds errs by the root of K (1.9e-7 at 640, 2.6e-7 at 1,280, 3.5e-7 at 2,048, 5.0e-7 at 4,096): no chunk
 // is longer than leaves such a sum as close to 64 bits as multiply-adds leave it.
 int chunk_of(int K) { return K < 1280 ? 4 : K < 2048 ? 6 : K < 4096 ? 7 : 8; }
+// A range's blocks in as few chunks as that allows, of equal length (a range of 8 as 4 + 4: 2,048 x 2,048 x 1,536 131 us, 147 as 6 + 2).
+// 8 + 7 + .. + 7 where that saves one: 3.0e-7 .. 3.3e-7, and 700 x 16,384 x 2,048 (64 blocks) 264 us for 271.
+void chunks_of(Cut& cut, int K) {
+  const int most = chunk_of(K);
+  cut.extra = most == 7 && cut.range_blocks > 8 && cut.range_blocks % 7 == 1;
+  const int visits = (cut.range_blocks + most - 1) / most;
+  cut.chunk = cut.extra ? most : (cut.range_blocks + visits - 1) / visits;
+}
 
 // Tokens per tile and whether an item is one range: the layout whose fullest SM ends first.
 struct Plan { int bt, split; };
@@ -869,9 +877,7 @@ int launch(const float* X, const float* W, float* out, int M, int N, int K, int6
   cut.blocks = (K + KB - 1) / KB;
   cut.tiles_n = (N + ROWS - 1) / ROWS, cut.tiles_m = (M + BT - 1) / BT;
   cut.split = split;
-  cut.chunk = chunk_of(K);
-  // (64 blocks as 8 + 7 + .. + 7: 3.0e-7, and a visit less: 700 x 16,384 x 2,048 264 us for 271)
-  cut.extra = cut.chunk == 7 && cut.range_blocks > 8 && cut.range_blocks % 7 == 1;
+  chunks_of(cut, K);
   const int64_t items = (int64_t)cut.tiles_n * cut.tiles_m * (split ? cut.ranges : 1);
   if (items > 0x7fffffff - 4096) return (int)cudaErrorInvalidValue;
   auto kernel = gemm_f32_parts_kernel<BT>;
