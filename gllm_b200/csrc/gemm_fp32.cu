@@ -10,7 +10,8 @@
 //   x = x0 + x1 + x2,  w = w0 + w1 + w2,
 //   x w = w0 x0 + (w0 x1 + w1 x0 + w0 x2 + w1 x1 + w2 x0) + terms of up to 2^-24 |x w|.
 // Everything else runs a plain 64 x 64 tile of 32-bit multiply-adds.  In both
-// multiply-add kernels an output is two sums, of even and of odd k.
+// multiply-add kernels an output is two sums, of even and odd k or of the first
+// and second half.
 //
 // The tensor cores' own additions truncate.  The leading products' accumulator
 // is therefore taken out of tensor memory every 128 .. 256 of K (chunk_of) and
@@ -52,37 +53,48 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
   const int tid = threadIdx.x;
   const int tx = tid % 16, ty = tid / 16;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[2][TM][TN];            // of the products with even and with odd k
+  // Two sums an output, of the first half of the k-tiles and of the rest: an addition's rounding is that of a sum half as long.
+  // (Sums of even and of odd k, live side by side in the loop, took 364 us for 700 x 2,048 x 2,049, one sum and these 254.)
+  float acc[TM][TN], first[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[0][i][j] = acc[1][i][j] = 0.f;
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
 
   // each thread loads 4 elements of A and 4 of B per k-tile
   const int lrow = tid / 4;        // 0..63
   const int lk = (tid % 4) * 4;    // 0,4,8,12
-  for (int k0 = 0; k0 < K; k0 += BK) {
+  const int half = (K + BK - 1) / BK / 2 * BK;
+  for (int part = 0; part < 2; ++part) {
+    for (int k0 = part == 0 ? 0 : half; k0 < (part == 0 ? half : K); k0 += BK) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int k = k0 + lk + e;
-      const int am = m0 + lrow, bn = n0 + lrow;
-      As[lk + e][lrow] = (am < M && k < K) ? A[(int64_t)am * lda + k] : 0.f;
-      Bs[lk + e][lrow] = (bn < N && k < K) ? B[(int64_t)bn * ldb + k] : 0.f;
+      for (int e = 0; e < 4; ++e) {
+        const int k = k0 + lk + e;
+        const int am = m0 + lrow, bn = n0 + lrow;
+        As[lk + e][lrow] = (am < M && k < K) ? A[(int64_t)am * lda + k] : 0.f;
+        Bs[lk + e][lrow] = (bn < N && k < K) ? B[(int64_t)bn * ldb + k] : 0.f;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int kk = 0; kk < BK; ++kk) {
+        float a[TM], b[TN];
+#pragma unroll
+        for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
+#pragma unroll
+        for (int j = 0; j < TN; ++j) b[j] = Bs[kk][tx * TN + j];
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+      }
+      __syncthreads();
     }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      float a[TM], b[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = Bs[kk][tx * TN + j];
+    if (part == 0) {
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[kk & 1][i][j] = fmaf(a[i], b[j], acc[kk & 1][i][j]);
+        for (int j = 0; j < TN; ++j) first[i][j] = acc[i][j], acc[i][j] = 0.f;
     }
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -91,7 +103,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       const int n = n0 + tx * TN + j;
-      if (n < N) C[(int64_t)m * ldc + n] = acc[0][i][j] + acc[1][i][j];
+      if (n < N) C[(int64_t)m * ldc + n] = first[i][j] + acc[i][j];
     }
   }
 }
