@@ -271,7 +271,7 @@ struct Shape {
   static constexpr int COLS = (2 + CROSS) * BT + CUT * A_COLS;
   static constexpr int TMEM_COLS = COLS <= 256 ? 256 : 512;
   static constexpr int SMEM = STAGES * RAW + CUT * PARTS + 1024;
-  static_assert(COLS <= 512 && STAGES >= GROUPS, "fits");
+  static_assert(COLS <= 512 && CUT >= GROUPS && STAGES >= CUT, "fits, and no wait is more than a phase behind");
 };
 
 // Shared-memory descriptor of a K-major tile with rows of 64 bytes, 64-byte swizzle, 8-row groups 512 bytes apart.
