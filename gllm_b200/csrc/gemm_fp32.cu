@@ -32,11 +32,12 @@
 // What bounds it: with many tokens the cutting (sixteen warps, about 400 issue
 // cycles for a block of 32 k) and shared memory (110 KB, 860 cycles), where the
 // products of 96 tokens take 583; with few the same chain at half of what
-// DRAM gives.  700 x 16,384 x 2,048: 260 us = 181 TFLOP/s, 1,018 us with
-// packed multiply-adds on the CUDA cores; 700 x 2,048 x 8,192: 154 for 629;
-// 8 x 16,384 x 2,048: 43 for 88; 250 x 2,048 x 2,048: 46 for 76.  Relative
-// error against 64 bits at K = 2,048 and 8,192: 2.4e-7 for 5.7e-7 and 1.2e-6
-// (every 128 of K instead of 256: 1.4e-7, and 5 to 30 % slower).
+// DRAM gives.  700 x 16,384 x 2,048: 266 us = 177 TFLOP/s, 1,014 us with
+// packed multiply-adds on the CUDA cores; 700 x 2,048 x 8,192: 148 for 627;
+// 8 x 16,384 x 2,048: 28 for 79; 300 x 2,048 x 2,048: 42 for 108.  Relative
+// error against 64 bits at K = 1,024, 2,048 and 8,192: 1.3e-7, 1.7e-7 and
+// 2.4e-7 for 4.1e-7, 5.7e-7 and 1.1e-6; operands of one sign 1.7e-7, 2.8e-7 ..
+// 3.3e-7 and 3.8e-7 for 2.5e-7, 3.5e-7 and 7.0e-7.
 #include "umma_utils.cuh"
 
 namespace {

@@ -933,7 +933,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
     """``x @ weight.T`` with ``weight`` stored ``[out, in]``
     (gllm/model/layers/linear.py:20).  fp32 inputs run a true 32-bit product
     (``csrc/gemm_fp32.cu``); bf16 inputs run the tensor-core kernels with fp32
-    accumulation.  With ``split_ok`` the result may be a SplitSum (for callers
+    accumulation and request ``weight`` ahead of the kernel before them on the
+    stream, so there it has to be older than that kernel (a stored parameter);
+    in fp32 it may be its result.  With ``split_ok`` the result may be a SplitSum (for callers
     that hand it to ``add_rmsnorm`` or ``rope_store``).  With ``add_into``
     (fp32 ``[m, n]``, the residual stream) the product may add itself there
     and return ``ADDED``; when it returns anything else, nothing was added.  With ``bias`` (fp32, one
